@@ -48,3 +48,52 @@ def test_product_of_a_column_range_and_unaligned_bases(ops):
         ops.linear_cols(base, col0, w, out)
         bound = 99 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
         assert bool(((out - ref).abs() <= bound).all()), col0
+
+
+# heads per stored head 1, 3, 2, 16 and 20 (two cuts); head sizes at and beside the element counts of the instances
+@pytest.mark.parametrize("nh,nkv,d,P,dtype", [(4, 4, 20, 5, torch.float32), (6, 2, 64, 16, torch.float32), (4, 2, 72, 64, torch.float32),
+                                              (16, 1, 130, 7, torch.float32), (20, 1, 128, 32, torch.float32), (8, 4, 256, 64, torch.float32),
+                                              (3, 1, 512, 16, torch.float32), (2, 1, 300, 16, torch.bfloat16), (6, 2, 40, 8, torch.bfloat16)])
+@pytest.mark.parametrize("window,keep,sink", [(0, 0, False), (40, 0, False), (33, 37, True)])
+def test_generic_attention(ops, nh, nkv, d, P, dtype, window, keep, sink):
+    """Rows of several requests in one launch, alone, and behind a list of rows: the same bits; against 64 bits; and a key
+    that a row does not see does not reach it, whatever its value holds."""
+    from test_gpu_kernels import _Ctx, _View, _paged_setup
+    lens = [1, 200, 31, 33, 64]
+    pages, table, ks, vs = _paged_setup(dtype, nh, nkv, d, P, lens, seed=11)
+    rows = [(1, p) for p in range(95, 130)] + [(-1, 0)] + [(2, p) for p in range(31)] + [(3, 32), (0, 0), (4, 63), (3, 31), (1, 199)]
+    g = torch.Generator().manual_seed(6)
+    q = torch.randn(len(rows), nh * d, generator=g).to(dtype).to(DEV)
+    dev_pages, dev_table = pages.to(DEV), table.to(DEV)
+
+    def attend(which, p=dev_pages):
+        ctx = _Ctx(torch.tensor([rows[i][1] for i in which], dtype=torch.int32, device=DEV),
+                   torch.tensor([rows[i][0] for i in which], dtype=torch.int32, device=DEV), dev_table)
+        out = torch.full((len(which), nh * d), float("nan"), dtype=dtype, device=DEV)
+        ops.paged_attention(q[which], out, ctx, _View(p, P), nh, nkv, d, d ** -0.5, 30.0, window or None, keep_first=keep, sink=sink)
+        return out
+
+    whole = attend(list(range(len(rows))))
+    assert float(whole[35].abs().max()) == 0.0                        # the padding row
+    for which in ([0], [34, 36], list(range(36, 50)), [71, 3]):
+        assert torch.equal(attend(which), whole[which])
+    for i, (r, p) in enumerate(rows):
+        if r < 0:
+            continue
+        see = torch.tensor([j for j in range(p + 1) if not window or p - j < window or j < keep])
+        kd, vd = ks[r][see].double(), vs[r][see].double()
+        kd, vd = kd.repeat_interleave(nh // nkv, 1), vd.repeat_interleave(nh // nkv, 1)
+        s = torch.einsum("jhd,hd->hj", kd, q[i].cpu().double().view(nh, d)) * d ** -0.5
+        s = 30.0 * torch.tanh(s / 30.0)
+        e = torch.exp(s - s.amax(1, keepdim=True))
+        w = e / (e.sum(1, keepdim=True) + (torch.exp(-s.amax(1, keepdim=True)) if sink else 0.0))
+        want = torch.einsum("hj,jhd->hd", w, vd)
+        err = (whole[i].cpu().double().view(nh, d) - want).abs().max()
+        # scores of size <= 30 err by (d + 4) 2^-24 of |q| |k| scale <= 8 sqrt(d) each; the weights by as much, relatively
+        bound = (d + 40) * 2.0 ** -24 * 8 * d ** 0.5 * vd.abs().max() + (2.0 ** -8 * want.abs().max() if dtype == torch.bfloat16 else 0)
+        assert float(err) <= float(bound), (i, float(err), float(bound))
+    # request 1, position 120: rows 0..24 (positions 95..119) must not see it
+    poisoned = pages.clone()
+    poisoned[table[1, 120 // P], 1, :, 120 % P] = float("inf")
+    got = attend(list(range(len(rows))), poisoned.to(DEV))
+    assert torch.equal(got[:25], whole[:25]) and not bool(got[25].isfinite().all())
