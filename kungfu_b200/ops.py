@@ -1157,13 +1157,13 @@ def repeat_rows(a, b, parts: int, out_a, out_b) -> None:
 
 
 def _grouped(x, x_off, ldx, x_gstride, row_index, row_div, w, w_gstride, out, o_off, ldo, o_gstride, tiles, max_tiles,
-             n_groups, T, N, K, gated, limit, what, row_scale=None):
+             n_groups, T, N, K, gated, limit, what, row_scale=None, most_rows=0):
     tg, tr, tn, nt = tiles if tiles is not None else (None, None, None, None)
     L = ctypes.c_long
     _check(library().kf_grouped_linear(_p(x), _dt(x), L(x_off), L(ldx), L(x_gstride), _p(row_index), int(row_div), _p(w),
                                        _dt(w), L(w_gstride), _p(out), _dt(out), L(o_off), L(ldo), L(o_gstride), _p(tg),
                                        _p(tr), _p(tn), _p(nt), int(max_tiles), int(n_groups), int(T), int(N), int(K),
-                                       int(gated), _f(limit), _p(row_scale), _stream()), what)
+                                       int(gated), _f(limit), _p(row_scale), int(most_rows), _stream()), what)
 
 
 def grouped_on_tensor_cores(on: bool) -> None:
@@ -1237,7 +1237,8 @@ def moe_linear(x, plan: dict, weight, out, *, gather: bool, gated: bool = False,
         raise KernelError(f"moe_linear: x{tuple(x.shape)} weight{tuple(weight.shape)} out{tuple(out.shape)} do not agree")
     tiles = (plan["tile_group"], plan["tile_row0"], plan["tile_nrows"], plan["n_tiles"])
     _grouped(x, 0, K, 0, plan["sorted_pair"] if gather else None, plan["top"] if gather else 1, weight, NW * K, out, 0, N, 0,
-             tiles, plan["max_tiles"], E, plan["pairs"], N, K, (2 if activation == "silu" else 1) if gated else 0, limit, "moe_linear", row_scale=row_scale)
+             tiles, plan["max_tiles"], E, plan["pairs"], N, K, (2 if activation == "silu" else 1) if gated else 0, limit, "moe_linear", row_scale=row_scale,
+             most_rows=plan["pairs"] // plan["top"])               # a token chooses an expert once
 
 
 @_dispatch("moe_combine")
