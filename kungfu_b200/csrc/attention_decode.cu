@@ -157,6 +157,56 @@ __device__ __forceinline__ void merge_splits(const float* __restrict__ partial, 
   }
 }
 
+// The same merge of a few records through shared memory: the records of a row's heads lie behind one another, so all of
+// them are asked for at once (16-byte cp.async) and the weights and sums are made from shared memory: one trip to L2 where
+// the loop above takes one for the maxima and another for every sixteen splits.  `buf` holds n_heads * n_splits records.
+// With the loads of the rotation in one trip too (below), a decode step of the 2B model at 8,192 tokens: one request 1.720 ->
+// 1.665 ms (33 splits), 64 requests of 100 to 1,000 tokens (no splits) 3.24 -> 3.16 ms.
+template <int D>
+__device__ __forceinline__ void merge_splits_shared(const float* __restrict__ partial, size_t first_record, int n_heads,
+                                                    int n_splits, __nv_bfloat16* __restrict__ o_first, float* buf) {
+  constexpr int PS = KF_PSTRIDE(D);
+  const float* rec0 = partial + first_record * PS;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n_warps = blockDim.x >> 5;
+  for (int i = tid; i < n_heads * n_splits * (PS / 4); i += blockDim.x) kf_mma::cp_async16(buf + 4 * i, rec0 + 4 * i, true);
+  kf_mma::cp_async_commit();
+  kf_mma::cp_async_wait<0>();
+  __syncthreads();
+  for (int h = warp; h < n_heads; h += n_warps) {
+    float* rec = buf + (size_t)h * n_splits * PS + D;              // maximum, sum; the maximum's place takes the weight
+    float m = -INFINITY;
+    for (int sp = lane; sp < n_splits; sp += 32) m = fmaxf(m, rec[sp * PS]);
+    m = kf_warp_max(m);
+    float l = 0.f;
+    for (int sp = lane; sp < n_splits; sp += 32) {
+      const float ms = rec[sp * PS];
+      const float c = (ms == -INFINITY) ? 0.f : exp2f(ms - m);
+      l += rec[sp * PS + 1] * c;
+      rec[sp * PS] = c;
+    }
+    l = kf_warp_sum(l);                                            // a fixed order: lanes hold interleaved splits
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+    __syncwarp();
+    for (int sp = lane; sp < n_splits; sp += 32) rec[sp * PS] *= inv;
+  }
+  __syncthreads();
+  for (int e = tid; e < n_heads * (D / 4); e += blockDim.x) {
+    const int h = e / (D / 4), i4 = e - h * (D / 4);
+    const float* rec = buf + (size_t)h * n_splits * PS;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int sp = 0; sp < n_splits; ++sp) {
+      const float4 v = *reinterpret_cast<const float4*>(rec + sp * PS + i4 * 4);
+      const float c = rec[sp * PS + D];
+      a.x += v.x * c; a.y += v.y * c; a.z += v.z * c; a.w += v.w * c;
+    }
+    uint2 packed;
+    packed.x = kf_mma::pack_bf16(a.x, a.y);
+    packed.y = kf_mma::pack_bf16(a.z, a.w);
+    *reinterpret_cast<uint2*>(o_first + (size_t)h * D + i4 * 4) = packed;
+  }
+}
+
 template <int D, int HT>
 __global__ void __launch_bounds__(DEC_WARPS * 32)
 attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ pages,
@@ -458,46 +508,64 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
 #pragma unroll
   for (int n = 0; n < DM_BUFS; ++n)
     if (n < n_loads && warp + (n >> 1) * DM_WARPS != own_tile) load_item(n, n);
+  if (qkv != nullptr)
+    for (int idx = G * CH + tid; idx < 16 * CH; idx += blockDim.x)
+      *reinterpret_cast<uint4*>(tile_ptr<D>(sQ, idx / CH, idx % CH)) = make_uint4(0, 0, 0, 0);
   kf_pdl_wait();
   q = kf_produced(q), qkv = kf_produced(qkv), cos_t = kf_produced(cos_t), sin_t = kf_produced(sin_t);
 
   if (qkv != nullptr) {
-    // ---- Q: rotated here; rows 0..G-1 are the heads of this kv head, the rest of the 16 rows are zero ---------------------
+    // ---- Q: rotated here; rows 0..G-1 are the heads of this kv head, the rest of the 16 rows are zero (written above) -----
     const float* in = qkv + (size_t)t * (nh + 2 * nkv) * D;
     const int half = rot >> 1;
     const float* cs = cos_t + (size_t)t * half;
     const float* sn = sin_t + (size_t)t * half;
+    // Eight elements of a head, rotated.  With whole 16-byte vectors on every side of the halves (`vec`) the eight loads of
+    // a chunk are asked for together: one trip to L2 where element by element, under the branches, took one per element.
+    const bool vec = (half & 7) == 0 && ((((uintptr_t)qkv) | ((uintptr_t)cos_t) | ((uintptr_t)sin_t)) & 15) == 0;
     auto rotated8 = [&](const float* head, int c8) -> uint4 {
       float v[8];
+      if (vec) {
+        const int i = c8 * 8;
+        const bool turned = i < rot, low = i < half;
+        const int at = low ? i : i - half;                       // place in the tables, and of the other half's elements
+        const float4* x4 = reinterpret_cast<const float4*>(head + i);
+        const float4* y4 = reinterpret_cast<const float4*>(head + (turned ? (low ? i + half : i - half) : i));
+        const float4* c4 = reinterpret_cast<const float4*>(turned ? cs + at : head + i);
+        const float4* s4 = reinterpret_cast<const float4*>(turned ? sn + at : head + i);
+        const float4 x0 = x4[0], x1 = x4[1], y0 = y4[0], y1 = y4[1], c0 = c4[0], c1 = c4[1], s0 = s4[0], s1 = s4[1];
+        const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, y[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
+        const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, n[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const int i = c8 * 8 + e;
-        float x = head[i];
-        if (i < half) x = x * cs[i] - head[i + half] * sn[i];
-        else if (i < rot) x = head[i - half] * sn[i - half] + x * cs[i - half];
-        v[e] = x;
+        for (int e = 0; e < 8; ++e) v[e] = !turned ? x[e] : low ? x[e] * c[e] - y[e] * n[e] : y[e] * n[e] + x[e] * c[e];
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int i = c8 * 8 + e;
+          float x = head[i];
+          if (i < half) x = x * cs[i] - head[i + half] * sn[i];
+          else if (i < rot) x = head[i - half] * sn[i - half] + x * cs[i - half];
+          v[e] = x;
+        }
       }
       return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
     };
-    for (int idx = tid; idx < 16 * CH; idx += blockDim.x) {
+    // The row's own key and value, written to the page by the block that will read them: chunks of their own behind those
+    // of the heads, so that other threads turn them at the same time.
+    const int own_page = write_kv && own_tile >= 0 ? tab[pos / page_size] : -1;
+    __nv_bfloat16* kdst = pages + ((long)max(own_page, 0) * 2 * nkv + kvh) * (long)head_stride + (long)(pos % page_size) * D;
+    for (int idx = tid; idx < (G + 2) * CH; idx += blockDim.x) {
       const int r = idx / CH, c = idx - r * CH;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (r < G) v = rotated8(in + (size_t)(h_first + r) * D, c);
-      *reinterpret_cast<uint4*>(tile_ptr<D>(sQ, r, c)) = v;
-    }
-    // ---- the row's own key and value: rotated, written to the page by the block that will read them ---------------------
-    if (write_kv && own_tile >= 0) {
-      const int page = tab[pos / page_size];
-      if (page >= 0) {
-        __nv_bfloat16* kdst = pages + ((long)page * 2 * nkv + kvh) * (long)head_stride + (long)(pos % page_size) * D;
-        const float* kin = in + (size_t)(nh + kvh) * D;
-        const float* vin = in + (size_t)(nh + nkv + kvh) * D;
-        for (int c = tid; c < CH; c += blockDim.x) {
-          *reinterpret_cast<uint4*>(kdst + c * 8) = rotated8(kin, c);
-          const float* vv = vin + c * 8;
-          *reinterpret_cast<uint4*>(kdst + v_off + c * 8) =
-              make_uint4(pack_bf16(vv[0], vv[1]), pack_bf16(vv[2], vv[3]), pack_bf16(vv[4], vv[5]), pack_bf16(vv[6], vv[7]));
-        }
+      if (r >= G && own_page < 0) continue;
+      const float* src = in + (size_t)(r < G ? h_first + r : r == G ? nh + kvh : nh + nkv + kvh) * D;
+      if (r <= G) {
+        const uint4 v = rotated8(src, c);
+        if (r < G) *reinterpret_cast<uint4*>(tile_ptr<D>(sQ, r, c)) = v;
+        else *reinterpret_cast<uint4*>(kdst + c * 8) = v;
+      } else {
+        const float* vv = src + c * 8;
+        *reinterpret_cast<uint4*>(kdst + v_off + c * 8) =
+            make_uint4(pack_bf16(vv[0], vv[1]), pack_bf16(vv[2], vv[3]), pack_bf16(vv[4], vv[5]), pack_bf16(vv[6], vv[7]));
       }
     }
   } else {
@@ -693,7 +761,10 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
   __syncthreads();
   if (!s_last) return;
   __threadfence();                                               // maxima here are base-2 scaled
-  merge_splits<D, true>(partial, ((size_t)t * nh + h_first) * n_splits, G, n_splits, orow + (size_t)h_first * D);
+  if (n_splits > 8 && (size_t)G * n_splits * PSTRIDE * sizeof(float) <= (size_t)DM_WARPS * DM_BUFS * TILE * sizeof(__nv_bfloat16))
+    merge_splits_shared<D>(partial, ((size_t)t * nh + h_first) * n_splits, G, n_splits, orow + (size_t)h_first * D, sm_o);
+  else
+    merge_splits<D, true>(partial, ((size_t)t * nh + h_first) * n_splits, G, n_splits, orow + (size_t)h_first * D);
   if (tid == 0) counters[cidx] = 0;
 }
 
