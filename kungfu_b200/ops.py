@@ -700,6 +700,11 @@ def head_gate(o, proj, gate_col0: int, n_heads: int, value_dim: int, head_dim: i
 
 
 chunked_scan = True          # False: a long prompt's recurrence is walked by one block per (request, head, 32 columns) only
+# The recurrence runs as products over blocks of 128 rows from this many rows in a step on, and on average per request (a block
+# of few rows costs nearly a whole one).  At 64 heads x 64 x 128, walk against blocks in us: one request of 128 rows 46 / 60,
+# 192 65 / 58, 512 156 / 71, 2,048 592 / 208; eight of 64 rows 79 / 97, of 128 139 / 130, of 256 260 / 208; 32 of 32 rows 154 / 251.
+SCAN_BLOCKS_FROM = 192
+SCAN_BLOCKS_ROWS_EACH = 96
 SCAN_CHUNK_ROWS = 256
 SCAN_CHUNKED_FROM = 1024     # rows of a step from which the chunks are walked side by side ...
 SCAN_CHUNKED_BLOCKS = 160    # ... if the plain walk would have at most this many blocks (about one per SM); with two per SM
@@ -725,9 +730,10 @@ def ssm_scan(xbc, proj, dt_col0: int, dt_bias, a_log, d_skip, state, y, heads: i
     """The state-space recurrence over the rows of every request of the step, from and into `state`
     [requests, heads, head_dim, state_dim] (32-bit): S = exp(-exp(a_log) dt) S + dt B x^T, y = S^T C + d_skip x, with
     dt = softplus(proj[:, dt_col0 + h] + dt_bias[h]); xbc rows are [x | B | C] (32-bit).
-    Steps of single rows run a kernel without staging; steps of a thousand rows and more whose requests are too few to
-    fill the GPU are cut into chunks of 256 rows that are walked side by side (their start states follow from a first
-    pass over the chunks): 435 against 590 us for one prompt of 2,048 tokens at 64 heads x 64 x 128; with two such
+    Steps of single rows run a kernel without staging.  Prompts of at most 128 states on whole vectors run as products
+    over blocks of 128 rows (see SCAN_BLOCKS_FROM).  Other sizes: steps of a thousand rows and more whose requests are too
+    few to fill the GPU are cut into chunks of 256 rows that are walked side by side (their start states follow from a
+    first pass over the chunks): 435 against 590 us for one prompt of 2,048 tokens at 64 heads x 64 x 128; with two such
     prompts the plain walk is already the faster one."""
     T = xbc.shape[0]
     lib = library()
@@ -735,6 +741,18 @@ def ssm_scan(xbc, proj, dt_col0: int, dt_bias, a_log, d_skip, state, y, heads: i
     common = (_p(xbc), xbc.shape[1], _p(proj), proj.shape[1], int(dt_col0), _p(dt_bias), _p(a_log), _p(d_skip), _dt(a_log),
               _p(state), _p(y), heads, groups, head_dim, state_dim, ctx.n_reqs, _p(ctx.req_row_start), _p(ctx.req_n_rows),
               _p(ctx.req_state_slot), int(writes))
+    if (chunked_scan and not single and T >= max(SCAN_BLOCKS_FROM, SCAN_BLOCKS_ROWS_EACH * ctx.n_reqs) and hasattr(ctx, "buf")
+            and lib.kf_ssm_blocks_supported(_p(xbc), xbc.shape[1], _p(state), heads, groups, head_dim, state_dim)):
+        L = lib.kf_ssm_blocks_rows()
+        n_blocks = T // L + ctx.n_reqs
+        blocks = ctx.buf("ssm_blocks", (2 * n_blocks + 2 * ctx.n_reqs,), torch.int32)
+        block_state = ctx.buf("ssm_block_state", (n_blocks, heads, head_dim, state_dim), torch.float32)
+        block_decay = ctx.buf("ssm_block_decay", (n_blocks, heads), torch.float32)
+        inside = ctx.buf("ssm_block_table", (n_blocks, groups, L, L), torch.float32)
+        _check(lib.kf_ssm_scan_blocks(*common, n_blocks, _p(blocks), _p(block_state), _p(block_decay), _p(inside), _stream()),
+               "ssm_scan (products over blocks of rows)")
+        add_launches(3)
+        return
     few = ctx.n_reqs * heads * -(-head_dim // 32) <= SCAN_CHUNKED_BLOCKS
     if chunked_scan and not single and few and T >= SCAN_CHUNKED_FROM and hasattr(ctx, "buf"):
         n_chunks = T // SCAN_CHUNK_ROWS + ctx.n_reqs

@@ -1,0 +1,59 @@
+"""The state-space recurrence as products over blocks of rows, against 64 bits, at the edges of its blocks and tiles."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _step(rows, slots):
+    starts = [sum(rows[:i]) for i in range(len(rows))]
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pool = {}
+
+    def buf(tag, shape, dtype):
+        return pool.setdefault(tag, torch.full(shape, float("nan") if dtype.is_floating_point else 0, dtype=dtype, device=DEV))
+    return types.SimpleNamespace(n_reqs=len(rows), req_row_start=ints(starts), req_n_rows=ints(rows), req_state_slot=ints(slots),
+                                 decode_only=False, buf=buf)
+
+
+# rows 1, 127, 128, 129 and several blocks, an empty slot; P of one tile, two tiles, the last ragged; N below, at and off 32s;
+# rates from almost none to ones whose decay over a block is far below the smallest number
+@pytest.mark.parametrize("heads,groups,P,N,rows", [(2, 1, 64, 128, (300, 0, 128)), (4, 2, 64, 128, (200, 1, 127)), (3, 3, 12, 20, (400,)),
+                                                   (2, 1, 68, 36, (130, 257)), (1, 1, 132, 4, (500,)), (2, 2, 4, 100, (256, 192))])
+@pytest.mark.parametrize("rate", [-4.0, 1.0, 5.0])
+def test_blocks_against_64_bits(heads, groups, P, N, rows, rate):
+    from kungfu_b200 import ops
+    g = torch.Generator().manual_seed(P + N + len(rows))
+    T, inner = sum(rows), heads * P
+    ld_x, ld_p, dt0 = inner + 2 * groups * N + 4, heads + 3, 2
+    x, pr = torch.randn(T + 1, ld_x, generator=g), torch.randn(T + 1, ld_p, generator=g)
+    a_log, dt_bias, D = rate + torch.rand(heads, generator=g), torch.randn(heads, generator=g) - 1, torch.randn(heads, generator=g)
+    slots = [2, 0, 3][:len(rows)]
+    state = torch.randn(4, heads, P, N, generator=g)
+    dev = state.to(DEV)
+    y = torch.full((T + 1, inner), 7.0, device=DEV)
+    before = ops.launch_count()
+    ops.ssm_scan(x.to(DEV), pr.to(DEV), dt0, dt_bias.to(DEV), a_log.to(DEV), D.to(DEV), dev, y, heads, groups, P, N, _step(rows, slots))
+    assert ops.launch_count() - before == 4
+    assert float(y[-1].min()) == 7.0 and torch.equal(dev[1].cpu(), state[1])
+    at = 0
+    for r, slot in zip(rows, slots):
+        S = state[slot].double()
+        size = S.abs()
+        for t in range(at, at + r):
+            B = x[t, inner:inner + groups * N].double().view(groups, N).repeat_interleave(heads // groups, 0)
+            C = x[t, inner + groups * N:inner + 2 * groups * N].double().view(groups, N).repeat_interleave(heads // groups, 0)
+            xs = x[t, :inner].double().view(heads, P)
+            dt = torch.nn.functional.softplus(pr[t, dt0:dt0 + heads].double() + dt_bias.double())
+            decay = torch.exp(-torch.exp(a_log.double()) * dt)[:, None, None]
+            S = decay * S + (dt[:, None] * xs)[:, :, None] * B[:, None, :]
+            size = decay * size + (dt[:, None] * xs).abs()[:, :, None] * B.abs()[:, None, :]
+            want = torch.einsum("hpn,hn->hp", S, C) + D.double()[:, None] * xs
+            # sizes of what is summed, times roundings: N + 128 terms, dt and the decays (relative to a few 2^-24)
+            bound = (N + 160) * 2.0 ** -24 * (torch.einsum("hpn,hn->hp", size, C.abs()) + (D.double()[:, None] * xs).abs()) + 1e-30
+            assert bool(((y[t].cpu().double().view(heads, P) - want).abs() <= bound).all()), t
+        assert bool(((dev[slot].cpu().double() - S).abs() <= 300 * 2.0 ** -24 * size + 1e-30).all())
+        at += r
