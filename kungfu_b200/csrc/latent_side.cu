@@ -15,7 +15,7 @@
 //                        second factor is looked up by token id.
 // kf_repeat_rows:        out[t * parts + j] = in[t] for two integer arrays at once: the positions and requests of a step
 //                        whose every row is presented to the attention kernels as `parts` rows of fewer heads.
-#include "common.cuh"
+#include "residual_norm.cuh"
 
 __global__ void repeat_rows_kernel(const int* __restrict__ a, const int* __restrict__ b, int* __restrict__ out_a,
                                    int* __restrict__ out_b, int T, int parts) {
@@ -230,6 +230,20 @@ __global__ void scale_add_rmsnorm_kernel(const float* __restrict__ a, const TS* 
 KF_API int kf_scale_add_rmsnorm(const float* a, const void* s, int s_dtype, float* x, const void* w, float eps, int plus_one,
                                 void* out, void* copy, int out_dtype, int T, int H, cudaStream_t stream) {
   if (T <= 0) return KF_OK;
+#define KF_ROW(TS, TO)                                                                                                    \
+  kf_launch_residual_norm<KF_RES_SCALED>(a, (const float*)nullptr, (const TS*)s, 0.f, 0, x, (const TS*)w, eps, plus_one ? 1 : 0, \
+                                         (TO*)out, (TO*)copy, T, H, stream)
+  const int s_size = s_dtype == KF_F32 ? 4 : 2;
+  if (kf_residual_norm_takes(a, nullptr, s, s_size, x, out ? w : nullptr, s_size, out, copy, out_dtype == KF_F32 ? 4 : 2, H)) {
+    if (s_dtype == KF_F32 && out_dtype == KF_F32) KF_ROW(float, float);
+    else if (s_dtype == KF_BF16 && out_dtype == KF_BF16) KF_ROW(__nv_bfloat16, __nv_bfloat16);
+    else if (s_dtype == KF_BF16 && out_dtype == KF_F32) KF_ROW(__nv_bfloat16, float);
+    else if (s_dtype == KF_F32 && out_dtype == KF_BF16) KF_ROW(float, __nv_bfloat16);
+    else return KF_ERR_DTYPE;
+    KF_CHECK_LAUNCH();
+    return KF_OK;
+  }
+#undef KF_ROW
   const int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
 #define KF_GO(TS, TO)                                                                                                     \
   kf_launch(scale_add_rmsnorm_kernel<TS, TS, TO, TO>, dim3(T), dim3(threads), 0, stream, a, (const TS*)s, x, (const TS*)w, \

@@ -1,8 +1,9 @@
 // The residual update of a block whose branches run side by side on one normed input:
 //   x[t] += a[t] + b[t]      (b may be absent), all in 32-bit,
 // and, in the same pass, the RMS norm the next block starts with: next[t] = x[t] / sqrt(mean(x[t]^2) + eps) * g,
-// g = w or 1 + w.  One block per row; a thread reads back only elements it wrote itself.
-#include "common.cuh"
+// g = w or 1 + w.  Rows of whole vectors run the kernel of residual_norm.cuh; others the one below, a block per row whose
+// threads read back only elements they wrote themselves.
+#include "residual_norm.cuh"
 
 template <typename TW, typename TO>
 __global__ void add2_rmsnorm_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ x,
@@ -31,6 +32,18 @@ __global__ void add2_rmsnorm_kernel(const float* __restrict__ a, const float* __
 KF_API int kf_add2_rmsnorm(const float* a, const float* b, float* x, const void* w, int w_dtype, float eps, int plus_one,
                            void* out, int out_dtype, int T, int H, cudaStream_t stream) {
   if (T <= 0) return KF_OK;
+#define KF_ROW(TW, TO)                                                                                                  \
+  kf_launch_residual_norm<KF_RES_PLAIN>(a, b, (const TW*)w, 0.f, 0, x, (const TW*)w, eps, plus_one ? 1 : 0, (TO*)out, (TO*)nullptr, T, H, stream)
+  if (kf_residual_norm_takes(a, b, nullptr, 4, x, out ? w : nullptr, w_dtype == KF_F32 ? 4 : 2, out, nullptr, out_dtype == KF_F32 ? 4 : 2, H)) {
+    if (!out || (w_dtype == KF_F32 && out_dtype == KF_F32)) KF_ROW(float, float);
+    else if (w_dtype == KF_BF16 && out_dtype == KF_BF16) KF_ROW(__nv_bfloat16, __nv_bfloat16);
+    else if (w_dtype == KF_BF16 && out_dtype == KF_F32) KF_ROW(__nv_bfloat16, float);
+    else if (w_dtype == KF_F32 && out_dtype == KF_BF16) KF_ROW(float, __nv_bfloat16);
+    else return KF_ERR_DTYPE;
+    KF_CHECK_LAUNCH();
+    return KF_OK;
+  }
+#undef KF_ROW
   const int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
 #define KF_GO(TW, TO)                                                                                                   \
   kf_launch(add2_rmsnorm_kernel<TW, TO>, dim3(T), dim3(threads), 0, stream, a, b, x, (const TW*)w, eps, plus_one, (TO*)out, H)
