@@ -402,6 +402,11 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 // S = Q K^T (16 heads x 16 keys) and O += P V run on mma.sync with 32-bit accumulators, the online softmax is the
 // one of the prompt kernel.  Warps are merged through shared memory in warp order, splits by the last block.
 constexpr int DM_WARPS = 8;                       // two per scheduler: a warp's tile is one chain of dependent instructions
+// More (row, kv head) pairs than blocks of eight warps fit the GPU, and short rows: a block then is mostly its start and its
+// merge, and blocks of four warps, two to an SM at heads of 256, cover each other's.  64 rows of 8 heads over 4 of 256, alone:
+// 64 keys 22.6 -> 16.4 us, 256 keys 30.8 -> 24.6, 577 keys 49.2 either way, 1,024 keys 67.6 -> 69.6.
+constexpr int DM_WARPS_SHORT = 4;
+constexpr int DM_KEYS_SHORT = 512;
 constexpr int DM_BUFS = 3;                        // buffers of one key tile or one value tile per warp: one in use, two in flight
 constexpr int DM_KEYS = 16;                       // keys per warp tile
 
@@ -413,7 +418,7 @@ constexpr int DM_KEYS = 16;                       // keys per warp tile
 //
 // SIG: no softmax.  Key j counts with sigmoid(s_j + sig_bias[h]) and the weights are not normalized: the weighted sum is
 // what is stored.  In the merges this is a maximum of 0 everywhere and a sum of 1 that the first split holds.
-template <int D, bool SIG>
+template <int D, bool SIG, int DM_WARPS>
 __global__ void __launch_bounds__(DM_WARPS * 32)
 attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restrict__ qkv, const float* __restrict__ cos_t,
                        const float* __restrict__ sin_t, int rot, int write_kv, __nv_bfloat16* pages,
@@ -770,14 +775,14 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
 
 // Blocks of the tensor-core decode kernel that one SM holds at a time (shared memory or registers, whichever binds), as
 // the runtime reports it; also sets the kernel's shared-memory limit.  0 if that fails.
-template <int D, bool SIG>
+template <int D, bool SIG, int DM_WARPS>
 int decode_mma_blocks_per_sm() {
   static int cached = -1;
   if (cached >= 0) return cached;
   const size_t smem = (size_t)(16 * D + DM_WARPS * DM_BUFS * DM_KEYS * D) * 2;
   int n = 0;
-  if (cudaFuncSetAttribute(attn_decode_mma_kernel<D, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_decode_mma_kernel<D, SIG>, DM_WARPS * 32, smem) != cudaSuccess) {
+  if (cudaFuncSetAttribute(attn_decode_mma_kernel<D, SIG, DM_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_decode_mma_kernel<D, SIG, DM_WARPS>, DM_WARPS * 32, smem) != cudaSuccess) {
     kf_record_cuda_error(cudaGetLastError());
     return 0;
   }
@@ -785,20 +790,36 @@ int decode_mma_blocks_per_sm() {
   return n;
 }
 
+template <int D, bool SIG, int DM_WARPS>
+int launch_decode_mma_warps(const float* qkv, const float* cos_t, const float* sin_t, int rot, int write_kv,
+                      const void* q, const void* pages, const int* items, int n_items, const int* positions,
+                      const int* row_req, const int* table, int table_stride, int page_size, int nh, int nkv, float scale,
+                      float softcap, int window, int vsplit, int keep_first, int sink, const float* sig_bias, int n_splits,
+                      float* partial, int* counters, void* out, cudaStream_t stream) {
+  const size_t smem = (size_t)(16 * D + DM_WARPS * DM_BUFS * DM_KEYS * D) * 2;
+  if (decode_mma_blocks_per_sm<D, SIG, DM_WARPS>() < 1) return KF_ERR_SETUP;
+  kf_launch(attn_decode_mma_kernel<D, SIG, DM_WARPS>, dim3(n_items * nkv, n_splits), dim3(DM_WARPS * 32), smem, stream,
+            (const __nv_bfloat16*)q, qkv, cos_t, sin_t, rot, write_kv, (__nv_bfloat16*)const_cast<void*>(pages), items, n_items,
+            positions, row_req, table, table_stride, page_size, nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias, n_splits,
+            partial, counters, (__nv_bfloat16*)out);
+  KF_CHECK_LAUNCH();
+  return KF_OK;
+}
+
+// n_splits 0: one split in blocks of DM_WARPS_SHORT warps.
 template <int D, bool SIG>
 int launch_decode_mma(const float* qkv, const float* cos_t, const float* sin_t, int rot, int write_kv,
                       const void* q, const void* pages, const int* items, int n_items, const int* positions,
                       const int* row_req, const int* table, int table_stride, int page_size, int nh, int nkv, float scale,
                       float softcap, int window, int vsplit, int keep_first, int sink, const float* sig_bias, int n_splits,
                       float* partial, int* counters, void* out, cudaStream_t stream) {
-  const size_t smem = (size_t)(16 * D + DM_WARPS * DM_BUFS * DM_KEYS * D) * 2;
-  if (decode_mma_blocks_per_sm<D, SIG>() < 1) return KF_ERR_SETUP;
-  kf_launch(attn_decode_mma_kernel<D, SIG>, dim3(n_items * nkv, n_splits), dim3(DM_WARPS * 32), smem, stream,
-            (const __nv_bfloat16*)q, qkv, cos_t, sin_t, rot, write_kv, (__nv_bfloat16*)const_cast<void*>(pages), items, n_items,
-            positions, row_req, table, table_stride, page_size, nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias, n_splits,
-            partial, counters, (__nv_bfloat16*)out);
-  KF_CHECK_LAUNCH();
-  return KF_OK;
+  if (n_splits == 0)
+    return launch_decode_mma_warps<D, SIG, DM_WARPS_SHORT>(
+        qkv, cos_t, sin_t, rot, write_kv, q, pages, items, n_items, positions, row_req, table, table_stride, page_size,
+        nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias, 1, partial, counters, out, stream);
+  return launch_decode_mma_warps<D, SIG, DM_WARPS>(
+        qkv, cos_t, sin_t, rot, write_kv, q, pages, items, n_items, positions, row_req, table, table_stride, page_size,
+        nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias, n_splits, partial, counters, out, stream);
 }
 
 template <int D, int HT>
@@ -834,20 +855,22 @@ static int g_forced_splits = 0;
 KF_API void kf_set_attention_decode_splits(int splits) { g_forced_splits = splits; }
 #endif
 
+// splits_out: how many parts a row's keys are cut into; 0 for one part in blocks of fewer warps (short rows, more of them than
+// the GPU holds blocks), which kf_attention_decode (ht = 0) and kf_attention_decode_fused take as it is.
 KF_API int kf_attention_decode_mma_plan(int n_items, int nh, int nkv, int d, int max_keys, int* splits_out) {
   if (g_forced_splits > 0) { *splits_out = g_forced_splits; return KF_OK; }
   const long blocks = (long)n_items * nkv;
   // fill one wave: as many splits as resident blocks allow
-  long per_sm = d == 256 ? decode_mma_blocks_per_sm<256, false>() : d == 128 ? decode_mma_blocks_per_sm<128, false>()
-              : d == 64 ? decode_mma_blocks_per_sm<64, false>() : d == 32 ? decode_mma_blocks_per_sm<32, false>()
-              : d == 16 ? decode_mma_blocks_per_sm<16, false>() : 0;
+  long per_sm = d == 256 ? decode_mma_blocks_per_sm<256, false, DM_WARPS>() : d == 128 ? decode_mma_blocks_per_sm<128, false, DM_WARPS>()
+              : d == 64 ? decode_mma_blocks_per_sm<64, false, DM_WARPS>() : d == 32 ? decode_mma_blocks_per_sm<32, false, DM_WARPS>()
+              : d == 16 ? decode_mma_blocks_per_sm<16, false, DM_WARPS>() : 0;
   if (per_sm > 8) per_sm = 8;
   if (per_sm < 1) per_sm = 1;
   int splits = (int)((kf_sm_count() * per_sm) / blocks);
   const int by_len = (max_keys + 255) / 256;
   if (splits > by_len) splits = by_len;
   if (splits > 64) splits = 64;
-  if (splits < 1) splits = 1;
+  if (splits < 1) splits = blocks > kf_sm_count() * per_sm && max_keys <= DM_KEYS_SHORT ? 0 : 1;
   *splits_out = splits;
   return KF_OK;
 }
@@ -880,7 +903,7 @@ KF_API int kf_attention_decode(const void* q, void* out, const void* pages, cons
   if (n_items <= 0) return KF_OK;
   if ((keep_first > 0 || sink || sig_bias) && ht != 0) return KF_ERR_SIZE;   // kept first tokens, the sink, sigmoid weights: tensor-core variant only
   if (window <= 0) keep_first = 0;
-  if (nkv < 1 || nh % nkv != 0 || page_size < 1 || n_splits < 1 || !kf_head_map_ok(nh, nkv, vsplit)) return KF_ERR_SIZE;
+  if (nkv < 1 || nh % nkv != 0 || page_size < 1 || n_splits < (ht == 0 ? 0 : 1) || !kf_head_map_ok(nh, nkv, vsplit)) return KF_ERR_SIZE;
   if (n_splits > 1 && (!partial || !counters)) return KF_ERR_SIZE;
   if (n_splits > MERGE_MAX_SPLITS || ht > MERGE_MAX_HEADS) return KF_ERR_SIZE;
   if (ht == 0) {                                     // tensor-core variant
@@ -919,7 +942,7 @@ KF_API int kf_attention_decode_fused(const float* qkv, const float* cos_t, const
                                      float softcap, int window, int n_splits, float* partial, int* counters,
                                      cudaStream_t stream) {
   if (n_items <= 0) return KF_OK;
-  if (!qkv || nkv < 1 || nh % nkv != 0 || nh / nkv > 16 || page_size < 1 || n_splits < 1) return KF_ERR_SIZE;
+  if (!qkv || nkv < 1 || nh % nkv != 0 || nh / nkv > 16 || page_size < 1 || n_splits < 0) return KF_ERR_SIZE;
   if (rot < 0 || rot > d || (rot & 1) || (rot > 0 && (!cos_t || !sin_t))) return KF_ERR_SIZE;
   if (n_splits > 1 && (!partial || !counters)) return KF_ERR_SIZE;
   if (n_splits > MERGE_MAX_SPLITS) return KF_ERR_SIZE;
