@@ -228,15 +228,19 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(KfDeltaArgs p, cons
 
 // Steps of single rows (decoding): one token per request, bound by the bytes of the states.  A block of 32 * LANES threads
 // owns (request, head, 32 value columns): a warp has NR rows of S, a lane a column, so that a row's 32 numbers are one
-// 128-byte access (the walk's lanes hold rows, two columns to a warp).  The states are requested before the grid dependency
-// is waited for (nothing in the step writes them before), and the vectors of `delta_prepare_kernel` are made here, without
-// scratch or a launch of their own.  Every sum has the order of the two kernels above (a lane's four interleaved partial
+// 128-byte access (the walk's lanes hold rows, two columns to a warp).  With `early` the states are requested before the
+// grid dependency is waited for (the caller says that nothing ahead in the stream that may still be running writes them),
+// and the vectors of `delta_prepare_kernel` are made here, without scratch or a launch of their own.  Every sum has the order of the two kernels above (a lane's four interleaved partial
 // sums, the butterfly over the lanes as a tree, the shares of o one after the other), so that a token gives the same bits.
 // Measured in place (16 heads x 128 x 128, eight requests): preparation and walk 22 us of a layer -> 8 us.
 template <int NR, int LANES, typename TW>
-__global__ void __launch_bounds__(32 * LANES) delta_step_kernel(KfDeltaArgs p) {
+__global__ void __launch_bounds__(32 * LANES) delta_step_kernel(KfDeltaArgs p, int early) {
   constexpr int DP = NR * LANES;
   kf_pdl_trigger();
+  if (!early) {
+    kf_pdl_wait();
+    p.state = kf_produced(p.state);
+  }
   __shared__ float q_s[DP], k_s[DP], g_s[DP], norm_s[2], small_s[2];
   __shared__ float part[2][LANES][32];
   const int req = blockIdx.x / p.H, h = blockIdx.x - req * p.H;
@@ -337,12 +341,12 @@ __global__ void __launch_bounds__(32 * LANES) delta_step_kernel(KfDeltaArgs p) {
 }
 
 template <typename TW>
-static void delta_step_launch(const KfDeltaArgs& p, cudaStream_t s) {
+static void delta_step_launch(const KfDeltaArgs& p, int early, cudaStream_t s) {
   const dim3 grid(p.n_reqs * p.H, kf_ceil_div(p.dv, 32));
-  if (p.d <= 32) kf_launch(delta_step_kernel<8, 4, TW>, grid, dim3(128), 0, s, p);
-  else if (p.d <= 64) kf_launch(delta_step_kernel<8, 8, TW>, grid, dim3(256), 0, s, p);
-  else if (p.d <= 128) kf_launch(delta_step_kernel<8, 16, TW>, grid, dim3(512), 0, s, p);
-  else kf_launch(delta_step_kernel<16, 16, TW>, grid, dim3(512), 0, s, p);
+  if (p.d <= 32) kf_launch(delta_step_kernel<8, 4, TW>, grid, dim3(128), 0, s, p, early);
+  else if (p.d <= 64) kf_launch(delta_step_kernel<8, 8, TW>, grid, dim3(256), 0, s, p, early);
+  else if (p.d <= 128) kf_launch(delta_step_kernel<8, 16, TW>, grid, dim3(512), 0, s, p, early);
+  else kf_launch(delta_step_kernel<16, 16, TW>, grid, dim3(512), 0, s, p, early);
 }
 
 // Rows per thread, lanes per column and threads per block by key size: few rows per thread, because one long prompt has
@@ -364,12 +368,13 @@ KF_API int kf_delta_rule_row_floats(int d) {
 }
 
 // d up to 256 key channels, any dv.  `single`: no request of the step has more than one row (the step kernel, which needs
-// no scratch); otherwise prep holds T * H * kf_delta_rule_row_floats(d) floats (16-byte aligned), small T * H * 2 floats.
+// no scratch; early: it may read the states before the kernels ahead have finished); otherwise prep holds
+// T * H * kf_delta_rule_row_floats(d) floats (16-byte aligned), small T * H * 2 floats.
 KF_API int kf_delta_rule(const float* qkv, int ld_qkv, int q0, int k0, int v0, const float* beta, int ld_beta, int beta0,
                          const float* decay, int ld_decay, int decay0, int per_channel, const void* dt_bias, const void* a_log,
                          int w_dtype, float* state, float* out, int ld_out, int H, int KH, int d, int dv, int n_reqs,
                          const int* req_row_start, const int* req_n_rows, const int* req_state_slot, int writes, int T,
-                         float* prep, float* small, int single, cudaStream_t stream) {
+                         float* prep, float* small, int single, int early, cudaStream_t stream) {
   if (n_reqs <= 0 || T <= 0) return KF_OK;
   if (d < 1 || d > 256 || dv < 1 || H < 1 || KH < 1 || H % KH) return KF_ERR_SIZE;
   if (w_dtype != KF_F32 && w_dtype != KF_BF16) return KF_ERR_DTYPE;
@@ -377,8 +382,8 @@ KF_API int kf_delta_rule(const float* qkv, int ld_qkv, int q0, int k0, int v0, c
   KfDeltaArgs p{qkv, ld_qkv, q0, k0, v0, beta, ld_beta, beta0, decay, ld_decay, decay0, per_channel, dt_bias, a_log,
                 state, out, ld_out, H, KH, d, dv, n_reqs, req_row_start, req_n_rows, req_state_slot, writes};
   if (single) {
-    if (w_dtype == KF_F32) delta_step_launch<float>(p, stream);
-    else delta_step_launch<__nv_bfloat16>(p, stream);
+    if (w_dtype == KF_F32) delta_step_launch<float>(p, early, stream);
+    else delta_step_launch<__nv_bfloat16>(p, early, stream);
     KF_CHECK_LAUNCH();
     return KF_OK;
   }

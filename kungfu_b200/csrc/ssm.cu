@@ -260,17 +260,22 @@ __global__ void ssm_chunk_fold_kernel(const float* __restrict__ state, float* __
   }
 }
 
-// One row per request (decoding): nothing is staged; every thread fetches its states (before the grid dependency is waited
-// for: nothing else in the step writes them), then its part of B and C and the row's x and dt straight from global memory.  Same split of the work and the same order of sums
-// as the walk above, so a token gives the same bits whether it came alone or in a portion.
+// One row per request (decoding): nothing is staged; every thread fetches its states, then its part of B and C and the
+// row's x and dt straight from global memory.  With `early` the states are requested before the grid dependency is waited
+// for: the caller says that nothing ahead in the stream that may still be running writes them.  Same split of the work and
+// the same order of sums as the walk above, so a token gives the same bits whether it came alone or in a walked portion.
 template <int K4, typename TW>
 __global__ void __launch_bounds__(SSM_THREADS)
 ssm_step_kernel(const float* xbc, int ld_x, const float* proj, int ld_p, int dt_col0,
                 const TW* __restrict__ dt_bias, const TW* __restrict__ a_log, const TW* __restrict__ d_skip,
                 float* state, float* __restrict__ y, int heads, int groups, int P, int N,
                 int n_reqs, const int* __restrict__ req_row_start, const int* __restrict__ req_n_rows,
-                const int* __restrict__ req_state_slot, int write_state, int vec) {
+                const int* __restrict__ req_state_slot, int write_state, int vec, int early) {
   kf_pdl_trigger();
+  if (!early) {
+    kf_pdl_wait();
+    state = kf_produced(state);
+  }
   const int req = blockIdx.x / heads, h = blockIdx.x - req * heads;
   if (req >= n_reqs || req_n_rows[req] <= 0) return;
   const int t = req_row_start[req], slot = req_state_slot[req];
@@ -304,7 +309,7 @@ ssm_step_kernel(const float* xbc, int ld_x, const float* proj, int ld_p, int dt_
       }
   }
   const float a = -expf(kf_load(a_log, h)), bias = kf_load(dt_bias, h), dsk = kf_load(d_skip, h);
-  kf_pdl_wait();                                            // the step's integers and the states were there before the step
+  kf_pdl_wait();
   xbc = kf_produced(xbc), proj = kf_produced(proj);
   const float* row = xbc + (size_t)t * ld_x;
   if (vec) {
@@ -387,10 +392,11 @@ static void ssm_launch_walk(dim3 grid, cudaStream_t stream, const float* xbc, in
 #undef KF_GO2
 }
 
+// single_rows: no request has more than one row; early: the states may then be read before the kernels ahead have finished.
 KF_API int kf_ssm_scan(const float* xbc, int ld_x, const float* proj, int ld_p, int dt_col0, const void* dt_bias,
                        const void* a_log, const void* d_skip, int w_dtype, float* state, float* y, int heads, int groups,
                        int P, int N, int n_reqs, const int* req_row_start, const int* req_n_rows,
-                       const int* req_state_slot, int write_state, int single_rows, cudaStream_t stream) {
+                       const int* req_state_slot, int write_state, int single_rows, int early, cudaStream_t stream) {
   if (n_reqs <= 0) return KF_OK;
   if (N < 1 || N > SSM_MAX_N || P < 1 || heads < 1 || groups < 1 || heads % groups) return KF_ERR_SIZE;
   if (w_dtype != KF_F32 && w_dtype != KF_BF16) return KF_ERR_DTYPE;
@@ -401,7 +407,7 @@ KF_API int kf_ssm_scan(const float* xbc, int ld_x, const float* proj, int ld_p, 
 #define KF_STEP(K4, TW)                                                                                                 \
   kf_launch(ssm_step_kernel<K4, TW>, grid, block, 0, stream, xbc, ld_x, proj, ld_p, dt_col0, (const TW*)dt_bias,         \
             (const TW*)a_log, (const TW*)d_skip, state, y, heads, groups, P, N, n_reqs, req_row_start, req_n_rows,      \
-            req_state_slot, write_state, (vec && (((uintptr_t)state) & 15) == 0) ? 1 : 0)
+            req_state_slot, write_state, (vec && (((uintptr_t)state) & 15) == 0) ? 1 : 0, early)
 #define KF_GO(TW)                                  \
   do {                                             \
     if (N <= 32) KF_STEP(1, TW);                   \

@@ -67,6 +67,11 @@ def _align4(n: int) -> int:
 class StepContext:
     """Everything parts may read during one step.  Integer arrays live on the device."""
 
+    # The step's integers are copied in by a stream operation that waits for every kernel before it, and a schedule has one
+    # writing call per cache slot, before any that only reads (`DecoderModel`): the call that moves a fixed state on finds it
+    # as the step before left it, however early it looks.
+    states_settled = True
+
     def __init__(self, runner: "Runner"):
         self._runner = runner
         self.act_dtype = runner.act_dtype

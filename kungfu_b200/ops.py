@@ -626,6 +626,15 @@ def rope_append_attend(qkv, cos, sin, rot: int, out, ctx, cache, n_heads: int, n
 _CONV_ACT = {None: 0, "none": 0, "silu": 1}
 
 
+def _state_settled(ctx, writes: bool) -> int:
+    """1: the kernel of a step of single rows may read its fixed states before the kernels ahead of it in the stream have
+    finished.  That holds for the one call of a step that moves a state on, under a context that says that states were
+    last written before the step (`StepContext.states_settled`).  A call that only reads comes after the one that writes,
+    and contexts made elsewhere say nothing: their kernels wait first, as every kernel does before it reads what another
+    one may be writing."""
+    return int(bool(writes) and bool(getattr(ctx, "states_settled", False)))
+
+
 @_dispatch("short_conv")
 def short_conv(proj, col0: int, in_bias, weight, out_bias, act, state, out, ctx, commit_inline: bool = False) -> bool:
     """out[t, c] = act(sum_j weight[c, j] * u_(t - taps + 1 + j)[c] + out_bias[c]) over the rows of every request of the step,
@@ -638,7 +647,8 @@ def short_conv(proj, col0: int, in_bias, weight, out_bias, act, state, out, ctx,
     inline = bool(commit_inline) and taps > 1
     _check(library().kf_short_conv(_p(proj), proj.shape[1], int(col0), _p(in_bias), _p(weight), _p(out_bias), _dt(weight), C,
                                    taps, _CONV_ACT[act], _p(state), _p(out), out.shape[1], _p(ctx.row_req),
-                                   _p(ctx.req_row_start), _p(ctx.req_state_slot), T, int(inline), _stream()), "short_conv")
+                                   _p(ctx.req_row_start), _p(ctx.req_state_slot), T, int(inline), _state_settled(ctx, inline), _stream()),
+           "short_conv")
     return inline
 
 
@@ -763,7 +773,7 @@ def ssm_scan(xbc, proj, dt_col0: int, dt_bias, a_log, d_skip, state, y, heads: i
                "ssm_scan (chunks side by side)")
         add_launches(3)
         return
-    _check(lib.kf_ssm_scan(*common, int(single), _stream()), "ssm_scan")
+    _check(lib.kf_ssm_scan(*common, int(single), _state_settled(ctx, writes), _stream()), "ssm_scan")
 
 
 @_dispatch("gated_group_norm")
@@ -907,7 +917,7 @@ def delta_rule(qkv, q0: int, k0: int, v0: int, beta, beta0: int, decay, decay0: 
                              _p(decay), decay.shape[1], int(decay0), int(bool(per_channel)), _p(dt_bias), _p(a_log),
                              _dt(a_log), _p(state), _p(out), out.shape[1], heads, kv_heads, dim, vdim, ctx.n_reqs,
                              _p(ctx.req_row_start), _p(ctx.req_n_rows), _p(ctx.req_state_slot), int(writes), T, _p(prep),
-                             _p(small), int(single), _stream()), "delta_rule")
+                             _p(small), int(single), _state_settled(ctx, writes), _stream()), "delta_rule")
     if not single:
         add_launches(1)
 
