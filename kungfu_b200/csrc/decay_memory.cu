@@ -40,6 +40,7 @@ struct DecayArgs {
   int writes;
   const float* cos; const float* sin; int rot;       // 0: nothing is turned
   float kscale;
+  int early;                                          // decay_decode_kernel: the state may be read before the kernels ahead have finished
 };
 
 // Element i of a head of q or k at row t: activated, then turned.
@@ -61,6 +62,10 @@ constexpr int DD_THREADS = 256;
 template <typename T, int NR>                          // NR rows of the state per thread: d <= 32 NR
 __global__ void __launch_bounds__(DD_THREADS) decay_decode_kernel(DecayArgs p) {
   kf_pdl_trigger();
+  if (!p.early) {
+    kf_pdl_wait();
+    p.state = kf_produced(p.state);
+  }
   __shared__ float qs[32 * NR], ks[32 * NR];
   __shared__ __align__(16) float vs[DD_COLS];
   __shared__ __align__(16) float4 red[8][8];
@@ -74,7 +79,7 @@ __global__ void __launch_bounds__(DD_THREADS) decay_decode_kernel(DecayArgs p) {
   const bool live = col < p.dv;                        // dv is a multiple of four
   float* S = p.state + ((size_t)p.slot[r] * p.H + h) * p.d * p.dv + col;
   const float a = p.powers[(size_t)h * p.n_powers + 1];
-  float4 s[NR];                                        // an earlier step left the state: readable at once
+  float4 s[NR];
 #pragma unroll
   for (int j = 0; j < NR; ++j) {
     const int row = r0 + 32 * j;
@@ -584,11 +589,12 @@ KF_API int kf_decay_rotate(const float* in, int ld, int q0, int k0, int v0, cons
 
 // rows: the base of the matrix that holds q, k and v in columns q0, k0, v0 (`ld` columns); dtype: its element type.
 // chunk_rows > 0 (a multiple of 64, below n_powers): chunks side by side; chunk_state then holds n_numbers * H * d * dv
-// floats, n_numbers at least the number of chunks of the step.  single: no request has more than one row.
+// floats, n_numbers at least the number of chunks of the step.  single: no request has more than one row; early: the states
+// may then be read before the kernels ahead in the stream have finished.
 KF_API int kf_decay_memory(const void* rows, int dtype, int ld, int q0, int k0, int v0, int act, const float* powers,
                            int n_powers, float* state, float* out, int H, int d, int dv, int n_reqs, const int* row_start,
                            const int* n_rows, const int* slot, int writes, int single, int chunk_rows, int n_numbers,
-                           float* chunk_state, const float* cos, const float* sin, int rot, float kscale, cudaStream_t stream) {
+                           float* chunk_state, const float* cos, const float* sin, int rot, float kscale, int early, cudaStream_t stream) {
   if (n_reqs <= 0) return KF_OK;
   if (rot < 0 || rot > d || (rot & 1) || (rot && (!cos || !sin))) return KF_ERR_SIZE;
   if (d < 1 || d > 256 || dv < 1 || H < 1 || n_powers < DC_ROWS + 1) return KF_ERR_SIZE;
@@ -596,7 +602,7 @@ KF_API int kf_decay_memory(const void* rows, int dtype, int ld, int q0, int k0, 
   const size_t es = dtype == KF_F32 ? 4 : 2;
   const char* base = (const char*)rows;
   DecayArgs p{base + q0 * es, base + k0 * es, base + v0 * es, ld, ld, ld, act, powers, n_powers, state, out, H, d, dv, n_reqs,
-              row_start, n_rows, slot, writes, cos, sin, rot, kscale};
+              row_start, n_rows, slot, writes, cos, sin, rot, kscale, early};
   if (single && dv % 4 == 0 && (((uintptr_t)state | (uintptr_t)out) & 15) == 0) {
     const dim3 grid((unsigned)((long)n_reqs * H * kf_ceil_div(dv, DD_COLS)));
 #define KF_GO(NR)                                                                                               \

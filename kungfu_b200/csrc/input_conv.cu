@@ -166,17 +166,23 @@ input_conv_kernel(const float* __restrict__ x, const TW* __restrict__ w, float* 
   }
 }
 
-// One block per row, every request of the step with at most one row: the row, its tail and the filters in registers.
+// One block per row, every request of the step with at most one row: the row, its tail and the filters in registers.  With
+// `early` the tail is requested before the grid dependency is waited for: nothing ahead in the stream that may still be
+// running writes it, says the caller.
 template <typename TW, typename TO, int TAPS, int NPT>
 __global__ void __launch_bounds__(512)
 add_rmsnorm_conv_kernel(const float* a, const TW* __restrict__ w1, float eps, float* x, const TW* __restrict__ w,
                         float* state, TO* __restrict__ out, int H, const int* __restrict__ row_req,
-                        const int* __restrict__ req_state_slot, int writes) {
+                        const int* __restrict__ req_state_slot, int writes, int early) {
   kf_pdl_trigger();
+  if (!early) {
+    kf_pdl_wait();
+    state = kf_produced(state);
+  }
   __shared__ float red[33];
   constexpr int TAIL = TAPS - 1;
   const int r = blockIdx.x;
-  const int req = row_req[r];                          // the step's integers, weights and earlier steps' tails: readable at once
+  const int req = row_req[r];                          // the step's integers and the weights: readable at once
   float g[NPT], wv[NPT][TAPS], tail[NPT][TAIL > 0 ? TAIL : 1];
   float* st = state + (size_t)(req >= 0 ? req_state_slot[req] : 0) * TAIL * H;
 #pragma unroll
@@ -262,14 +268,14 @@ KF_API int kf_add_rmsnorm_conv_supported(int H, int taps) { return H >= 1 && H <
 
 KF_API int kf_add_rmsnorm_conv(const float* a, const void* w1, const void* w, int w_dtype, float eps, float* x, int taps,
                                float* state, void* out, int out_dtype, const int* row_req, const int* req_state_slot, int T,
-                               int H, int writes, cudaStream_t stream) {
+                               int H, int writes, int early, cudaStream_t stream) {
   if (T <= 0) return KF_OK;
   if (!kf_add_rmsnorm_conv_supported(H, taps) || (taps > 1 && !state)) return KF_ERR_SIZE;
   const int threads = H > 1024 ? 512 : (H >= 512 ? 256 : 128);
   const int npt = kf_ceil_div(H, threads);
 #define KF_LAUNCH(TW, TO, TAPS, NPT)                                                                                   \
   kf_launch(add_rmsnorm_conv_kernel<TW, TO, TAPS, NPT>, dim3(T), dim3(threads), 0, stream, a, (const TW*)w1, eps, x, \
-            (const TW*)w, state, (TO*)out, H, row_req, req_state_slot, writes)
+            (const TW*)w, state, (TO*)out, H, row_req, req_state_slot, writes, early)
 #define KF_PICK(TW, TO, TAPS)                                                                                         \
   do {                                                                                                                \
     if (npt <= 4) KF_LAUNCH(TW, TO, TAPS, 4);                                                               \

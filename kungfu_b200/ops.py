@@ -1065,7 +1065,7 @@ def add_rmsnorm_conv(branch, weight, eps: float, residual, conv_weight, state, o
         return False
     _check(lib.kf_add_rmsnorm_conv(_p(branch), _p(weight), _p(conv_weight), _dt(weight), _f(eps), _p(residual),
                                    int(conv_weight.shape[1]), _p(state), _p(out), _dt(out), _p(ctx.row_req),
-                                   _p(ctx.req_state_slot), T, H, int(writes), _stream()), "add_rmsnorm_conv")
+                                   _p(ctx.req_state_slot), T, H, int(writes), _state_settled(ctx, writes), _stream()), "add_rmsnorm_conv")
     return True
 
 
@@ -1127,7 +1127,8 @@ def decay_memory(rows, q0: int, k0: int, v0: int, act, powers, state, out, heads
     _check(lib.kf_decay_memory(_p(rows), _dt(rows), rows.shape[1], int(q0), int(k0), int(v0), int(act == "silu"), _p(powers),
                                powers.shape[1], _p(state), _p(out), heads, dim, vdim, ctx.n_reqs, _p(ctx.req_row_start),
                                _p(ctx.req_n_rows), _p(ctx.req_state_slot), int(writes), int(single), chunk_rows, n_numbers,
-                               _p(chunk_state), _p(cos), _p(sin), int(rot), _f(key_scale), _stream()), "decay_memory")
+                               _p(chunk_state), _p(cos), _p(sin), int(rot), _f(key_scale), _state_settled(ctx, writes), _stream()),
+           "decay_memory")
     if chunk_rows:
         add_launches(2)
 

@@ -7,6 +7,7 @@ import torch
 
 import bolonex_cases as bx
 import helpers
+import lurisun_cases as lu
 import petanex_cases as px
 
 gpu = pytest.mark.gpu
@@ -18,6 +19,8 @@ class _Recorder:
 
     def __getattr__(self, name):
         def call(*args):
+            if name.endswith("_supported"):
+                return 1
             self.last = (name, args)
             return 0
         return call
@@ -30,7 +33,9 @@ def _calls(ops, ctx, writes):
     out = []
     for run in (lambda: ops.ssm_scan(f(2, 24), f(2, 4), 0, f(2), f(2), f(2), f(2, 2, 4, 8), f(2, 8), 2, 1, 4, 8, ctx, writes),
                 lambda: ops.delta_rule(f(2, 24), 0, 8, 16, f(2, 2), 0, f(2, 2), 0, False, f(2), f(2), f(2, 2, 4, 4), f(2, 8), 2, 2, 4, 4, ctx, writes),
-                lambda: ops.short_conv(f(2, 8), 0, None, f(8, 3), None, "silu", f(2, 2, 8), f(2, 8), ctx, commit_inline=writes)):
+                lambda: ops.short_conv(f(2, 8), 0, None, f(8, 3), None, "silu", f(2, 2, 8), f(2, 8), ctx, commit_inline=writes),
+                lambda: ops.decay_memory(f(2, 24), 0, 8, 16, None, f(2, 513), f(2, 2, 4, 4), f(2, 8), 2, 4, 4, ctx, writes),
+                lambda: ops.add_rmsnorm_conv(f(2, 8), f(8), 1e-5, f(2, 8), f(8, 3), f(2, 2, 8), f(2, 8), ctx, writes)):
         run()
         out.append(lib.last)
     return out
@@ -54,7 +59,7 @@ def test_states_are_read_early_only_by_the_writer_of_a_step(monkeypatch, writes,
     for name, args in _calls(ops, ctx, writes):
         names.add(name)
         assert args[-1] == "stream" and args[-2] == int(writes and settled is True), name
-    assert names == {"kf_ssm_scan", "kf_delta_rule", "kf_short_conv"}
+    assert names == {"kf_ssm_scan", "kf_delta_rule", "kf_short_conv", "kf_decay_memory", "kf_add_rmsnorm_conv"}
 
 
 def test_a_step_says_that_its_states_are_settled():
@@ -68,7 +73,7 @@ def test_a_step_says_that_its_states_are_settled():
 
 
 @gpu
-@pytest.mark.parametrize("family,kind", [("bolonex", "Mamba2Mixer"), ("petanex", "GatedDeltaMixer")])
+@pytest.mark.parametrize("family,kind", [("bolonex", "Mamba2Mixer"), ("petanex", "GatedDeltaMixer"), ("lurisun", "LightningAttention")])
 @pytest.mark.parametrize("graphs", [False, True])
 def test_a_second_call_that_only_reads(tmp_path, family, kind, graphs):
     """The schedule runs a recurrent layer a second time on the same slot without writing: prompts of unequal length, then
@@ -76,8 +81,7 @@ def test_a_second_call_that_only_reads(tmp_path, family, kind, graphs):
     from kungfu_b200 import api, ops
     from kungfu_b200.engine import StepEntry
     from kungfu_b200.parts.model import DecoderModel, LayerCall
-    cases = bx if family == "bolonex" else px
-    cfg_dict = bx.BX_E if family == "bolonex" else px.PX_E
+    cases, cfg_dict = {"bolonex": (bx, bx.BX_E), "petanex": (px, px.PX_E), "lurisun": (lu, lu.LU_E)}[family]
     folder = cases.write_model(str(tmp_path / "m"), cfg_dict, seed=4)
     toks = {f"r{i}": helpers.random_tokens(n + 12, cfg_dict["vocab"], 50 + i) for i, n in enumerate((3, 40, 9))}
     runs = []
