@@ -57,3 +57,31 @@ def test_blocks_against_64_bits(heads, groups, P, N, rows, rate):
             assert bool(((y[t].cpu().double().view(heads, P) - want).abs() <= bound).all()), t
         assert bool(((dev[slot].cpu().double() - S).abs() <= 300 * 2.0 ** -24 * size + 1e-30).all())
         at += r
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("row", [0, 31, 32, 70, 127, 128, 299])
+def test_what_is_not_finite_stays_in_its_column_and_does_not_travel_back(row, bad):
+    """One number of x that is not finite, at edges of bands and blocks: earlier rows, other columns, other heads and the other
+    request keep their bits."""
+    from kungfu_b200 import ops
+    heads, groups, P, N, rows, slots = 3, 1, 68, 36, (300, 130), [2, 0]
+    g = torch.Generator().manual_seed(row)
+    T, inner = sum(rows), heads * P
+    x, pr = torch.randn(T, inner + 2 * N, generator=g), torch.randn(T, heads, generator=g)
+    a_log, dt_bias, D = -1 + torch.rand(heads, generator=g), torch.randn(heads, generator=g) - 1, torch.randn(heads, generator=g)
+    state = torch.randn(4, heads, P, N, generator=g)
+    res = []
+    for poison in (False, True):
+        v, dev, y = x.clone(), state.to(DEV), torch.empty(T, inner, device=DEV)
+        if poison:
+            v[row, P + 5] = bad                                       # head 1, column 5
+        ops.ssm_scan(v.to(DEV), pr.to(DEV), 0, dt_bias.to(DEV), a_log.to(DEV), D.to(DEV), dev, y, heads, groups, P, N, _step(rows, slots))
+        res.append((y.view(T, heads, P).cpu(), dev.cpu()))
+    (y0, s0), (y1, s1) = res
+    hit = torch.zeros(T, heads, P, dtype=torch.bool)
+    hit[row:rows[0], 1, 5] = True
+    assert torch.equal(y0[~hit], y1[~hit]) and not bool(torch.isfinite(y1[row, 1, 5]))
+    hit = torch.zeros(4, heads, P, N, dtype=torch.bool)
+    hit[slots[0], 1, 5] = True
+    assert torch.equal(s0[~hit], s1[~hit]) and not bool(torch.isfinite(s1[hit]).any())
