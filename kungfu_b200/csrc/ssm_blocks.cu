@@ -11,12 +11,13 @@
 //   1. per (block, head): the block's own contribution to the state at its end; per (block, group): the table C_t . B_s;
 //   2. the states at the blocks' starts, one after the other from the request's stored state, which takes the last one;
 //   3. per (block, head): y.
-// All arithmetic is 32-bit (packed FMAs, 8 x 8 outputs per thread); the running sums of log decays are kept as a pair of
-// floats rounded from 64-bit sums, so that exp(la_t - la_s) does not lose what the sums have in common.
+// All products are 32-bit (packed FMAs, 8 x 8 outputs per thread); the running sums of log decays are kept as a pair of
+// floats rounded from 64-bit sums, so that exp(la_t - la_s) does not lose what the sums have in common, and C_t . B_s is summed
+// in 64 bits eight products at a time, because its error is that of every term inside a block.
 // What bounds them is the FMA pipe (2.8 G multiply-adds at 2,048 rows of 64 heads x 64 x 128) at the rate that shared-memory
 // reads leave it; the states between the kernels stay in L2.  One prompt of 2,048 rows: the walk 592 us, in chunks side by
-// side 435 us, this 208 us with a cold L2 (60 + 9 + 126 us in place); error of y against 64 bits 1.2e-7 (the walk 1.0e-7 to
-// 1.7e-7 over 128 to 2,048 rows, one to eight requests), of the state 6e-8 to 1.1e-7 (8e-8 to 2.0e-7).
+// side 435 us, this 210 us with a cold L2.  Errors against 64 bits (2-norms; 128 to 2,048 rows, one to eight requests, decays of
+// e^-0.01 to e^-3 a row): of y 6.9e-8 to 9.9e-8 (the walk 7.5e-8 to 2.9e-6), of the state 4.7e-8 to 1.5e-7 (4.9e-8 to 3.9e-6).
 #include "common.cuh"
 
 namespace {
@@ -97,62 +98,72 @@ __global__ void __launch_bounds__(THREADS, 2) ssm_block_state_kernel(const Args 
   const int tx = (lane & 7) + 8 * (warp & 1), ty = (lane >> 3) + 4 * (warp >> 1);      // 16 x 8 threads
   const int cr = tid >> 3, cc = (tid & 7) * 4;                  // this thread copies rows cr + 16 i, four columns from cc + 32 j on
   int job = blockIdx.y;
-  if (job < 2 * p.groups) {
-    // the table of a group: rows t of one half of the block, all s (half 0 needs s < 64 only; the rest is never read)
-    const int g = job >> 1, half = job & 1;
-    if (64 * half >= rows) return;
+  if (job < 3 * p.groups) {
+    // The table of a group, 64 rows t x 64 columns s a job: (t, s) halves (0, 0), (1, 0) and (1, 1); nothing reads (0, 1).
+    // Eight products at a time are summed in 32 bits, as four even and four odd states, and those sums in 64 bits: every
+    // term of y that is made inside a block has one of these numbers in it.
+    const int g = job / 3, th = (job % 3 + 1) >> 1, sh = job % 3 >> 1;
+    if (64 * th >= rows) return;
     float* Cs = sm;                                             // [64][LD]
-    float* Bs = sm + 64 * LD;                                   // [128][LD]
+    float* Bs = sm + 64 * LD;                                   // [64][LD]
     const float* b0 = p.xbc + inner + g * N;
     const float* c0 = b0 + p.groups * N;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int n = cc + 32 * j;
 #pragma unroll
-      for (int r = cr; r < L; r += 16) {
-        const bool in = n < N && r < rows;
-        cp16(Bs + r * LD + n, in ? b0 + (size_t)(row0 + r) * p.ld_x + n : p.xbc, in);
-      }
-#pragma unroll
       for (int r = cr; r < 64; r += 16) {
-        const int t = 64 * half + r;
-        const bool in = n < N && t < rows;
-        cp16(Cs + r * LD + n, in ? c0 + (size_t)(row0 + t) * p.ld_x + n : p.xbc, in);
+        const int t = 64 * th + r, s = 64 * sh + r;
+        const bool in_b = n < N && s < rows, in_c = n < N && t < rows;
+        cp16(Bs + r * LD + n, in_b ? b0 + (size_t)(row0 + s) * p.ld_x + n : p.xbc, in_b);
+        cp16(Cs + r * LD + n, in_c ? c0 + (size_t)(row0 + t) * p.ld_x + n : p.xbc, in_c);
       }
       commit();
     }
-    pair_t acc[8][8];
+    double sum[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+      for (int j = 0; j < 4; ++j) sum[i][j] = 0.;
     auto slice = [&](int s) {
-      for (int k = 32 * s; k < min(N, 32 * s + 32); k += 4) {
-        ulonglong2 a[8];
+      for (int k0 = 32 * s; k0 < min(N, 32 * s + 32); k0 += 8) {
+        pair_t acc[8][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(Cs + (ty + 8 * i) * LD + k);
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(Bs + (tx + 16 * j) * LD + k);
+          for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].x, b.x);
+        for (int k = k0; k < k0 + 8; k += 4) {                  // columns from N on are zeros
+          ulonglong2 a[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].y, b.y);
+          for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(Cs + (ty + 8 * i) * LD + k);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(Bs + (tx + 16 * j) * LD + k);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].x, b.x);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].y, b.y);
+          }
         }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) sum[i][j] += (double)lo_of(acc[i][j]) + (double)hi_of(acc[i][j]);
       }
     };
     wait_groups<3>(); __syncthreads(); slice(0);
     wait_groups<2>(); __syncthreads(); slice(1);
     wait_groups<1>(); __syncthreads(); slice(2);
     wait_groups<0>(); __syncthreads(); slice(3);
-    float* out = p.table + ((size_t)blk * p.groups + g) * L * L + (size_t)64 * half * L;
+    float* out = p.table + ((size_t)blk * p.groups + g) * L * L + (size_t)64 * th * L + 64 * sh;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) out[(ty + 8 * i) * L + tx + 16 * j] = lo_of(acc[i][j]) + hi_of(acc[i][j]);
+      for (int j = 0; j < 4; ++j) out[(ty + 8 * i) * L + tx + 16 * j] = (float)sum[i][j];
     return;
   }
-  job -= 2 * p.groups;
+  job -= 3 * p.groups;
   const int ptiles = (P + PT - 1) / PT, h = job / ptiles, pb = job % ptiles * PT, g = h / (p.heads / p.groups);
   float* Bs = sm;                                               // [128][NMAX]
   float* Xs = sm + L * NMAX;                                    // [128][PT]
@@ -491,7 +502,7 @@ int launch(const Args& a, cudaStream_t s) {
   if (e1 != cudaSuccess || e2 != cudaSuccess) { kf_record_cuda_error(e1 != cudaSuccess ? e1 : e2); return KF_ERR_SETUP; }
   const int ptiles = kf_ceil_div(a.P, PT), PN = a.P * a.N;
   // without the programmatic-dependent-launch attribute: blocks of 100 KB that wait would keep the kernel before them off the SMs
-  ssm_block_state_kernel<TW><<<dim3(a.max_blocks, 2 * a.groups + a.heads * ptiles), THREADS, SMEM, s>>>(a);
+  ssm_block_state_kernel<TW><<<dim3(a.max_blocks, 3 * a.groups + a.heads * ptiles), THREADS, SMEM, s>>>(a);
   kf_launch(ssm_block_fold_kernel, dim3(a.n_reqs, a.heads, kf_ceil_div(PN, 1024)), dim3(256), 0, s, a);
   ssm_block_out_kernel<TW><<<dim3(a.max_blocks, a.heads * ptiles), THREADS, SMEM, s>>>(a);
   KF_CHECK_LAUNCH();
@@ -504,7 +515,7 @@ int launch(const Args& a, cudaStream_t s) {
 KF_API int kf_ssm_blocks_rows() { return L; }
 KF_API int kf_ssm_blocks_supported(const float* xbc, int ld_x, const float* state, int heads, int groups, int P, int N) {
   return N >= 4 && N <= NMAX && N % 4 == 0 && P % 4 == 0 && ld_x % 4 == 0 && groups >= 1 && heads % groups == 0 &&
-         (((uintptr_t)xbc | (uintptr_t)state) & 15) == 0 && 2L * groups + (long)heads * kf_ceil_div(P, PT) <= 65535;
+         (((uintptr_t)xbc | (uintptr_t)state) & 15) == 0 && 3L * groups + (long)heads * kf_ceil_div(P, PT) <= 65535;
 }
 
 // As kf_ssm_scan.  Scratch from the caller, with max_blocks >= rows / 128 + n_reqs: `list` 2 * max_blocks + 2 * n_reqs ints,

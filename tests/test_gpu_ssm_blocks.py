@@ -85,3 +85,34 @@ def test_what_is_not_finite_stays_in_its_column_and_does_not_travel_back(row, ba
     hit = torch.zeros(4, heads, P, N, dtype=torch.bool)
     hit[slots[0], 1, 5] = True
     assert torch.equal(s0[~hit], s1[~hit]) and not bool(torch.isfinite(s1[hit]).any())
+
+
+@pytest.mark.parametrize("rate", [-1.0, 0.5, 2.0])
+@pytest.mark.parametrize("rows", [(192,), (512,), (100, 300)])
+def test_blocks_are_no_further_from_64_bits_than_the_walk(rows, rate, monkeypatch):
+    """The same rows by both routes, errors of y and of the state as 2-norms over all heads; decays from e^-0.1 to e^-7 a row.
+    (Measured: y 0.75 to 0.95 of the walk's error, the state 0.6 to 1.0; the bound leaves room for another draw.)"""
+    from kungfu_b200 import ops
+    heads, P, N = 16, 64, 128
+    g = torch.Generator().manual_seed(sum(rows))
+    T, inner = sum(rows), heads * P
+    x = torch.nn.functional.silu(torch.randn(T, inner + 2 * N, generator=g)).to(DEV)
+    pr = torch.randn(T, heads, generator=g).to(DEV)
+    a_log, dt_bias, D = (rate + torch.rand(heads, generator=g)).to(DEV), (torch.randn(heads, generator=g) - 2).to(DEV), torch.randn(heads, generator=g).to(DEV)
+    state = torch.randn(len(rows), heads, P, N, generator=g).to(DEV)
+    want_y, want_s = torch.empty(T, heads, P, dtype=torch.float64, device=DEV), state.double()
+    dt = torch.nn.functional.softplus(pr.double() + dt_bias.double())
+    decay, xs, at = torch.exp(-torch.exp(a_log.double()) * dt), x.double(), 0
+    for r, n in enumerate(rows):
+        for t in range(at, at + n):
+            v = xs[t, :inner].view(heads, P)
+            want_s[r] = decay[t][:, None, None] * want_s[r] + (dt[t][:, None] * v)[:, :, None] * xs[t, inner:inner + N]
+            want_y[t] = torch.einsum("hpn,n->hp", want_s[r], xs[t, inner + N:]) + D.double()[:, None] * v
+        at += n
+    err = {}
+    for blocks in (True, False):
+        monkeypatch.setattr(ops, "SCAN_BLOCKS_FROM", 1 if blocks else T + 1)
+        dev, y = state.clone(), torch.empty(T, inner, device=DEV)
+        ops.ssm_scan(x, pr, 0, dt_bias, a_log, D, dev, y, heads, 1, P, N, _step(list(rows), list(range(len(rows)))))
+        err[blocks] = (float((y.view(T, heads, P).double() - want_y).norm()), float((dev.double() - want_s).norm()))
+    assert err[True][0] <= 1.1 * err[False][0] and err[True][1] <= 1.15 * err[False][1], err
