@@ -160,6 +160,7 @@ attention_generic_kernel(const TQ* __restrict__ q, TQ* __restrict__ out, const T
           }
         }
         float pv[2];
+        bool see[2];
         bool all = true;                                    // every pair sees every key of the run
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
@@ -167,6 +168,7 @@ attention_generic_kernel(const TQ* __restrict__ q, TQ* __restrict__ out, const T
           const bool mine = s_row[p] >= 0 && row >= a && row < b;
           const bool seen = mine && j <= s_pos[p] && (j >= s_lo[p] || j < s_kept[p]);
           all = all && (s_row[p] < 0 || seen);
+          see[u] = seen;
           const float sum = (lo_of(dot[u][0]) + hi_of(dot[u][0])) + (lo_of(dot[u][1]) + hi_of(dot[u][1]));
           const float s = seen ? kf_softcap(sum * scale, softcap) : -INFINITY;
           float corr = 1.f;
@@ -182,7 +184,8 @@ attention_generic_kernel(const TQ* __restrict__ q, TQ* __restrict__ out, const T
           }
           if (lane == 0) s_corr[p] = corr;
         }
-        *reinterpret_cast<float2*>(s_p + lane * PLD + p0) = make_float2(pv[0], pv[1]);
+        // a weight below zero marks a key that its pair does not see (a seen one's may have underflowed to zero)
+        *reinterpret_cast<float2*>(s_p + lane * PLD + p0) = make_float2(see[0] ? pv[0] : -1.f, see[1] ? pv[1] : -1.f);
         all = __syncthreads_and(all);                       // the keys are free, the weights are there
         copy(next, 0);
         asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -208,7 +211,8 @@ attention_generic_kernel(const TQ* __restrict__ q, TQ* __restrict__ out, const T
             }
           }
         } else {
-          // a key that a pair does not see is left out, not multiplied by zero: its value may be infinite
+          // A key that a pair does not see is left out, not multiplied by zero: its value may be infinite.  One that it sees
+          // is multiplied whatever its weight is, as above, so that a row's result does not depend on the block's other rows.
           for (int u = 0; u < RUN; ++u)
 #pragma unroll
             for (int i = 0; i < PAIRS; ++i) {
@@ -217,7 +221,7 @@ attention_generic_kernel(const TQ* __restrict__ q, TQ* __restrict__ out, const T
               for (int e = 0; e < DPT; ++e) {
                 const float v = de + e * DT < d ? Vs[u * ld + de + e * DT] : 0.f;
                 const float x = lo_of(acc[e][i]), y1 = hi_of(acc[e][i]);
-                acc[e][i] = pair_of(w0 != 0.f ? fmaf(w0, v, x) : x, w1 != 0.f ? fmaf(w1, v, y1) : y1);
+                acc[e][i] = pair_of(w0 < 0.f ? x : fmaf(w0, v, x), w1 < 0.f ? y1 : fmaf(w1, v, y1));
               }
             }
         }

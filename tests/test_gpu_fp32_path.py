@@ -97,3 +97,27 @@ def test_generic_attention(ops, nh, nkv, d, P, dtype, window, keep, sink):
     poisoned[table[1, 120 // P], 1, :, 120 % P] = float("inf")
     got = attend(list(range(len(rows))), poisoned.to(DEV))
     assert torch.equal(got[:25], whole[:25]) and not bool(got[25].isfinite().all())
+
+
+def test_a_seen_key_counts_the_same_beside_any_other_rows(ops):
+    """A key that a row sees with a weight below the smallest number, and whose value is infinite: the row holds what it holds
+    alone, also where its block walks rows that do not see the key."""
+    from test_gpu_kernels import _Ctx, _View, _paged_setup
+    nh, d, P = 16, 32, 16
+    pages, table, _, _ = _paged_setup(torch.float32, nh, nh, d, P, [41], seed=3)
+    pages[table[0, 0], 0, :, 5] = -30.0                               # q is all ones: a score of -170 at position 5
+    pages[table[0, 0], 1, :, 5, 3] = float("inf")
+    dev_pages, dev_table = pages.to(DEV), table.to(DEV)
+    places = [40 if i % 2 else 4 for i in range(200)]                 # enough rows for blocks of several
+
+    def attend(at):
+        ctx = _Ctx(torch.tensor(at, dtype=torch.int32, device=DEV), torch.zeros(len(at), dtype=torch.int32, device=DEV), dev_table)
+        out = torch.empty(len(at), nh * d, device=DEV)
+        ops.paged_attention(torch.ones(len(at), nh * d, device=DEV), out, ctx, _View(dev_pages, P), nh, nh, d, d ** -0.5, 0.0, None)
+        return out.view(len(at), nh, d)
+
+    low, high = attend([4])[0], attend([40])[0]
+    assert bool(low.isfinite().all()) and not bool(high[:, 3].isfinite().any()) and bool(high[:, 4:].isfinite().all())
+    together = attend(places)
+    for i, p in enumerate(places):
+        assert torch.equal(together[i].nan_to_num(7.0), (high if p == 40 else low).nan_to_num(7.0)), i
