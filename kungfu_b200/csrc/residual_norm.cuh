@@ -8,7 +8,8 @@
 // sum costs one barrier (every warp adds the warps' sums itself).
 // The kernel is bound by latency at a few rows and by bytes at many.  A few rows (`kf_residual_norm_threads`) take a thread
 // per vector; many rows take four vectors a thread, so that an SM holds six or more rows at different stages of this chain
-// where eight rows of two blocks, in step with one another, left the memory idle in turns.
+// where eight rows of two blocks, in step with one another, left the memory idle in turns.  The order of a row's sums is a
+// function of H alone (`kf_row_sum`): a row has the same bits whatever else is in the step.
 // Measured in place (one B200), the kernels it took the place of -> this one: NORMED at 2,048 rows of 2,304 20 -> 14 us
 // (66 MB: 4.9 TB/s), SCALED at 8 rows of 2,048 4.5 -> 1.8 us, PLAIN at 8 rows 4.9 -> 2.1 us and at 2,048 rows 19 -> 14 us.
 #pragma once
@@ -37,13 +38,36 @@ __device__ __forceinline__ void kf_put4(__nv_bfloat16* o, float4 v) {
   *reinterpret_cast<uint2*>(o) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 
-// the block's sum in every thread, warps in a fixed order; `red` holds 32 floats and is used for one sum only
-__device__ __forceinline__ float kf_row_sum(float v, float* red) {
-  const int lane = threadIdx.x & 31;
-  v = kf_warp_sum(v);
-  if (lane == 0) red[threadIdx.x >> 5] = v;
+__device__ __forceinline__ float kf_square4(float4 v) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x))); }
+
+// The block's sum of a row of which thread t holds vectors t, t + blockDim.x, ...: part[k] is what vector t + k * blockDim.x
+// adds.  In every thread; `red` holds 32 floats and is used for one sum only.  Up to 1,024 vectors the sum has one order for
+// both thread counts: 32 neighbouring vectors as a tree, then those sums as another.  With four vectors a thread (256 threads
+// at most) a warp makes its four trees together: lanes 8 k .. 8 k + 7 go on with tree k after two exchanges.  Rows of more
+// vectors always have four a thread, which are added first.
+template <int NV>
+__device__ __forceinline__ float kf_row_sum(const float (&part)[NV], float* red) {
+  static_assert(NV == 1 || NV == 4, "a vector per thread or four");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int n = blockDim.x >> 5;
+  if (NV == 4 && blockDim.x <= 256) {
+    const bool h16 = lane & 16, h8 = lane & 8;
+    const float a = (h16 ? part[NV / 2] : part[0]) + __shfl_xor_sync(0xffffffffu, h16 ? part[0] : part[NV / 2], 16);
+    const float b = (h16 ? part[NV - 1] : part[NV / 4]) + __shfl_xor_sync(0xffffffffu, h16 ? part[NV / 4] : part[NV - 1], 16);
+    float v = (h8 ? b : a) + __shfl_xor_sync(0xffffffffu, h8 ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((lane & 7) == 0) red[warp + (lane >> 3) * n] = v;
+    n *= 4;
+  } else {
+    float v = part[0];
+#pragma unroll
+    for (int k = 1; k < NV; ++k) v += part[k];
+    v = kf_warp_sum(v);
+    if (lane == 0) red[warp] = v;
+  }
   __syncthreads();
-  return kf_warp_sum(lane < ((blockDim.x + 31) >> 5) ? red[lane] : 0.f);
+  return kf_warp_sum(lane < n ? red[lane] : 0.f);
 }
 
 template <int MODE, typename TW1, typename TW2, typename TO, int NV, int MAXT>
@@ -82,31 +106,32 @@ residual_norm_kernel(const float* a, const float* b, const TW1* __restrict__ w1,
   }
   float inv = 1.f;
   if (MODE == KF_RES_NORMED) {
-    float ss = 0.f;
+    float ss[NV];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
-    inv = 1.f / sqrtf(kf_row_sum(ss, red1) / (float)H + eps1);
+    for (int k = 0; k < NV; ++k) ss[k] = kf_square4(v[k]);
+    inv = 1.f / sqrtf(kf_row_sum<NV>(ss, red1) / (float)H + eps1);
   }
   const float p1 = plus1 ? 1.f : 0.f;
-  float ss = 0.f;
+  float ss[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     const int i = 4 * (threadIdx.x + k * blockDim.x);
+    ss[k] = 0.f;
     if (i < H) {
       if (MODE == KF_RES_PLAIN) {
         v[k] = make_float4(v[k].x + xv[k].x, v[k].y + xv[k].y, v[k].z + xv[k].z, v[k].w + xv[k].w);
       } else {
         const float4 g = r1[k].get();
-        v[k] = make_float4(xv[k].x + v[k].x * inv * (g.x + p1), xv[k].y + v[k].y * inv * (g.y + p1), xv[k].z + v[k].z * inv * (g.z + p1),
-                           xv[k].w + v[k].w * inv * (g.w + p1));
+        v[k] = make_float4(fmaf(v[k].x * inv, g.x + p1, xv[k].x), fmaf(v[k].y * inv, g.y + p1, xv[k].y),
+                           fmaf(v[k].z * inv, g.z + p1, xv[k].z), fmaf(v[k].w * inv, g.w + p1, xv[k].w));
       }
       kf_put4(x + base + i, v[k]);
       if (copy != nullptr) kf_put4(copy + base + i, v[k]);
-      ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+      ss[k] = kf_square4(v[k]);
     }
   }
   if (out == nullptr) return;
-  const float inv2 = plus2 == 2 ? 1.f : 1.f / sqrtf(kf_row_sum(ss, red2) / (float)H + eps2);
+  const float inv2 = plus2 == 2 ? 1.f : 1.f / sqrtf(kf_row_sum<NV>(ss, red2) / (float)H + eps2);
   const float p2 = plus2 ? 1.f : 0.f;
 #pragma unroll
   for (int k = 0; k < NV; ++k) {

@@ -40,3 +40,28 @@ def test_branch_and_next_norm(T, H, wd, od, mode):
     assert float(out[T].float().min()) == 3.0
     if mode == "scaled":
         assert torch.equal(copy.cpu(), dx.cpu().to(od))
+
+
+# one warp of vectors, ragged and whole warps, 1,024 vectors, more than those, and no whole vectors
+@pytest.mark.parametrize("H", [4, 132, 2048, 2304, 4096, 4100, 130])
+@pytest.mark.parametrize("mode", ["normed", "scaled", "plain2", "gated"])
+def test_a_row_has_the_same_bits_in_steps_of_255_and_256_rows(H, mode):
+    import types
+    from kungfu_b200 import ops
+    g = torch.Generator().manual_seed(H)
+    a, b, x = (torch.randn(256, H, generator=g).to(DEV) for _ in range(3))
+    w1, w2 = torch.randn(H, generator=g).to(DEV), torch.randn(H, generator=g).to(DEV)
+    got = []
+    for T in (255, 256):
+        dx, out = x[:T].clone(), torch.empty(T, H, device=DEV)
+        nxt = dict(next_weight=w2, next_eps=1e-5, next_plus_one=True, next_out=out)
+        if mode == "normed":
+            ops.add_rmsnorm(a[:T], w1, 1e-6, True, dx, **nxt)
+        elif mode == "scaled":
+            ops.scale_add_rmsnorm(a[:T], w1, dx, **nxt)
+        elif mode == "plain2":
+            ops.add2_rmsnorm(a[:T], b[:T], dx, **nxt)
+        else:
+            ops.gated_group_norm(a[:T], b[:T], 0, w1, 1e-5, 1, out, types.SimpleNamespace(row_req=torch.zeros(T, dtype=torch.int32, device=DEV)))
+        got.append((dx[:255], out[:255]))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
