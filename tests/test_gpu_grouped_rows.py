@@ -17,11 +17,13 @@ class _Ctx:
         return torch.empty(shape, dtype=dtype, device=DEV)
 
 
-# tokens 1..33 cross the counts of row tiles (8, 16, 32) and the rule's line; with T = 60 over 40 experts the mean is small and
-# one expert has every token (60 rows: two passes); N and K off the tiles of 32 features, 64 features and 64 k
+# tokens 1..33 cross the counts of row tiles (8, 16, 32) and the rule's line; with T = 60 and 100 over more experts the mean is
+# small and one expert has every token (60 rows: eight row tiles; 100: two tiles of the plan); N and K off the tiles of 32
+# features, 64 features and 64 k
 @pytest.mark.parametrize("T,E,top,N,K,out", [(1, 4, 1, 33, 72, "bfloat16"), (8, 32, 3, 256, 2048, "bfloat16"), (9, 8, 2, 100, 64, "float32"),
                                              (16, 3, 2, 64, 136, "float32"), (17, 5, 2, 31, 200, "bfloat16"), (32, 2, 1, 96, 8, "float32"),
-                                             (33, 64, 2, 40, 328, "bfloat16"), (60, 40, 2, 70, 264, "float32"), (33, 2, 2, 70, 264, "float32")])
+                                             (33, 64, 2, 40, 328, "bfloat16"), (60, 40, 2, 70, 264, "float32"), (100, 64, 2, 70, 264, "bfloat16"),
+                                             (33, 2, 2, 70, 264, "float32")])
 @pytest.mark.parametrize("gated", [False, True])
 def test_few_rows_per_expert(ops, T, E, top, N, K, out, gated):
     g = torch.Generator().manual_seed(T + N)
@@ -54,6 +56,25 @@ def test_few_rows_per_expert(ops, T, E, top, N, K, out, gated):
     if not gated:
         ops.moe_linear(x[pair // top].to(DEV), plan, w.to(DEV), again, gather=False)
         assert torch.equal(again, got[:-1])
+
+
+@pytest.mark.parametrize("T", [1, 9, 20, 30])
+@pytest.mark.parametrize("gated", [False, True])
+def test_a_row_has_the_same_bits_in_a_step_of_few_rows_and_of_many(ops, T, gated):
+    """The first T of 70 tokens over two experts, alone (streamed weights) and in the whole step (tiles of 64 rows)."""
+    g = torch.Generator().manual_seed(T)
+    E, N, K = 2, 70, 264
+    ids = torch.randint(0, E, (70, 1), generator=g).to(torch.int32)
+    x = torch.randn(70, K, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(E, 2 * N if gated else N, K, generator=g) * K ** -0.5).to(torch.bfloat16).to(DEV)
+    got = {}
+    for n in (T, 70):
+        plan = ops.moe_plan(ids[:n].to(DEV), E, _Ctx())
+        out = torch.empty(n, N, device=DEV)
+        ops.moe_linear(x[:n], plan, w, out, gather=True, gated=gated, limit=0.9)
+        got[n] = torch.empty_like(out)
+        got[n][plan["sorted_pair"].long()[:n]] = out
+    assert torch.equal(got[T], got[70][:T])
 
 
 @pytest.mark.parametrize("T", [1, 8, 9, 17, 32, 33])
