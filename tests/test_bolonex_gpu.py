@@ -250,7 +250,9 @@ def test_state_space_scan_in_portions(wdtype, heads, groups, P, N):
     assert float(state[1].min()) == 3.0 and float(y[-1].min()) == 5.0
 
 
-@pytest.mark.parametrize("heads,groups,P,N", [(2, 1, 16, 16), (3, 3, 12, 10), (4, 2, 64, 128)])
+# the first three sizes would run as products over blocks of rows (but for the second, whose states are no whole vectors);
+# more than 128 states always come here
+@pytest.mark.parametrize("heads,groups,P,N", [(2, 1, 16, 16), (3, 3, 12, 10), (4, 2, 64, 128), (2, 1, 16, 132), (1, 1, 8, 256)])
 def test_long_portions_walked_in_chunks_side_by_side(heads, groups, P, N, monkeypatch):
     """Steps of many rows cut the recurrence into chunks (states at the chunks' starts from a first pass).
     Requests of 700, 1 and 130 rows and one of 128 exactly (chunks of 128 here), two of them with a state from before; against the same
@@ -266,16 +268,21 @@ def test_long_portions_walked_in_chunks_side_by_side(heads, groups, P, N, monkey
     proj = torch.randn(st.n_rows, ld_p, generator=g).to(DEV)
     state0 = torch.randn(4, heads, P, N, generator=g).to(DEV)
     state0[[2, 1]] = 0.0
-    out = {}
+    out, asked, buf = {}, set(), st.buf
+    st.buf = lambda tag, shape, dtype: (asked.add(tag), buf(tag, shape, dtype))[1]
     for chunked in (False, True):
         monkeypatch.setattr(ops, "chunked_scan", chunked)
         monkeypatch.setattr(ops, "SCAN_CHUNKED_FROM", 512)
         monkeypatch.setattr(ops, "SCAN_CHUNK_ROWS", 128)
+        if N <= 128:
+            monkeypatch.setattr(ops, "SCAN_BLOCKS_FROM", st.n_rows + 1)
         state = state0.clone()
         y = torch.full((st.n_rows, inner), 7.0, device=DEV)
+        asked.clear()
         before = ops.launch_count()
         ops.ssm_scan(xbc, proj, dt0, dt_bias, a_log, d_skip, state, y, heads, groups, P, N, st)
         assert ops.launch_count() - before == (4 if chunked else 1)
+        assert asked == ({"ssm_chunk_table", "ssm_chunk_state", "ssm_chunk_decay"} if chunked else set())      # the way it went
         out[chunked] = (y, state)
     scale = float(out[False][0][:-1].abs().max())
     assert float((out[True][0][:-1] - out[False][0][:-1]).abs().max()) / scale < 2e-5

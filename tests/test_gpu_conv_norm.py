@@ -14,12 +14,14 @@ DEV = "cuda:0"
 @pytest.mark.parametrize("taps", [1, 2, 4, 8])
 @pytest.mark.parametrize("rows", [(1, 1, 1), (5, 0, 2, 9), (70, 3, 1, 17), (1030, 6)])
 @pytest.mark.parametrize("bias", [False, True])
-def test_short_conv(C, taps, rows, bias):
+@pytest.mark.parametrize("wdtype", [torch.float32, torch.bfloat16])
+def test_short_conv(C, taps, rows, bias, wdtype):
     from kungfu_b200 import ops
     g = torch.Generator().manual_seed(C + taps + len(rows))
     T, ld, col0 = sum(rows) + 2, C + 8, 4
     x, w = torch.randn(T, ld, generator=g), torch.randn(C, taps, generator=g)
     ib, ob = (torch.randn(C, generator=g), torch.randn(C, generator=g)) if bias else (None, None)
+    w, ib, ob = (None if t is None else t.to(wdtype) for t in (w, ib, ob))
     state = torch.randn(6, max(taps - 1, 1), C, generator=g)
     ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
     starts, slots, req = [sum(rows[:i]) for i in range(len(rows))], [4, 0, 2, 5][:len(rows)], []

@@ -24,13 +24,15 @@ def _step(rows, slots):
 @pytest.mark.parametrize("heads,groups,P,N,rows", [(2, 1, 64, 128, (300, 0, 128)), (4, 2, 64, 128, (200, 1, 127)), (3, 3, 12, 20, (400,)),
                                                    (2, 1, 68, 36, (130, 257)), (1, 1, 132, 4, (500,)), (2, 2, 4, 100, (256, 192))])
 @pytest.mark.parametrize("rate", [-4.0, 1.0, 5.0])
-def test_blocks_against_64_bits(heads, groups, P, N, rows, rate):
+@pytest.mark.parametrize("wdtype", [torch.float32, torch.bfloat16])
+def test_blocks_against_64_bits(heads, groups, P, N, rows, rate, wdtype):
     from kungfu_b200 import ops
     g = torch.Generator().manual_seed(P + N + len(rows))
     T, inner = sum(rows), heads * P
     ld_x, ld_p, dt0 = inner + 2 * groups * N + 4, heads + 3, 2
     x, pr = torch.randn(T + 1, ld_x, generator=g), torch.randn(T + 1, ld_p, generator=g)
     a_log, dt_bias, D = rate + torch.rand(heads, generator=g), torch.randn(heads, generator=g) - 1, torch.randn(heads, generator=g)
+    a_log, dt_bias, D = a_log.to(wdtype), dt_bias.to(wdtype), D.to(wdtype)
     slots = [2, 0, 3][:len(rows)]
     state = torch.randn(4, heads, P, N, generator=g)
     dev = state.to(DEV)
@@ -116,3 +118,45 @@ def test_blocks_are_no_further_from_64_bits_than_the_walk(rows, rate, monkeypatc
         ops.ssm_scan(x, pr, 0, dt_bias, a_log, D, dev, y, heads, 1, P, N, _step(list(rows), list(range(len(rows)))))
         err[blocks] = (float((y.view(T, heads, P).double() - want_y).norm()), float((dev.double() - want_s).norm()))
     assert err[True][0] <= 1.1 * err[False][0] and err[True][1] <= 1.15 * err[False][1], err
+
+
+@pytest.mark.parametrize("rate", [-4.0, 0.0, 2.0])
+def test_one_prompt_by_every_route(rate):
+    """A prompt of 400 rows whole (blocks), in portions on both sides of the line (191 rows walked, 209 in blocks) and beside
+    single rows of other requests (the step's average is then below the line: walked): within rounding of one another."""
+    from kungfu_b200 import ops
+    heads, P, N, n, more = 2, 64, 128, 400, 4
+    g = torch.Generator().manual_seed(8)
+    inner, T = heads * P, n + more
+    x, pr = torch.randn(T, inner + 2 * N, generator=g), torch.randn(T, heads, generator=g)
+    a_log, dt_bias, D = rate + torch.rand(heads, generator=g), torch.randn(heads, generator=g) - 1, torch.randn(heads, generator=g)
+    state = torch.randn(1 + more, heads, P, N, generator=g)
+
+    def run(dev, lo, hi, others=0):
+        st = _step([hi - lo] + [1] * others, list(range(1 + others)))
+        asked, buf = [], st.buf
+        st.buf = lambda tag, shape, dtype: (asked.append(tag), buf(tag, shape, dtype))[1]
+        rows = list(range(lo, hi)) + list(range(n, n + others))
+        y = torch.empty(len(rows), inner, device=DEV)
+        ops.ssm_scan(x[rows].to(DEV), pr[rows].to(DEV), 0, dt_bias.to(DEV), a_log.to(DEV), D.to(DEV), dev, y, heads, 1, P, N, st)
+        return y[:hi - lo].cpu().double(), "ssm_block_state" in asked
+
+    got = []
+    for cuts, others, blocks in (([0, n], 0, [True]), ([0, 191, n], 0, [False, True]), ([0, n], more, [False])):
+        dev = state.to(DEV)
+        parts = [run(dev, a, b, others) for a, b in zip(cuts, cuts[1:])]
+        assert [went for _, went in parts] == blocks
+        got.append((torch.cat([y for y, _ in parts]), dev[0].cpu().double()))
+    # sizes of what is summed, in 64 bits
+    dt = torch.nn.functional.softplus(pr.double() + dt_bias.double())
+    decay = torch.exp(-torch.exp(a_log.double()) * dt)
+    size, y_size = state[0].double().abs(), torch.empty(n, inner, dtype=torch.float64)
+    for t in range(n):
+        xs = x[t, :inner].double().view(heads, P).abs()
+        size = decay[t][:, None, None] * size + (dt[t][:, None] * xs)[:, :, None] * x[t, inner:inner + N].double().abs()
+        y_size[t] = (torch.einsum("hpn,n->hp", size, x[t, inner + N:].double().abs()) + D.double().abs()[:, None] * xs).reshape(-1)
+    # N + 160 roundings of those on a block's route; a walked row's state has three a row for as long as it lasts, at most n rows
+    unit = 2.0 ** -24
+    for y, s in got[1:]:
+        assert bool(((y - got[0][0]).abs() <= 2 * (N + 160 + 3 * n) * unit * y_size).all())
+        assert bool(((s - got[0][1]).abs() <= 2 * (300 + 3 * n) * unit * size).all())
