@@ -259,14 +259,14 @@ static int grouped_mma_go(const KfGroupedArgs& p, int max_tiles, int n_groups, c
 //     three or four blocks per SM have 120 to 160 KB of weights on their way.
 // Shared rows are 128 bytes with their 16-byte chunks XOR-swizzled by the row.  A row's sums run over k in ascending order
 // and do not depend on the other rows, nor on which of the two kernels runs: the order over k is the same.  A tile with more
-// rows than 8 * NT takes several passes over its weights; with `passes` = 2 neighbouring blocks take every other one, so that
-// both read the same pieces at about the same time.
+// rows than 8 * NT takes several passes over its weights; with `two` = 1 neighbouring blocks take every other one, so that both
+// read the same pieces at about the same time.
 // Measured (one B200, experts of 2 x 2,048 x 2,048 and 2,048 x 2,048, eight tokens with three of 32 each, in place in a
 // decode step): gate and up 103 -> 49 us, down 80 -> 26 us, about 6.5 TB/s of the chosen experts' weights.
 constexpr int SWR = 64, SK = 64, SSTAGES = 6;
 
 template <typename TO, int GATED, int NT>
-__global__ void __launch_bounds__(128) grouped_stream_kernel(KfGroupedArgs p, int passes) {
+__global__ void __launch_bounds__(128) grouped_stream_kernel(KfGroupedArgs p, int two) {
   using namespace kf_mma;
   constexpr int ROWS = 8 * NT, STAGE = (SWR + ROWS) * SK, NOUT = GATED ? SWR / 2 : SWR;
   kf_pdl_trigger();
@@ -281,9 +281,9 @@ __global__ void __launch_bounds__(128) grouped_stream_kernel(KfGroupedArgs p, in
     g = blockIdx.z; r0 = 0; nrows = p.T;
   }
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
-  const int pass0 = blockIdx.x % passes * ROWS;
+  const int pass0 = ((int)blockIdx.x & two) * ROWS;
   if (pass0 >= nrows) return;
-  const int col0 = blockIdx.x / passes * NOUT, N = p.N, K = p.K, nk = (K + SK - 1) / SK;
+  const int col0 = (int)(blockIdx.x >> two) * NOUT, N = p.N, K = p.K, nk = (K + SK - 1) / SK;
   const __nv_bfloat16* x = (const __nv_bfloat16*)p.x + (size_t)g * p.x_gstride;
   const __nv_bfloat16* w = (const __nv_bfloat16*)p.w + (size_t)g * p.w_gstride;
   TO* out = (TO*)p.out + (size_t)g * p.o_gstride;
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(128) grouped_stream_kernel(KfGroupedArgs p, in
     wok[i] = feat < N;
     wsrc[i] = w + (wok[i] ? (size_t)(GATED && (r & 8) ? N + feat : feat) * K + ce : 0);
   }
-  for (int pass = pass0; pass < nrows; pass += passes * ROWS) {
+  for (int pass = pass0; pass < nrows; pass += ROWS << two) {
     const int here = min(ROWS, nrows - pass), tiles = (here + 7) >> 3;
     const __nv_bfloat16* xsrc[(NT + 1) / 2];
     bool xin[(NT + 1) / 2], xok[(NT + 1) / 2];
@@ -383,21 +383,21 @@ __global__ void __launch_bounds__(128) grouped_stream_kernel(KfGroupedArgs p, in
 }
 
 template <typename TO, int GATED, int NT>
-static int grouped_stream_launch(const KfGroupedArgs& p, int max_tiles, int n_groups, int passes, cudaStream_t s) {
+static int grouped_stream_launch(const KfGroupedArgs& p, int max_tiles, int n_groups, int two, cudaStream_t s) {
   auto kernel = grouped_stream_kernel<TO, GATED, NT>;
   constexpr int smem = SSTAGES * (SWR + 8 * NT) * SK * 2;
   const cudaError_t e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) { kf_record_cuda_error(e); return KF_ERR_SETUP; }
-  const dim3 grid(kf_ceil_div(p.N, GATED ? SWR / 2 : SWR) * passes, p.tile_group ? max_tiles : 1, p.tile_group ? 1 : n_groups);
-  kf_launch(kernel, grid, dim3(128), smem, s, p, passes);
+  const dim3 grid(kf_ceil_div(p.N, GATED ? SWR / 2 : SWR) << two, p.tile_group ? max_tiles : 1, p.tile_group ? 1 : n_groups);
+  kf_launch(kernel, grid, dim3(128), smem, s, p, two);
   KF_CHECK_LAUNCH();
   return KF_OK;
 }
 
 template <typename TO>
-static int grouped_stream_go(const KfGroupedArgs& p, int nt, int passes, int max_tiles, int n_groups, cudaStream_t s) {
-#define KF_NT(G) (nt == 1 ? grouped_stream_launch<TO, G, 1>(p, max_tiles, n_groups, passes, s) \
-                  : nt == 2 ? grouped_stream_launch<TO, G, 2>(p, max_tiles, n_groups, passes, s) : grouped_stream_launch<TO, G, 4>(p, max_tiles, n_groups, passes, s))
+static int grouped_stream_go(const KfGroupedArgs& p, int nt, int two, int max_tiles, int n_groups, cudaStream_t s) {
+#define KF_NT(G) (nt == 1 ? grouped_stream_launch<TO, G, 1>(p, max_tiles, n_groups, two, s) \
+                  : nt == 2 ? grouped_stream_launch<TO, G, 2>(p, max_tiles, n_groups, two, s) : grouped_stream_launch<TO, G, 4>(p, max_tiles, n_groups, two, s))
   return p.gated ? KF_NT(1) : KF_NT(0);
 #undef KF_NT
 }
@@ -438,9 +438,9 @@ KF_API int kf_grouped_linear(const void* x, int x_dtype, long x_off, long ldx, l
     // all on twelve, the worst found, 74 / 53 -> 82 / 43 (92 / 51).
     const int most = tile_group ? most_rows : T;
     if (x_dtype == KF_BF16 && (most <= 32 || (tile_group && T <= 16L * n_groups))) {
-      const int nt = most <= 8 ? 1 : most <= 16 ? 2 : 4, passes = most <= 32 ? 1 : 2;
-      if (out_dtype == KF_BF16) return grouped_stream_go<__nv_bfloat16>(p, nt, passes, max_tiles, n_groups, stream);
-      if (out_dtype == KF_F32) return grouped_stream_go<float>(p, nt, passes, max_tiles, n_groups, stream);
+      const int nt = most <= 8 ? 1 : most <= 16 ? 2 : 4, two = most > 32;
+      if (out_dtype == KF_BF16) return grouped_stream_go<__nv_bfloat16>(p, nt, two, max_tiles, n_groups, stream);
+      if (out_dtype == KF_F32) return grouped_stream_go<float>(p, nt, two, max_tiles, n_groups, stream);
     }
     if (x_dtype == KF_BF16 && out_dtype == KF_BF16) return grouped_mma_go<__nv_bfloat16, __nv_bfloat16>(p, max_tiles, n_groups, stream);
     if (x_dtype == KF_BF16 && out_dtype == KF_F32) return grouped_mma_go<__nv_bfloat16, float>(p, max_tiles, n_groups, stream);

@@ -12,6 +12,8 @@
 // function of H alone (`kf_row_sum`): a row has the same bits whatever else is in the step.
 // Measured in place (one B200), the kernels it took the place of -> this one: NORMED at 2,048 rows of 2,304 20 -> 14 us
 // (66 MB: 4.9 TB/s), SCALED at 8 rows of 2,048 4.5 -> 1.8 us, PLAIN at 8 rows 4.9 -> 2.1 us and at 2,048 rows 19 -> 14 us.
+// The one order of the sums costs 0.4 us at 2,048 rows and 0.1 us at 512 in a chain of such kernels (8.9 -> 9.3 us); vectors dealt
+// to the threads of a few rows so that both add up alike without exchanges cost those 0.35 us of 1.94 each.
 #pragma once
 #include "common.cuh"
 
@@ -41,16 +43,16 @@ __device__ __forceinline__ void kf_put4(__nv_bfloat16* o, float4 v) {
 __device__ __forceinline__ float kf_square4(float4 v) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x))); }
 
 // The block's sum of a row of which thread t holds vectors t, t + blockDim.x, ...: part[k] is what vector t + k * blockDim.x
-// adds.  In every thread; `red` holds 32 floats and is used for one sum only.  Up to 1,024 vectors the sum has one order for
-// both thread counts: 32 neighbouring vectors as a tree, then those sums as another.  With four vectors a thread (256 threads
+// adds.  In every thread; `red` holds 32 floats and is used for one sum only.  SHORT: at most 1,024 vectors; their sum has one
+// order for both thread counts: 32 neighbouring vectors as a tree, then those sums as another.  With four vectors a thread (256 threads
 // at most) a warp makes its four trees together: lanes 8 k .. 8 k + 7 go on with tree k after two exchanges.  Rows of more
 // vectors always have four a thread, which are added first.
-template <int NV>
+template <int NV, bool SHORT>
 __device__ __forceinline__ float kf_row_sum(const float (&part)[NV], float* red) {
   static_assert(NV == 1 || NV == 4, "a vector per thread or four");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int n = blockDim.x >> 5;
-  if (NV == 4 && blockDim.x <= 256) {
+  if (NV == 4 && SHORT) {
     const bool h16 = lane & 16, h8 = lane & 8;
     const float a = (h16 ? part[NV / 2] : part[0]) + __shfl_xor_sync(0xffffffffu, h16 ? part[0] : part[NV / 2], 16);
     const float b = (h16 ? part[NV - 1] : part[NV / 4]) + __shfl_xor_sync(0xffffffffu, h16 ? part[NV / 4] : part[NV - 1], 16);
@@ -109,7 +111,7 @@ residual_norm_kernel(const float* a, const float* b, const TW1* __restrict__ w1,
     float ss[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) ss[k] = kf_square4(v[k]);
-    inv = 1.f / sqrtf(kf_row_sum<NV>(ss, red1) / (float)H + eps1);
+    inv = 1.f / sqrtf(kf_row_sum<NV, NV == 1 || MAXT == 256>(ss, red1) / (float)H + eps1);
   }
   const float p1 = plus1 ? 1.f : 0.f;
   float ss[NV];
@@ -131,7 +133,7 @@ residual_norm_kernel(const float* a, const float* b, const TW1* __restrict__ w1,
     }
   }
   if (out == nullptr) return;
-  const float inv2 = plus2 == 2 ? 1.f : 1.f / sqrtf(kf_row_sum<NV>(ss, red2) / (float)H + eps2);
+  const float inv2 = plus2 == 2 ? 1.f : 1.f / sqrtf(kf_row_sum<NV, NV == 1 || MAXT == 256>(ss, red2) / (float)H + eps2);
   const float p2 = plus2 ? 1.f : 0.f;
 #pragma unroll
   for (int k = 0; k < NV; ++k) {

@@ -528,8 +528,8 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ y, const float
 // The same in whole vectors: NV of them per thread, the gains requested before the grid dependency is waited for, one
 // barrier.  One row of 4,096: 1,024 threads of a vector at a few rows, 256 of four at many, the sum in one order for both.
 // Measured in place: 8 rows 5.9 -> 3.2 us, 2,048 rows 33 -> 21 us.
-template <typename TW, typename TO, int NV>
-__global__ void __launch_bounds__(1024)
+template <typename TW, typename TO, int NV, int MAXT>
+__global__ void __launch_bounds__(MAXT)
 gated_group_norm_vec_kernel(const float* y, const float* z, int ld, int z_col0, const TW* __restrict__ w, float eps, int inner,
                             int parts, TO* __restrict__ out, const int* __restrict__ row_req) {
   kf_pdl_trigger();
@@ -562,7 +562,7 @@ gated_group_norm_vec_kernel(const float* y, const float* z, int ld, int z_col0, 
     v[k].z *= u[k].z / (1.f + expf(-u[k].z)); v[k].w *= u[k].w / (1.f + expf(-u[k].w));
     ss[k] = kf_square4(v[k]);
   }
-  const float inv = 1.f / sqrtf(kf_row_sum<NV>(ss, red) / (float)len + eps);
+  const float inv = 1.f / sqrtf(kf_row_sum<NV, NV == 1 || MAXT == 256>(ss, red) / (float)len + eps);
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     const int j = 4 * (threadIdx.x + k * blockDim.x);
@@ -585,9 +585,11 @@ KF_API int kf_gated_group_norm(const float* y, const float* z, int ld, int z_col
     const bool one = n4 <= 1024 && T < 256;
     const dim3 block((unsigned)(kf_ceil_div(one ? n4 : kf_ceil_div(n4, 4), 32) * 32));
 #define KF_VEC(TW, TO)                                                                                                  \
-    if (one) kf_launch(gated_group_norm_vec_kernel<TW, TO, 1>, dim3(T, parts), block, 0, stream, y, z, ld, z_col0, (const TW*)w, eps, \
-                       inner, parts, (TO*)out, row_req);                                                                \
-    else kf_launch(gated_group_norm_vec_kernel<TW, TO, 4>, dim3(T, parts), block, 0, stream, y, z, ld, z_col0, (const TW*)w, eps, \
+    if (one) kf_launch(gated_group_norm_vec_kernel<TW, TO, 1, 1024>, dim3(T, parts), block, 0, stream, y, z, ld, z_col0, (const TW*)w, \
+                       eps, inner, parts, (TO*)out, row_req);                                                           \
+    else if (n4 <= 1024) kf_launch(gated_group_norm_vec_kernel<TW, TO, 4, 256>, dim3(T, parts), block, 0, stream, y, z, ld, z_col0, \
+                                   (const TW*)w, eps, inner, parts, (TO*)out, row_req);                                 \
+    else kf_launch(gated_group_norm_vec_kernel<TW, TO, 4, 1024>, dim3(T, parts), block, 0, stream, y, z, ld, z_col0, (const TW*)w, eps, \
                    inner, parts, (TO*)out, row_req)
     if (w_dtype == KF_F32 && out_dtype == KF_F32) { KF_VEC(float, float); }
     else if (w_dtype == KF_BF16 && out_dtype == KF_BF16) { KF_VEC(__nv_bfloat16, __nv_bfloat16); }
