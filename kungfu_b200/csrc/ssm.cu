@@ -7,8 +7,9 @@
 //   y_t = S^T C_t + D[h] * x_t
 // x, B, C come from one 32-bit matrix (the output of the short convolution and its activation) laid out as
 // [ heads*P | groups*N | groups*N ] per row; dt_raw is a column range of the projection's 32-bit result.
-// The tokens of a request are walked in order, whatever the step holds of it (one token, a portion, a whole prompt),
-// so the result at a token does not depend on how the sequence was cut.
+// The kernels of this file walk the tokens of a request in order, whatever the step holds of it (one token, a portion, a whole
+// prompt), so the walk's result at a token does not depend on how the sequence was cut.  Long prompts take other routes (chunks
+// side by side, below, and the products of ssm_blocks.cu), chosen from the step's rows and requests: equal to rounding.
 //
 // Work split: a block of 128 threads owns (request, head, 32 values of p).  Thread (pl, ns) keeps S[n][p] for two values
 // of p and every n whose group of four, n / 4, is ns modulo 8: up to 64 numbers in registers, as pairs of neighbouring
