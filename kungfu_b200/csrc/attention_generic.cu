@@ -42,9 +42,11 @@ __device__ __forceinline__ float hi_of(unsigned long long v) { return __uint_as_
 // floats between rows in shared memory: rows of eight neighbouring keys start in different banks
 __host__ __device__ constexpr int row_pitch(int d) { return (d + 31) / 32 * 32 + 4; }
 
-// DT: threads along the head's elements (64, 128 or 256), DPT: elements per thread.
+// DT: threads along the head's elements (64, 128 or 256), DPT: elements per thread.  At heads of 256, where shared memory allows two
+// blocks per SM, the compiler is told so: left to itself it takes 79 registers and reads less ahead (eight rows of 2,048 keys
+// 490 us, with 128 registers 442; a step of 97 and 60 rows 51 -> 45).  Below, its own choice of 62 to 64 is the better one.
 template <typename TQ, typename TKV, int DT, int DPT>
-__global__ void __launch_bounds__(ATHREADS)
+__global__ void __launch_bounds__(ATHREADS, DT == 256 ? 2 : 0)
 attention_generic_kernel(const TQ* __restrict__ q, TQ* __restrict__ out, const TKV* __restrict__ pages,
                          const int* __restrict__ items, const int* __restrict__ positions,
                          const int* __restrict__ row_req, const int* __restrict__ block_table, int table_stride,
@@ -213,17 +215,23 @@ attention_generic_kernel(const TQ* __restrict__ q, TQ* __restrict__ out, const T
         } else {
           // A key that a pair does not see is left out, not multiplied by zero: its value may be infinite.  One that it sees
           // is multiplied whatever its weight is, as above, so that a row's result does not depend on the block's other rows.
-          for (int u = 0; u < RUN; ++u)
+          for (int u = 0; u < RUN; ++u) {
+            float v[DPT];
+#pragma unroll
+            for (int e = 0; e < DPT; ++e) v[e] = de + e * DT < d ? Vs[u * ld + de + e * DT] : 0.f;
 #pragma unroll
             for (int i = 0; i < PAIRS; ++i) {
               const float w0 = s_p[u * PLD + pg + 2 * i], w1 = s_p[u * PLD + pg + 2 * i + 1];
+              if (!(w0 < 0.f)) {
 #pragma unroll
-              for (int e = 0; e < DPT; ++e) {
-                const float v = de + e * DT < d ? Vs[u * ld + de + e * DT] : 0.f;
-                const float x = lo_of(acc[e][i]), y1 = hi_of(acc[e][i]);
-                acc[e][i] = pair_of(w0 < 0.f ? x : fmaf(w0, v, x), w1 < 0.f ? y1 : fmaf(w1, v, y1));
+                for (int e = 0; e < DPT; ++e) acc[e][i] = pair_of(fmaf(w0, v[e], lo_of(acc[e][i])), hi_of(acc[e][i]));
+              }
+              if (!(w1 < 0.f)) {
+#pragma unroll
+                for (int e = 0; e < DPT; ++e) acc[e][i] = pair_of(lo_of(acc[e][i]), fmaf(w1, v[e], hi_of(acc[e][i])));
               }
             }
+          }
         }
         __syncthreads();                                    // the values and the weights are free
         copy(next, 1);
