@@ -8,10 +8,10 @@
 //
 // Shape of the kernel (gemm_split_kernel): weights are the MMA's A operand (128 features = 128 lanes), rows of x its N.
 //   warp 0      TMA: weights as they are, 128 x 64 floats a stage, and the three planes of x (cut by `split_rows_kernel`)
-//   warps 2-5   read the weights of a stage, cut them in registers and put the three planes into tensor memory (the MMA
+//   warps 2-9   read the weights of a stage, cut them in registers and put the three planes into tensor memory (the MMA
 //               takes A from there), so that the weights cross the memory system once, in 32 bits, and no copy is kept
 //   warp 1      24 MMAs a chunk (six products of four steps of 16 k) into one of two accumulators
-//   warps 6-..  add a finished accumulator to their sums in registers while the next is being filled
+//   warps 10-.. add a finished accumulator to their sums in registers while the next is being filled
 // K is cut into parts (`split_parts`, from N and K alone) so that the feature tiles fill the SMs.  Up to 16 rows the parts of
 // a tile are a cluster of CTAs, two of them to an SM, and meet in shared memory; beyond, a CTA walks (tile, part) units
 // and leaves the parts' sums in memory for `sum_parts_kernel`.  Either way an output's sum is the chunks of a part in
@@ -29,6 +29,7 @@ using namespace kf_tc;
 constexpr int CK = 64;                                          // k of a chunk: the life of an accumulator
 constexpr int W_STAGE = BM * CK * 4;                            // 32 KB: two boxes of 128 rows x 32 floats
 constexpr int A_COLS = 3 * CK / 2;                              // tensor-memory columns of a chunk's three weight planes
+constexpr int CUTTERS = 256;                                    // threads that cut weights: two per feature
 constexpr int FLAG_SETS = 8;                                    // units by which converters may be ahead of the sums, and more
 constexpr int SMALL_T = 16, LARGE_T = 160;                      // rows of a tile, at most
 constexpr uint32_t TINY = 0x12800000u;                          // 2^-90
@@ -119,17 +120,17 @@ struct SplitArgs {
   const int* row_odd;
   int* error_flag;
   float softcap;
-  int T, N, K, parts, bn, w_stages;                              // bn: rows of a tile, a multiple of 16
+  int T, N, K, parts, bn, w_stages;                              // bn: rows of a tile, 16 or a multiple of 32
 };
 
-// LARGE: a CTA per SM, up to 160 rows, the sums in eight warps.  Otherwise two CTAs per SM, 16 rows, the sums in four.
+// LARGE: a CTA per SM, up to 160 rows, the sums in sixteen warps.  Otherwise two CTAs per SM, 16 rows, the sums in four.
 template <bool LARGE>
 struct SplitShape {
   static constexpr int MAX_T = LARGE ? LARGE_T : SMALL_T;
-  static constexpr int SUM_GROUPS = LARGE ? 2 : 1;
+  static constexpr int SUM_GROUPS = LARGE ? 4 : 1;
   static constexpr int COLS = MAX_T / SUM_GROUPS;                // accumulator columns of a thread, at most
-  static constexpr int BATCH = 16;                               // columns per wait on tensor memory
-  static constexpr int THREADS_ = 64 + 128 + 128 * SUM_GROUPS;
+  static constexpr int BATCH = LARGE ? COLS / 5 : 16;             // columns per wait on tensor memory
+  static constexpr int THREADS_ = 64 + CUTTERS + 128 * SUM_GROUPS;
   static constexpr int TMEM = LARGE ? 512 : 256;
   static constexpr int X_STAGES = 2;
 };
@@ -153,7 +154,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   uint64_t* acc_free = done + 2;                                  // [2] its accumulator has been read
   uint32_t* tmem_slot = (uint32_t*)(acc_free + 2);
   volatile int* s_abort = (volatile int*)(tmem_slot + 1);
-  volatile uint8_t* s_odd = (volatile uint8_t*)(tmem_slot + 2);   // [FLAG_SETS][128] features that need the plain product
+  volatile uint8_t* s_odd = (volatile uint8_t*)(tmem_slot + 2);   // [FLAG_SETS][CUTTERS] features that need the plain product
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int chunks = (a.K + CK - 1) / CK;
@@ -161,9 +162,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   const int n_units = n_ft * n_tt * a.parts;                      // unit = ((feature tile) * n_tt + row tile) * parts + part
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < ws; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 128); }
+    for (int s = 0; s < ws; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], CUTTERS); }
     for (int s = 0; s < S::X_STAGES; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&a_full[b], 128); mbar_init(&done[b], 1); mbar_init(&acc_free[b], 128 * S::SUM_GROUPS); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&a_full[b], CUTTERS); mbar_init(&done[b], 1); mbar_init(&acc_free[b], 128 * S::SUM_GROUPS); }
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -261,9 +262,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       }
     }
     __syncwarp();
-  } else if (warp < 6) {
-    // ---- weights: a thread per feature, 64 k at a time from shared memory into three planes of tensor memory ------------------
-    const int quarter = warp & 3, r = quarter * 32 + lane;
+  } else if (warp < 2 + CUTTERS / 32) {
+    // ---- weights: two threads per feature, 32 k each at a time from shared memory into three planes of tensor memory ----------
+    const int quarter = warp & 3, half = (warp - 2) >> 2, r = quarter * 32 + lane;
     const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
     int c = 0, slot = 0, set = 0;
     uint32_t ph = 0;
@@ -277,25 +278,22 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         ok = mbar_wait(&w_full[slot], ph) && (c < 2 || mbar_wait(&done[b], (uint32_t)((c >> 1) - 1) & 1)) && !*s_abort;
         if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) give_up(ERR_WAIT_FULL); ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint8_t* row = sw + (size_t)slot * W_STAGE + half * (W_STAGE / 2) + r * 128;
+        const uint32_t dst = lane_addr + b * A_COLS + half * 16;
+        uint32_t p1[16], p2[16], p3[16];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const uint8_t* row = sw + (size_t)slot * W_STAGE + h * (W_STAGE / 2) + r * 128;
-          uint32_t p1[16], p2[16], p3[16];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {                           // 16-byte piece j of a row stands at j ^ (row % 8)
-            const float4 v = *reinterpret_cast<const float4*>(row + ((j ^ (r & 7)) << 4));
-            largest = max(max(largest, __float_as_uint(fabsf(v.x))), __float_as_uint(fabsf(v.y)));
-            largest = max(max(largest, __float_as_uint(fabsf(v.z))), __float_as_uint(fabsf(v.w)));
-            cut_pair(v.x, v.y, p1[2 * j], p2[2 * j], p3[2 * j]);
-            cut_pair(v.z, v.w, p1[2 * j + 1], p2[2 * j + 1], p3[2 * j + 1]);
-          }
-          const uint32_t dst = lane_addr + b * A_COLS + h * 16;
-          tmem_st16(dst, p1);
-          tmem_st16(dst + CK / 2, p2);
-          tmem_st16(dst + CK, p3);
+        for (int j = 0; j < 8; ++j) {                             // 16-byte piece j of a row stands at j ^ (row % 8)
+          const float4 v = *reinterpret_cast<const float4*>(row + ((j ^ (r & 7)) << 4));
+          largest = max(max(largest, __float_as_uint(fabsf(v.x))), __float_as_uint(fabsf(v.y)));
+          largest = max(max(largest, __float_as_uint(fabsf(v.z))), __float_as_uint(fabsf(v.w)));
+          cut_pair(v.x, v.y, p1[2 * j], p2[2 * j], p3[2 * j]);
+          cut_pair(v.z, v.w, p1[2 * j + 1], p2[2 * j + 1], p3[2 * j + 1]);
         }
+        tmem_st16(dst, p1);
+        tmem_st16(dst + CK / 2, p2);
+        tmem_st16(dst + CK, p3);
         mbar_arrive(&w_empty[slot]);
-        if (i + 1 == last) s_odd[set * 128 + r] = odd_range(largest);
+        if (i + 1 == last) s_odd[set * CUTTERS + threadIdx.x - 64] = odd_range(largest);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         mbar_arrive(&a_full[b]);
@@ -305,8 +303,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     }
     __syncwarp();
   } else {
-    // ---- sums: a thread per feature and half of the rows -----------------------------------------------------------------------
-    const int quarter = warp & 3, group = (warp - 6) >> 2;
+    // ---- sums: a thread per feature and a quarter of the rows (the small tile: all of them) --------------------------------------
+    const int quarter = warp & 3, group = (warp - 2 - CUTTERS / 32) >> 2;
     const int fl = quarter * 32 + lane;
     const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
     const int cols = bn / S::SUM_GROUPS, col0 = group * cols;
@@ -346,7 +344,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       // ---- the unit's outputs: the parts of a product in a cluster through shared memory, else to memory -----------------------
       const int z = unit % a.parts, t0 = (unit / a.parts % n_tt) * bn, f = unit / a.parts / n_tt * BM + fl;
       const int k0 = first * CK, k1 = min(a.K, last * CK);
-      const bool f_odd = s_odd[set * 128 + fl] != 0;
+      const int at = set * CUTTERS + ((quarter + 2) & 3) * 32 + lane;   // the cutting threads of this feature: warps 2-5 and 6-9
+      const bool f_odd = (s_odd[at] | s_odd[at + 128]) != 0;
       set = (set + 1) % FLAG_SETS;
       uint32_t t_odd[(S::COLS + 31) / 32];
 #pragma unroll
@@ -387,8 +386,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     const int z = blockIdx.x % a.parts, f0 = blockIdx.x / a.parts * BM;
-    if (warp >= 6) {
-      const int fl = threadIdx.x - 192, f = f0 + fl;
+    if (warp >= 2 + CUTTERS / 32) {
+      const int fl = threadIdx.x - 64 - CUTTERS, f = f0 + fl;
       const uint32_t red = smem_u32(sw);
       for (int t = z; t < min(a.T, SMALL_T); t += a.parts) {
         float part[8];
@@ -461,7 +460,7 @@ template <bool LARGE, typename TO>
 int launch_split(const CUtensorMap& tw, const CUtensorMap& tx, SplitArgs a, cudaStream_t stream) {
   using S = SplitShape<LARGE>;
   constexpr size_t LIMIT = LARGE ? SMEM_LIMIT : 112 * 1024;       // two CTAs of the small one share an SM
-  const size_t fixed = (size_t)S::X_STAGES * 3 * a.bn * CK * 2 + 1024 + 256 + FLAG_SETS * 128;
+  const size_t fixed = (size_t)S::X_STAGES * 3 * a.bn * CK * 2 + 1024 + 256 + FLAG_SETS * CUTTERS;
   a.w_stages = (int)((LIMIT - fixed) / W_STAGE);
   if (a.w_stages > 6) a.w_stages = 6;
   const size_t smem = fixed + (size_t)a.w_stages * W_STAGE;
@@ -510,7 +509,7 @@ int linear_split(const float* x, const float* w, TO* out, int T, int N, int K, f
   a.parts = split_parts(N, K);
   const bool large = T > SMALL_T;
   const int n_tt = kf_ceil_div(T, large ? LARGE_T : SMALL_T);
-  a.bn = (kf_ceil_div(T, n_tt) + 15) & ~15;
+  a.bn = large ? (kf_ceil_div(T, n_tt) + 31) & ~31 : SMALL_T;
   __nv_bfloat16* planes = (__nv_bfloat16*)scratch;
   a.row_odd = (int*)(scratch + plane_floats(T, K));
   a.partial = scratch + plane_floats(T, K) + ((T + 3) & ~3);
