@@ -522,6 +522,13 @@ struct RopeArgs {
   __nv_bfloat16* q_out;                                           // [T, nh * head size]
 };
 
+// Feature and token tile of a persistent kernel's tile number: token tiles fastest, so that the CTAs running side by side read a
+// few weight tiles and all the rows, and the weights, by far the larger operand of a prompt, come from memory once.
+__device__ __forceinline__ void tile_place(int tile, int n_tt, int& ft, int& tt) {
+  ft = tile / n_tt;
+  tt = tile - ft * n_tt;
+}
+
 template <int EPI, int PN>                                        // PN: tokens of the pair's tile = MMA N (256, or 128 for EPI_ROPE)
 __device__ __forceinline__ void
 gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __restrict__ out, int T, int N, int K, int ld_out,
@@ -583,8 +590,10 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
       bool ok = true;
       const uint32_t full0 = map_to_rank(smem_u32(&full[0]), 0);   // the leader's full[0], as a cluster address
       for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
-        const int f0 = ((tile % n_ft) * 2 + (int)rank) * (ROPE ? 2 * BM : BM);
-        const int t0 = (tile / n_ft) * PN + (int)rank * (PN / 2);
+        int ft, tt;
+        tile_place(tile, n_tt, ft, tt);
+        const int f0 = (ft * 2 + (int)rank) * (ROPE ? 2 * BM : BM);
+        const int t0 = tt * PN + (int)rank * (PN / 2);
         for (int kb = 0; kb < nkb; ++kb) {
           if (!mbar_wait(&empty[s], ph)) {
             atomicExch(error_flag, ERR_WAIT_EMPTY);
@@ -650,11 +659,13 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
     int ti = 0;
     for (int tile = pair; tile < n_tiles; tile += n_pairs, ++ti) {
       const int buf = ti % NBUF;
-      const int f0 = ((tile % n_ft) * 2 + (int)rank) * (ROPE ? 2 * BM : BM), t0 = (tile / n_ft) * PN;
+      int ft, tt;
+      tile_place(tile, n_tt, ft, tt);
+      const int f0 = (ft * 2 + (int)rank) * (ROPE ? 2 * BM : BM), t0 = tt * PN;
       const int f = f0 + quarter * 32 + lane;
       // ROPE: where this warp's PN / 4 rows go (one or two rows per lane), looked up while the accumulator is still being filled:
       // for k and v heads the row's slot in the pages (in rows of 256), for q heads 0; -1 for rows of no request
-      const int head = ((tile % n_ft) * 2 + (int)rank) * hpc + (hpc == 2 ? quarter >> 1 : 0);
+      const int head = (ft * 2 + (int)rank) * hpc + (hpc == 2 ? quarter >> 1 : 0);
       const bool is_q = ROPE && head < ra.nh, is_k = ROPE && !is_q && head < ra.nh + ra.nkv;
       const bool is_v = ROPE && !is_q && !is_k && head < ra.nh + 2 * ra.nkv;
       const bool rope_work = is_q || ((is_k || is_v) && ra.write_kv);
@@ -685,6 +696,12 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = lane_addr + buf * NACC * PN;
+      // The next tile's products may begin once this thread's last columns are in registers: with one accumulator set they wait
+      // for the slowest thread, which needs not have stored.
+      auto release = [&]() {
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        mbar_arrive_cluster(map_to_rank(smem_u32(&acc_empty[buf]), 0));
+      };
       if constexpr (ROPE) {
         // this CTA's head: a q head (rotated to q_out), a k head (rotated into the page), a v head (into the page) or none
         const int i = (quarter * 32 + lane) & (ra.half - 1);                         // the rotation pair (i, i + half) of the head
@@ -706,6 +723,7 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
             float v[16], u[16];
             tmem_ld16(acc + c0, v);
             tmem_ld16(acc + PN + c0, u);
+            if (cc + 1 == PN / 64) release();
             const int meta = (cc & 2) ? meta_b : meta_a;
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
@@ -730,6 +748,8 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
               }
             }
           }
+        } else {
+          release();
         }
       } else {
 #pragma unroll 1
@@ -737,6 +757,7 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
           float v[32], u[32];
           if (GATED) tmem_ld32x2(acc + c0, acc + PN + c0, v, u);
           else tmem_ld32(acc + c0, v);
+          if (c0 + 32 == (col_half + 1) * (PN / 4)) release();
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const int t = t0 + c0 + j;
@@ -751,8 +772,6 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
           }
         }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      mbar_arrive_cluster(map_to_rank(smem_u32(&acc_empty[buf]), 0));
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
