@@ -185,8 +185,9 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
 }
 
 // The 64-key tiles a tile of query rows reads (and its first key), and into how many runs they are cut: `n_parts` runs for
-// every tile when `run_tiles` is 0; otherwise as many runs of at most `run_tiles` key tiles as the tile needs, at most
-// n_parts (short tiles then stay whole and write their rows themselves, long ones are shared between blocks).
+// every tile when `run_tiles` is 0; as many as the tile's own length is worth, up to n_parts, when it is RUNS_BY_LENGTH;
+// otherwise as many runs of at most `run_tiles` key tiles as the tile needs, at most n_parts (short tiles then stay whole and
+// write their rows themselves, long ones are shared between blocks).
 // With kept first tokens (keys 0..keep_first-1 stay visible behind the window) the tiles of those keys that lie before
 // the window's first tile are walked first: `*n_kept` of them, tile i of the walk starting at key_of_tile(i, ...).
 __device__ __forceinline__ int tile_key_tiles(int row0, int nrows, const int* positions, const int* row_req, int window,
@@ -200,8 +201,17 @@ __device__ __forceinline__ int tile_key_tiles(int row0, int nrows, const int* po
 __device__ __forceinline__ int key_of_tile(int i, int kt_first, int n_kept) {
   return i < n_kept ? i * BKV : kt_first + (i - n_kept) * BKV;
 }
+// A launch is planned for the longest context that its step may have; a tile whose own keys are few gains nothing from being
+// cut: a key tile takes a block about 0.93 us, the partial rows and their merge as much as MERGE_TILES of them.
+constexpr int RUNS_BY_LENGTH = -1, MERGE_TILES = 9;
 __device__ __forceinline__ int tile_runs(int n_key_tiles, int n_parts, int run_tiles) {
   if (n_parts <= 1) return 1;
+  if (run_tiles == RUNS_BY_LENGTH) {
+    int best = 1;
+    for (int p = 2; p <= n_parts; ++p)
+      if ((n_key_tiles + p - 1) / p + MERGE_TILES < (n_key_tiles + best - 1) / best + (best > 1 ? MERGE_TILES : 0)) best = p;
+    return best;
+  }
   if (run_tiles <= 0) return n_parts;
   const int p = (n_key_tiles + run_tiles - 1) / run_tiles;
   return p < 1 ? 1 : (p > n_parts ? n_parts : p);
@@ -616,13 +626,14 @@ attn_prefill_merge_kernel(const float* __restrict__ partial, const int* __restri
                           const int* __restrict__ row_req, int window, int keep_first, int nh, int n_parts_max,
                           int run_tiles, __nv_bfloat16* __restrict__ out) {
   kf_pdl_trigger();
-  kf_pdl_wait();
-  const int tile = blockIdx.x, r = blockIdx.y;
-  if (r >= tile_nrows[tile]) return;
+  const int tile = blockIdx.x, r = blockIdx.y;                // the step's integers may be read before the wait
+  const int nrows = tile_nrows[tile];
   int kt_first, n_kept;
-  const int n_parts = tile_runs(tile_key_tiles(tile_row0[tile], tile_nrows[tile], positions, row_req, window, keep_first,
+  const int n_parts = tile_runs(tile_key_tiles(tile_row0[tile], nrows, positions, row_req, window, keep_first,
                                                &kt_first, &n_kept), n_parts_max, run_tiles);
-  if (n_parts == 1) return;                                   // a tile with one run wrote its rows itself
+  kf_pdl_wait();
+  if (r >= nrows || n_parts == 1) return;                     // a tile with one run wrote its rows itself
+  partial = kf_produced(partial);
   const int row = tile_row0[tile] + r;
   constexpr int REC = D + 4;
   for (int e = threadIdx.x; e < nh * (D / 4); e += blockDim.x) {
@@ -765,7 +776,7 @@ KF_API int kf_attention_prefill_tc_plan(int n_tiles, int nh, int max_keys, int* 
 
 // q, out: [T, nh*d] bfloat16; pages: [n_pages, 2, nkv, page_size, d] bfloat16.  tile_row0/tile_nrows: tiles of up to 128
 // consecutive rows of one request (consecutive positions).  n_parts > 1 cuts a tile's keys into up to that many runs
-// (every tile's when run_tiles is 0, else those of tiles with more than run_tiles key tiles);
+// (every tile's when run_tiles is 0, by the tiles' own lengths when it is -1, else those of tiles with more than run_tiles key tiles);
 // `partial` then holds T * nh * n_parts * (d + 4) floats.
 KF_API int kf_attention_prefill_tc(const void* q, void* out, const void* pages, long n_pages, int T, const int* tile_row0,
                                    const int* tile_nrows, int n_tiles, const int* positions, const int* row_req,
@@ -776,7 +787,7 @@ KF_API int kf_attention_prefill_tc(const void* q, void* out, const void* pages, 
   if (window <= 0) keep_first = 0;
   if (nkv < 1 || nh % nkv != 0 || page_size % 64 != 0 || !kf_head_map_ok(nh, nkv, vsplit)) return KF_ERR_SIZE;
   const KfHeadMap hm = kf_head_map(0, 0, nh, nkv, vsplit);
-  if (n_parts < 1 || n_parts > 8 || (n_parts > 1 && !partial) || run_tiles < 0) return KF_ERR_SIZE;
+  if (n_parts < 1 || n_parts > 8 || (n_parts > 1 && !partial) || run_tiles < RUNS_BY_LENGTH) return KF_ERR_SIZE;
   CUtensorMap tq, tkv;
   if (!tensor_map(q, T, (long)hm.n_query * d, BMQ, &tq)) return KF_ERR_SETUP;
   if (!tensor_map(pages, n_pages * 2 * hm.n_stored * page_size, d, BKV, &tkv)) return KF_ERR_SETUP;

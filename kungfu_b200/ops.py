@@ -584,6 +584,8 @@ def paged_attention(q, out, ctx, cache, n_heads: int, n_kv_heads: int, head_dim:
             parts, run_tiles = int(prefill_plan_override[0]), ctypes.c_int(int(prefill_plan_override[1]))
         else:
             parts = lib.kf_attention_prefill_tc_plan(ctx.n_wide, n_heads, int(max_keys), ctypes.byref(run_tiles)) if split_prompt_keys else 1
+            if parts > 1 and run_tiles.value == 0:
+                run_tiles = ctypes.c_int(-1)               # planned for the longest context: tiles of few keys stay whole
         partial = _partial(q.device, T * n_heads * parts * (head_dim + 4)) if parts > 1 else None
         _check(lib.kf_attention_prefill_tc(_p(q), _p(out), _p(pages), ctypes.c_long(pages.shape[0]), T, _p(ctx.wide_row0),
                                            _p(ctx.wide_nrows), ctx.n_wide, *common, _p(sc["error"]), parts, run_tiles.value,
