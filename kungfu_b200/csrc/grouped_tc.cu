@@ -1,0 +1,197 @@
+// Products of a mixture's experts over many rows, on tcgen05:  out[r, n] = sum_k x[r, k] w[e(r)][n, k]  for the sorted pairs r
+// of a plan (grouped.cu), bfloat16 operands, 32-bit accumulation; gated: gate and up rows of an expert in two accumulators.
+//
+// A block owns 128 features of an expert x up to 128 of its rows (two neighbouring tiles of the plan's list): weights are the
+// MMA's A operand (128 lanes), rows its N (64 or 128), K in stages of 64 through a TMA ring, one tile per block; roles as in
+// gemm_tc.cu.  Rows that are read through the plan (one row per token) are first copied in sorted order, which costs less
+// than a row-wise gather in every feature tile.  What bounds it is what an SM takes in: 48 KB a stage for 16.8 M multiply-adds.
+#include "common.cuh"
+#include "tc_common.cuh"
+
+namespace {
+
+using namespace kf_tc;
+
+constexpr int GT_ROWS = 128, GT_PLAN = 64;                      // rows of a block; of a tile of the plan
+
+struct GroupedTc {
+  const int* tile_group; const int* tile_row0; const int* tile_nrows; const int* n_tiles;
+  const int* row_index; const float* row_scale;                 // gated: gate and up of sorted row r times row_scale[row_index[r]]
+  void* out;
+  int* error_flag;
+  int N, K, silu, stages;
+  float limit;
+};
+
+// dst[r] = src[index[r] / div]: rows of 16-byte chunks
+__global__ void __launch_bounds__(256) sorted_rows_kernel(const uint4* src, const int* index, int div, uint4* dst, int rows, int chunks) {
+  kf_pdl_trigger();
+  kf_pdl_wait();
+  const int r = blockIdx.x;
+  const uint4* from = src + (size_t)(index[r] / div) * chunks;
+  for (int i = threadIdx.x; i < chunks; i += 256) dst[(size_t)r * chunks + i] = from[i];
+}
+
+template <int GATED, typename TO>
+__global__ void __launch_bounds__(THREADS)
+grouped_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ GroupedTc p) {
+  constexpr int NACC = GATED ? 2 : 1, A_BYTES = BM * BK * 2, B_BYTES = GT_ROWS * BK * 2, STAGE = NACC * A_BYTES + B_BYTES;
+  constexpr int TMEM = 128 * NACC;
+  kf_pdl_trigger();
+  kf_pdl_wait();                                                  // the plan and the rows come from the kernels ahead
+  const int ti = blockIdx.y;
+  if (ti >= *p.n_tiles) return;
+  const int g = p.tile_group[ti];
+  int first = ti;
+  while (first > 0 && p.tile_group[first - 1] == g) --first;
+  if ((ti - first) & 1) return;                                   // the second of two tiles
+  const int r0 = p.tile_row0[ti];
+  const bool pair = ti + 1 < *p.n_tiles && p.tile_group[ti + 1] == g;
+  const int nrows = p.tile_nrows[ti] + (pair ? p.tile_nrows[ti + 1] : 0);
+  const int f0 = blockIdx.x * BM, nkb = (p.K + BK - 1) / BK;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = (uint64_t*)(smem + (size_t)p.stages * STAGE);
+  uint64_t* empty = full + p.stages;
+  uint64_t* acc_full = empty + p.stages;
+  uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
+  volatile int* s_abort = (volatile int*)(tmem_slot + 1);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    mbar_init(acc_full, 1);
+    *s_abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  const int bytes = NACC * A_BYTES + (pair ? B_BYTES : B_BYTES / 2);
+  auto give_up = [&](int code) { atomicExch(p.error_flag, code); *s_abort = 1; };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const int w0 = g * NACC * p.N + f0;                         // the expert's gate rows, then its up rows
+      int s = 0;
+      uint32_t ph = 1;
+      for (int i = 0; i < nkb; ++i) {
+        if (!mbar_wait(&empty[s], ph)) { give_up(ERR_WAIT_EMPTY); break; }
+        uint8_t* st = smem + (size_t)s * STAGE;
+        mbar_expect_tx(&full[s], bytes);
+        tma_load_2d(st, &tm_w, &full[s], i * BK, w0);
+        if (GATED) tma_load_2d(st + A_BYTES, &tm_w, &full[s], i * BK, w0 + p.N);
+        tma_load_2d(st + NACC * A_BYTES, &tm_x, &full[s], i * BK, r0);
+        if (pair) tma_load_2d(st + NACC * A_BYTES + B_BYTES / 2, &tm_x, &full[s], i * BK, r0 + GT_PLAN);
+        if (++s == p.stages) { s = 0; ph ^= 1; }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = umma_idesc(pair ? GT_ROWS : GT_PLAN);
+      const uint64_t da0 = umma_desc(smem), du0 = umma_desc(smem + A_BYTES), db0 = umma_desc(smem + NACC * A_BYTES);
+      int s = 0;
+      uint32_t ph = 0;
+      for (int i = 0; i < nkb; ++i) {
+        if (!mbar_wait(&full[s], ph)) { give_up(ERR_WAIT_FULL); break; }
+        const uint64_t so = (uint64_t)((uint32_t)s * (uint32_t)(STAGE >> 4));
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k) {
+          umma(tmem, da0 + so + 2 * k, db0 + so + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+          if (GATED) umma(tmem + GT_ROWS, du0 + so + 2 * k, db0 + so + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+        }
+        umma_commit(&empty[s]);
+        if (++s == p.stages) { s = 0; ph ^= 1; }
+      }
+      umma_commit(acc_full);
+    }
+    __syncwarp();
+  } else {
+    const int quarter = warp & 3, f = f0 + quarter * 32 + lane;
+    const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+    const bool ok = mbar_wait(acc_full, 0) && !*s_abort;
+    if (!ok && lane == 0) give_up(ERR_WAIT_ACC);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (__all_sync(0xffffffffu, ok)) {
+      TO* out = (TO*)p.out;
+      for (int c0 = 0; c0 < nrows; c0 += 16) {
+        float v[16], u[16];
+        tmem_ld16(lane_addr + c0, v);
+        if (GATED) tmem_ld16(lane_addr + GT_ROWS + c0, u);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int r = r0 + c0 + j;
+          if (c0 + j >= nrows || f >= p.N) continue;
+          float y = v[j];
+          if (GATED) {
+            const float rs = p.row_scale ? p.row_scale[p.row_index ? p.row_index[r] : r] : 1.f;
+            const float ga = v[j] * rs, up = u[j] * rs;
+            y = p.silu ? ga / (1.f + expf(-ga)) * up : kf_clamped_swish(ga, up, p.limit);
+          }
+          kf_store(out, (size_t)r * p.N + f, y);
+        }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM) : "memory");
+  }
+}
+
+template <int GATED, typename TO>
+int launch(const CUtensorMap& tw, const CUtensorMap& tx, GroupedTc p, int max_tiles, cudaStream_t s) {
+  constexpr int STAGE = (GATED ? 2 : 1) * BM * BK * 2 + GT_ROWS * BK * 2;
+  p.stages = GATED ? 4 : 3;                                       // gated: one block per SM; otherwise two, of 96 KB
+  const size_t smem = (size_t)p.stages * STAGE + 1024 + 256;
+  auto kernel = grouped_tc_kernel<GATED, TO>;
+  static bool configured = false;                                 // per instantiation
+  if (!configured) {
+    if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+      kf_record_cuda_error(cudaGetLastError());
+      return KF_ERR_SETUP;
+    }
+    configured = true;
+  }
+  kf_launch(kernel, dim3(kf_ceil_div(p.N, BM), max_tiles), dim3(THREADS), smem, s, tw, tx, p);
+  KF_CHECK_LAUNCH();
+  return KF_OK;
+}
+
+}  // namespace
+
+// Whether this kernel takes a mixture's product: `pairs` rows over `groups` experts of [NW, K] bfloat16 weights, one behind the
+// other.  From 64 rows an expert on average: below, the weights' bytes bound the product and the kernels of grouped.cu, which
+// read only the experts and rows that exist, are the better ones.
+KF_API int kf_grouped_tc_supported(const void* x, const void* w, long pairs, int groups, int N, int K) {
+  return pairs >= 64l * groups && N >= 128 && K > 0 && K % 8 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0 && tensor_maps_available();
+}
+
+// x: [pairs, K], or with row_index one row per row_index[r] / row_div, copied to `sorted` [pairs, K] first.  gated: 0, 1 (the
+// clamped form with `limit`) or 2 (silu(gate) * up), w [groups, 2N, K] then, else [groups, N, K].  out [pairs, N].
+KF_API int kf_grouped_tc(const void* x, const int* row_index, int row_div, void* sorted, const void* w, void* out, int out_dtype,
+                         const int* tile_group, const int* tile_row0, const int* tile_nrows, const int* n_tiles, int max_tiles,
+                         int groups, int pairs, int N, int K, int gated, float limit, const float* row_scale, int* error_flag,
+                         cudaStream_t stream) {
+  if (pairs <= 0) return KF_OK;
+  if (!kf_grouped_tc_supported(x, w, pairs, groups, N, K) || max_tiles < 1 || max_tiles > 65535 || (row_index && (!sorted || row_div < 1))) return KF_ERR_SIZE;
+  if (row_index) {
+    kf_launch(sorted_rows_kernel, dim3(pairs), dim3(256), 0, stream, (const uint4*)x, row_index, row_div, (uint4*)sorted, pairs, K / 8);
+    KF_CHECK_LAUNCH();
+    x = sorted;
+  }
+  CUtensorMap tw, tx;
+  if (!tensor_map(w, (long)groups * (gated ? 2 : 1) * N, K, BM, &tw) || !tensor_map(x, pairs, K, GT_PLAN, &tx)) return KF_ERR_SETUP;
+  const GroupedTc p{tile_group, tile_row0, tile_nrows, n_tiles, row_index, row_scale, out, error_flag, N, K, gated == 2, 0, limit};
+  if (out_dtype == KF_BF16) return gated ? launch<1, __nv_bfloat16>(tw, tx, p, max_tiles, stream) : launch<0, __nv_bfloat16>(tw, tx, p, max_tiles, stream);
+  if (out_dtype == KF_F32) return gated ? launch<1, float>(tw, tx, p, max_tiles, stream) : launch<0, float>(tw, tx, p, max_tiles, stream);
+  return KF_ERR_DTYPE;
+}

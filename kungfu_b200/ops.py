@@ -1225,9 +1225,14 @@ def _grouped(x, x_off, ldx, x_gstride, row_index, row_div, w, w_gstride, out, o_
                                        int(gated), _f(limit), _p(row_scale), int(most_rows), _stream()), what)
 
 
+grouped_on_tcgen05 = True       # False: experts of many rows run the mma.sync kernel too
+
+
 def grouped_on_tensor_cores(on: bool) -> None:
     """False: grouped products (per-head maps, experts) with bfloat16 weights run the generic 32-bit FMA kernel too
     (tests reach it that way)."""
+    global grouped_on_tcgen05
+    grouped_on_tcgen05 = bool(on)
     library().kf_grouped_use_tensor_cores(int(bool(on)))
 
 
@@ -1295,8 +1300,18 @@ def moe_linear(x, plan: dict, weight, out, *, gather: bool, gated: bool = False,
     if out.shape[0] != plan["pairs"] or out.shape[1] != N or x.shape[1] != K:
         raise KernelError(f"moe_linear: x{tuple(x.shape)} weight{tuple(weight.shape)} out{tuple(out.shape)} do not agree")
     tiles = (plan["tile_group"], plan["tile_row0"], plan["tile_nrows"], plan["n_tiles"])
+    act = (2 if activation == "silu" else 1) if gated else 0
+    lib = library()
+    if (grouped_on_tcgen05 and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
+            and lib.kf_grouped_tc_supported(_p(x), _p(weight), ctypes.c_long(plan["pairs"]), E, N, K)):
+        sorted_rows = _partial(x.device, plan["pairs"] * K // 2) if gather else None
+        _check(lib.kf_grouped_tc(_p(x), _p(plan["sorted_pair"] if gather else None), plan["top"] if gather else 1, _p(sorted_rows), _p(weight),
+                                 _p(out), _dt(out), *(_p(t) for t in tiles), plan["max_tiles"], E, plan["pairs"], N, K, act, _f(limit),
+                                 _p(row_scale), _p(_dev_scratch(x.device)["error"]), _stream()), "moe_linear (tcgen05)")
+        add_launches(1 if gather else 0)
+        return
     _grouped(x, 0, K, 0, plan["sorted_pair"] if gather else None, plan["top"] if gather else 1, weight, NW * K, out, 0, N, 0,
-             tiles, plan["max_tiles"], E, plan["pairs"], N, K, (2 if activation == "silu" else 1) if gated else 0, limit, "moe_linear", row_scale=row_scale,
+             tiles, plan["max_tiles"], E, plan["pairs"], N, K, act, limit, "moe_linear", row_scale=row_scale,
              most_rows=plan["pairs"] // plan["top"])               # a token chooses an expert once
 
 

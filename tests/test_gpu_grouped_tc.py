@@ -1,0 +1,62 @@
+"""Experts of many rows on tcgen05: ragged sizes, one and two tiles of the plan a block, experts without rows."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+class _Ctx:
+    def buf(self, name, shape, dtype):
+        return torch.empty(shape, dtype=dtype, device=DEV)
+
+
+# rows an expert: 130 (two tiles and one of 2 rows), 64 exactly, 1 to 300 with one empty expert; features and k around tiles of
+# 128 and 64, k shorter than the ring
+@pytest.mark.parametrize("counts,top,N,K", [((130, 130), 1, 128, 72), ((64, 64, 64), 1, 300, 264), ((1, 300, 0, 65, 128, 129, 63, 200), 1, 200, 520),
+                                            ((128, 129, 200), 2, 1000, 64)])
+@pytest.mark.parametrize("act", ["", "clamped_swish", "silu"])
+@pytest.mark.parametrize("out", ["bfloat16", "float32"])
+def test_many_rows_per_expert(counts, top, N, K, act, out):
+    from kungfu_b200 import ops
+    E = len(counts)
+    g = torch.Generator().manual_seed(N + K)
+    first = torch.cat([torch.full((n,), e) for e, n in enumerate(counts)])
+    first = first[torch.randperm(len(first), generator=g)]
+    ids = torch.stack([(first + j) % E for j in range(top)], 1).to(torch.int32)
+    T, gated = len(first), bool(act)
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16)
+    w = (torch.randn(E, 2 * N if gated else N, K, generator=g) * K ** -0.5).to(torch.bfloat16)
+    scale = torch.rand(T, top, generator=g) if act == "silu" else None
+    assert ops.library().kf_grouped_tc_supported(0, 0, T * top, E, N, K)
+    plan = ops.moe_plan(ids.to(DEV), E, _Ctx())
+    got = torch.full((T * top + 1, N), float("nan"), dtype=getattr(torch, out), device=DEV)
+    ops.moe_linear(x.to(DEV), plan, w.to(DEV), got[:-1], gather=True, gated=gated, limit=0.9, activation=act or "clamped_swish",
+                   row_scale=scale.to(DEV) if scale is not None else None)
+    assert bool(got[-1].isnan().all())
+    pair = plan["sorted_pair"].cpu().long()
+    e_of = ids.view(-1).long()[pair]
+    xs = x.double()[pair // top]
+    y, err = torch.empty(T * top, w.shape[1], dtype=torch.float64), torch.empty(T * top, w.shape[1], dtype=torch.float64)
+    for e in range(E):
+        rows = e_of == e
+        y[rows] = xs[rows] @ w[e].double().T
+        err[rows] = K * 2.0 ** -23 * (xs[rows].abs() @ w[e].double().abs().T)       # 32-bit sums of exact products
+    if gated:
+        r = scale.view(-1)[pair][:, None].double() if scale is not None else 1.0
+        gate, up = y[:, :N] * r, y[:, N:] * r
+        if act == "silu":
+            size = 1 + up.abs().clamp(min=gate.abs())
+            y = gate * torch.sigmoid(gate) * up
+        else:
+            size = 4.0
+            gate, up = gate.clamp(max=0.9), up.clamp(-0.9, 0.9)
+            y = gate * torch.sigmoid(1.702 * gate) * (up + 1)
+        err = 2 * size * (err[:, :N] + err[:, N:]) + 1e-6                          # slopes of the activations
+    err = err + (2.0 ** -8 if out == "bfloat16" else 2.0 ** -22) * y.abs() + 1e-7
+    assert bool(((got[:-1].cpu().double() - y).abs() <= err).all())
+    if not gated:
+        again = torch.empty_like(got[:-1])
+        ops.moe_linear(x[pair // top].to(DEV), plan, w.to(DEV), again, gather=False)
+        assert torch.equal(again, got[:-1])
+    ops.raise_on_device_error()
