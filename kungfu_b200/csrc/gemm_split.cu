@@ -7,7 +7,8 @@
 // sums of those chunks are added in registers, rounded to nearest.
 //
 // Shape of the kernel (gemm_split_kernel): weights are the MMA's A operand (128 features = 128 lanes), rows of x its N.
-//   warp 0      TMA: weights as they are, 128 x 64 floats a stage, and the three planes of x (cut by `split_rows_kernel`)
+//   warp 0      TMA: weights as they are, 128 x 64 floats a stage, and the three planes of x (cut by `split_rows_kernel`; up to
+//               16 rows the summing warps cut x themselves, into shared memory, two chunks ahead)
 //   warps 2-9   read the weights of a stage, cut them in registers and put the three planes into tensor memory (the MMA
 //               takes A from there), so that the weights cross the memory system once, in 32 bits, and no copy is kept
 //   warp 1      24 MMAs a chunk (six products of four steps of 16 k) into one of two accumulators
@@ -47,17 +48,26 @@ __device__ __forceinline__ void cut_pair(float a, float b, uint32_t& p1, uint32_
   p3 = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 
-// The three planes [3][T][pitch] of x [T, K], K a multiple of 4, zeros from K to the pitch, and per row whether it needs the
-// plain product.  A block per row.
+// The three planes [3][T][pitch] of x [T, K], K a multiple of 4, zeros from K to the pitch, and per row and part of K whether
+// it needs the plain product (row_odd [parts][T]).  A block per row.
 __global__ void __launch_bounds__(256)
-split_rows_kernel(const float* x, __nv_bfloat16* planes, int* row_odd, int T, int K, int pitch) {
+split_rows_kernel(const float* x, __nv_bfloat16* planes, int* row_odd, int T, int K, int pitch, int parts) {
   kf_pdl_trigger();
   kf_pdl_wait();
-  const int t = blockIdx.x;
+  const int t = blockIdx.x, chunks = (K + CK - 1) / CK;
   const float4* src = reinterpret_cast<const float4*>(x + (size_t)t * K);
+  __shared__ uint32_t s_largest[8];
+  if (threadIdx.x < 8) s_largest[threadIdx.x] = 0u;
+  __syncthreads();
   uint32_t largest = 0;
+  int part = 0;
 #pragma unroll 4
   for (int i = threadIdx.x; i < pitch / 4; i += 256) {
+    const int z = min(parts - 1, ((4 * i / CK + 1) * parts - 1) / chunks);
+    if (z != part) {
+      if (largest) atomicMax(&s_largest[part], largest);
+      largest = 0, part = z;
+    }
     const float4 v = 4 * i < K ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     uint2 p[3];
     cut_pair(v.x, v.y, p[0].x, p[1].x, p[2].x);
@@ -67,15 +77,9 @@ split_rows_kernel(const float* x, __nv_bfloat16* planes, int* row_odd, int T, in
 #pragma unroll
     for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(planes + ((size_t)j * T + t) * pitch + 4 * i) = p[j];
   }
-  __shared__ uint32_t s_largest[8];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, o));
-  if ((threadIdx.x & 31) == 0) s_largest[threadIdx.x >> 5] = largest;
+  if (largest) atomicMax(&s_largest[part], largest);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 1; i < 8; ++i) largest = max(largest, s_largest[i]);
-    row_odd[t] = odd_range(largest);
-  }
+  if (threadIdx.x < parts) row_odd[(size_t)threadIdx.x * T + t] = odd_range(s_largest[threadIdx.x]);
 }
 
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
@@ -154,7 +158,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   uint64_t* acc_free = done + 2;                                  // [2] its accumulator has been read
   uint32_t* tmem_slot = (uint32_t*)(acc_free + 2);
   volatile int* s_abort = (volatile int*)(tmem_slot + 1);
-  volatile uint8_t* s_odd = (volatile uint8_t*)(tmem_slot + 2);   // [FLAG_SETS][CUTTERS] features that need the plain product
+  uint32_t* s_rows = tmem_slot + 2;                               // rows of x with: something not finite, 2^-90 or more, not zero
+  volatile uint8_t* s_odd = (volatile uint8_t*)(tmem_slot + 6);   // [FLAG_SETS][CUTTERS] features that need the plain product
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int chunks = (a.K + CK - 1) / CK;
@@ -163,9 +168,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < ws; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], CUTTERS); }
-    for (int s = 0; s < S::X_STAGES; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], 1); }
+    for (int s = 0; s < S::X_STAGES; ++s) { mbar_init(&x_full[s], LARGE ? 1 : 128); mbar_init(&x_empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&a_full[b], CUTTERS); mbar_init(&done[b], 1); mbar_init(&acc_free[b], 128 * S::SUM_GROUPS); }
     *s_abort = 0;
+    s_rows[0] = s_rows[1] = s_rows[2] = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -189,7 +195,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     // ---- TMA: weights run ahead of x by as many stages as there are, and begin before the kernel ahead has ended ------------
     if (lane == 0) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_w) : "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_x) : "memory");
+      if (LARGE) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_x) : "memory");
       auto load_w = [&](int unit, int c, int s) {
         const int f0 = unit / a.parts / n_tt * BM;
         mbar_expect_tx(&w_full[s], W_STAGE);
@@ -206,7 +212,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         if (++wc == wl) { wu += gridDim.x; if (wu < n_units) range(wu, wc, wl); }
       };
       for (int i = 0; i < ws && wu < n_units; ++i) next_w();      // the ring is empty: nothing to wait for
-      kf_pdl_wait();                                              // the planes of x come from the kernel ahead
+      if (!LARGE) {
+        while (wu < n_units) {
+          if (!mbar_wait(&w_empty[w_slot], w_ph)) { give_up(ERR_WAIT_EMPTY); break; }
+          next_w();
+        }
+        xu = n_units;
+      }
+      if (LARGE) kf_pdl_wait();                                   // the planes of x come from the kernel ahead
       unsigned long long idle_since = 0;
       int idle = 0;
       while (xu < n_units) {                                      // the weights' walk is never behind
@@ -310,7 +323,51 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     const int cols = bn / S::SUM_GROUPS, col0 = group * cols;
     int c = 0, set = 0;
     bool ok = true;
-    kf_pdl_wait();                                                // before anything is written, and for the rows' flags
+    kf_pdl_wait();                                                // before anything is written, and for x or the rows' flags
+    // The small tile: these 128 threads cut x.  Thread i has 4 floats at k 4 (i % 16) of rows i / 16 and i / 16 + 8; a chunk's
+    // stage is its accumulator's number, free when its products are done; the next chunk's floats are on their way meanwhile.
+    const int ct = threadIdx.x - 64 - CUTTERS, cj = ct & 15;
+    int xu = blockIdx.x, xc = 0, xl = 0;
+    float4 xv[2];
+    uint32_t told = 0;                                            // what this thread has told of its rows
+    auto ask_x = [&]() {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int t = (ct >> 4) + 8 * u, k = xc * CK + 4 * cj;
+        xv[u] = xu < n_units && t < a.T && k < a.K ? *reinterpret_cast<const float4*>(a.x + (size_t)t * a.K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    };
+    auto cut_x = [&](int stage) {
+      if (xu >= n_units) return;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int t = (ct >> 4) + 8 * u;
+        uint2 q[3];
+        cut_pair(xv[u].x, xv[u].y, q[0].x, q[1].x, q[2].x);
+        cut_pair(xv[u].z, xv[u].w, q[0].y, q[1].y, q[2].y);
+        const uint32_t big = max(max(__float_as_uint(fabsf(xv[u].x)), __float_as_uint(fabsf(xv[u].y))),
+                                 max(__float_as_uint(fabsf(xv[u].z)), __float_as_uint(fabsf(xv[u].w))));
+        const uint32_t news = ((big >= 0x7f800000u ? 1u : 0u) | (big >= TINY ? 2u : 0u) | (big != 0u ? 4u : 0u)) << (3 * u);
+        if (news & ~told) {
+          told |= news;
+#pragma unroll
+          for (int e = 0; e < 3; ++e) if (news >> (3 * u + e) & 1u) atomicOr(&s_rows[e], 1u << t);
+        }
+        uint8_t* dst = sx + (size_t)stage * x_stage + t * 128 + (((cj >> 1) ^ (t & 7)) << 4) + (cj & 1) * 8;
+#pragma unroll
+        for (int e = 0; e < 3; ++e) *reinterpret_cast<uint2*>(dst + e * (SMALL_T * CK * 2)) = q[e];
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      mbar_arrive(&x_full[stage]);
+      if (++xc == xl) { xu += gridDim.x; if (xu < n_units) range(xu, xc, xl); }
+      ask_x();
+    };
+    if (!LARGE) {
+      if (xu < n_units) range(xu, xc, xl);
+      ask_x();
+      cut_x(0);
+      cut_x(1);
+    }
     for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
       int first, last;
       range(unit, first, last);
@@ -322,6 +379,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         ok = mbar_wait(&done[b], (uint32_t)(c >> 1) & 1) && !*s_abort;
         if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) give_up(ERR_WAIT_ACC); ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (!LARGE) cut_x(b);
         const uint32_t acc = lane_addr + 2 * A_COLS + b * S::MAX_T + col0;
 #pragma unroll
         for (int j0 = 0; j0 < S::COLS; j0 += S::BATCH) {
@@ -351,7 +409,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
 #pragma unroll
       for (int q = 0; q < (S::COLS + 31) / 32; ++q) {
         const int t = t0 + col0 + 32 * q + lane;
-        t_odd[q] = __ballot_sync(0xffffffffu, 32 * q + lane < cols && t < a.T && __ldcg(a.row_odd + t) != 0);
+        t_odd[q] = LARGE ? __ballot_sync(0xffffffffu, 32 * q + lane < cols && t < a.T && __ldcg(a.row_odd + (size_t)z * a.T + t) != 0)
+                         : *(volatile uint32_t*)&s_rows[0] | (*(volatile uint32_t*)&s_rows[2] & ~*(volatile uint32_t*)&s_rows[1]);
       }
       const bool in_cluster = !LARGE && a.parts > 1;
       float* red = reinterpret_cast<float*>(sw);                  // [16][128]: the ring is free by then
@@ -512,13 +571,15 @@ int linear_split(const float* x, const float* w, TO* out, int T, int N, int K, f
   a.bn = large ? (kf_ceil_div(T, n_tt) + 31) & ~31 : SMALL_T;
   __nv_bfloat16* planes = (__nv_bfloat16*)scratch;
   a.row_odd = (int*)(scratch + plane_floats(T, K));
-  a.partial = scratch + plane_floats(T, K) + ((T + 3) & ~3);
+  a.partial = scratch + plane_floats(T, K) + ((a.parts * T + 3) & ~3);
   CUtensorMap tw, tx;
-  if (!tensor_map_f32(w, N, K, BM, &tw) || !tensor_map(planes, 3l * T, pitch, a.bn, &tx)) return KF_ERR_SETUP;
-  kf_launch(split_rows_kernel, dim3(T), dim3(256), 0, stream, x, planes, (int*)a.row_odd, T, K, pitch);
+  if (!tensor_map_f32(w, N, K, BM, &tw)) return KF_ERR_SETUP;
+  if (!large) return launch_split<false, TO>(tw, tw, a, stream);
+  if (!tensor_map(planes, 3l * T, pitch, a.bn, &tx)) return KF_ERR_SETUP;
+  kf_launch(split_rows_kernel, dim3(T), dim3(256), 0, stream, x, planes, (int*)a.row_odd, T, K, pitch, a.parts);
   KF_CHECK_LAUNCH();
-  const int s = large ? launch_split<true, TO>(tw, tx, a, stream) : launch_split<false, TO>(tw, tx, a, stream);
-  if (s != KF_OK || !large || a.parts == 1) return s;
+  const int s = launch_split<true, TO>(tw, tx, a, stream);
+  if (s != KF_OK || a.parts == 1) return s;
   const long n = (long)T * N;
   kf_launch(sum_parts_kernel<TO>, dim3(kf_ceil_div(n, 1024)), dim3(256), 0, stream, (const float*)a.partial, out, n, a.parts, softcap);
   KF_CHECK_LAUNCH();
@@ -536,9 +597,9 @@ KF_API int kf_linear_split_supported(const void* x, const void* w, int N, int K)
 // Floats of scratch that a call needs, and the kernels that it launches.
 KF_API long kf_linear_split_scratch(int T, int N, int K) {
   const int parts = split_parts(N, K);
-  return plane_floats(T, K) + ((T + 3) & ~3) + (T > SMALL_T && parts > 1 ? (long)parts * T * N : 0);
+  return T <= SMALL_T ? 0 : plane_floats(T, K) + (((long)parts * T + 3) & ~3l) + (parts > 1 ? (long)parts * T * N : 0);
 }
-KF_API int kf_linear_split_launches(int T, int N, int K) { return T > SMALL_T && split_parts(N, K) > 1 ? 3 : 2; }
+KF_API int kf_linear_split_launches(int T, int N, int K) { return T <= SMALL_T ? 1 : split_parts(N, K) > 1 ? 3 : 2; }
 
 // out[T, N] = x[T, K] . w[N, K]^T, all 32-bit (out may be bfloat16); softcap > 0 applies cap * tanh(v / cap).
 KF_API int kf_linear_split(const float* x, const float* w, void* out, int out_dtype, int T, int N, int K, float softcap,
