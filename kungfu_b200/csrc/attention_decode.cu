@@ -403,14 +403,12 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 // O += P V run on mma.sync with 32-bit accumulators, the online softmax is the one of the prompt kernel.  Warps are merged
 // through shared memory in warp order, the parts of a row by the block that arrives last.
 //
-// Two ways to share out the work.  Few pairs (row, kv head): a pair's keys are cut into n_splits equal parts, a block each.
-// Many (RUNS): the tiles of all pairs lie one pair behind the other, each block takes an equal run of them, counted from the
-// rows' own lengths on the device (a replayed step is planned for the longest context there may be), and walks the pairs or
-// parts of pairs in it.  A change of pairs costs a block about 10 us in which its ring runs empty, so these blocks have four
-// warps and two of them share an SM; the next piece's first tiles are requested before the warps are merged.  A run is DM_LEAST
-// tiles or more (fewer blocks then work), and long enough that a pair has at most MERGE_MAX_SPLITS records.
-// A part of a pair leaves a record; a pair's records lie behind one another, from place pair * n_splits or (RUNS) from
-// (block + pair) on.
+// The work is the tiles of all pairs (row, kv head), one pair behind the other.  Each block takes an equal run of them,
+// counted from the rows' own lengths on the device (a replayed step is planned for the longest context there may be), and
+// walks the pairs or parts of pairs in it; it requests the next one's first tiles before it merges its warps.  A part of a
+// pair leaves a record at place (block + pair), so a pair's records lie behind one another.  A run is DM_LEAST tiles or
+// more (fewer blocks then work), and long enough that a pair has at most MERGE_MAX_SPLITS records.
+// With whole pairs (n_splits 1) a block takes the pair of its own number.
 constexpr int DM_WARPS = 8;                       // two per scheduler: a warp's tile is one chain of dependent instructions
 // More (row, kv head) pairs than blocks of eight warps fit the GPU, and short rows: a block then is mostly its start and its
 // merge, and blocks of four warps, two to an SM at heads of 256, cover each other's.  64 rows of 8 heads over 4 of 256, alone:
@@ -442,14 +440,14 @@ struct DmRun { long total; int at, end, item, item_at, n_blocks, n_open; };
 struct DmPiece { int t, req, pos, kvh, pair, tile0, n_tiles, alone, more; };
 struct DmOpen { int pair, records, first_block, t; };
 
-template <int D, bool SIG, int DM_WARPS, bool RUNS>
+template <int D, bool SIG, int DM_WARPS>
 __global__ void __launch_bounds__(DM_WARPS * 32, dm_blocks_per_sm(D, DM_WARPS))
 attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restrict__ qkv, const float* __restrict__ cos_t,
                        const float* __restrict__ sin_t, int rot, int write_kv, __nv_bfloat16* pages,
                        const int* __restrict__ items, int n_items, const int* __restrict__ positions,
                        const int* __restrict__ row_req, const int* __restrict__ table, int table_stride, int page_size,
                        int nh, int nkv, float scale, float softcap, int window, int vsplit, int keep_first, int sink,
-                       const float* __restrict__ sig_bias, int n_splits, int apart, float* __restrict__ partial, int* __restrict__ counters,
+                       const float* __restrict__ sig_bias, int whole_pairs, int apart, float* __restrict__ partial, int* __restrict__ counters,
                        __nv_bfloat16* __restrict__ out) {
   using namespace kf_mma;
   kf_pdl_trigger();
@@ -478,36 +476,16 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
     const int req = row_req[t], pos = positions[t], lo = kf_first_key(pos, window);
     return req < 0 ? 0 : (pos + 1 - lo + (window > 0 ? min(keep_first, lo) : 0) + DM_KEYS - 1) / DM_KEYS;
   };
-  const size_t head_stride = (size_t)page_size * D;
-  // ---- the piece of a pair that is being walked ---------------------------------------------------------------------------
-  int t, pos, kvh, lo, lo_v, k_begin, k_end, own_tile, n_mine, key_head, pair = 0;
-  bool first_part = false;
-  const int* tab;
-  size_t v_off;
-  // row `t` of request `req` at `pos`, head `kvh`: `begin` keys into the walk, up to `count` of them
-  auto take = [&](int req, int begin, int count) {
-    const KfHeadMap hm = kf_head_map(kvh * G, kvh, nh, nkv, vsplit);   // with the rotation inside (qkv given) vsplit is 0
-    key_head = hm.key;
-    // Kept first tokens: keys [0, kept) are seen behind the window.  The keys are walked by a running index u in
-    // [lo_v, pos]: u >= lo is key u itself, u in [lo_v, lo) is key u - lo_v, so the walk below does not know of the gap.
-    lo = kf_first_key(pos, window);
-    lo_v = lo - (window > 0 ? min(keep_first, lo) : 0);
-    k_begin = lo_v + begin;
-    k_end = min(pos + 1, k_begin + count);
-    // the tile that holds the row's own key: an earlier kernel of this step writes that key (or this block does)
-    own_tile = pos >= k_begin && pos < k_end ? (pos - k_begin) / DM_KEYS : -1;
-    tab = table + (size_t)req * table_stride;
-    v_off = (size_t)(hm.n_stored + hm.value - hm.key) * head_stride;
-    // A warp walks its tiles (warp, warp + DM_WARPS, ...) as the sequence K0 V0 K1 V1 ...: item n is the keys (n even) or
-    // the values (n odd) of its tile n / 2 and lands in buffer n % DM_BUFS.
-    const int n_tiles = k_end > k_begin ? (k_end - k_begin + DM_KEYS - 1) / DM_KEYS : 0;
-    n_mine = n_tiles > warp ? (n_tiles - warp + DM_WARPS - 1) / DM_WARPS : 0;
-    first_part = begin == 0;
-  };
-  auto take_piece = [&](const DmPiece& p) {
-    t = p.t, pos = p.pos, kvh = p.kvh, pair = p.pair;
-    take(p.req, p.tile0 * DM_KEYS, p.n_tiles * DM_KEYS);
-  };
+  // rows of no request: zeros
+  for (int item = whole_pairs ? blockIdx.x / nkv : blockIdx.x; item < n_items; item += gridDim.x) {
+    const int t = row_of(item);
+    if (row_req[t] < 0) {
+      kf_pdl_wait();
+      const int first = whole_pairs ? blockIdx.x % nkv * G * D : 0, n = whole_pairs ? G * D : nh * D;
+      for (int e = tid; e < n; e += blockDim.x) out[(size_t)t * nh * D + first + e] = __float2bfloat16_rn(0.f);
+    }
+    if (whole_pairs) break;
+  }
 
   // the piece from the run's place on, to the end of its pair or of the run, whichever comes first
   auto plan = [&](DmPiece& p) {
@@ -534,16 +512,14 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
     p.more = r.at < r.end;
     s_run = r;
   };
-  if constexpr (RUNS) {
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {   // rows of no request: zeros
-      const int row = row_of(item);
-      if (row_req[row] < 0) {
-        kf_pdl_wait();
-        for (int e = tid; e < nh * D; e += blockDim.x) out[(size_t)row * nh * D + e] = __float2bfloat16_rn(0.f);
-      }
-    }
-    if (warp == 0) {
-      DmRun r = {};
+  if (warp == 0) {
+    DmRun r = {};
+    if (whole_pairs) {
+      r.item = blockIdx.x / nkv;
+      const int nt = tiles_of(r.item);
+      r.at = blockIdx.x % nkv * nt;
+      r.end = r.at + nt;
+    } else {
       int sum = 0, most = 0;
       for (int i = lane; i < n_items; i += 32) {
         const int n = tiles_of(i);
@@ -578,36 +554,41 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
         }
         r.item_at += __shfl_sync(0xffffffffu, n, 31);
       }
-      if (lane == 0) {
-        s_run = r;
-        s_piece[0].n_tiles = 0;
-        if (r.at < r.end) plan(s_piece[0]);
-      }
     }
-    __syncthreads();
-    if (s_piece[0].n_tiles == 0) return;
-    take_piece(s_piece[0]);
-  } else {
-    const int item = blockIdx.x / nkv;
-    t = row_of(item);
-    kvh = blockIdx.x - item * nkv;
-    pair = blockIdx.x;
-    const int req = row_req[t];
-    if (req < 0) {
-      kf_pdl_wait();
-      if (blockIdx.y == 0)
-        for (int e = tid; e < G * D; e += blockDim.x) out[((size_t)t * nh + kvh * G) * D + e] = __float2bfloat16_rn(0.f);
-      return;
+    if (lane == 0) {
+      s_run = r;
+      s_piece[0].n_tiles = 0;
+      if (r.at < r.end) plan(s_piece[0]);
     }
-    pos = positions[t];
-    const int first = kf_first_key(pos, window);
-    const int n_keys = pos + 1 - first + (window > 0 ? min(keep_first, first) : 0);
-    const int per = ((n_keys + n_splits - 1) / n_splits + 63) & ~63;
-    take(req, blockIdx.y * per, per);
   }
+  __syncthreads();
+  if (s_piece[0].n_tiles == 0) return;
 
+  const size_t head_stride = (size_t)page_size * D;
   __nv_bfloat16* my = sKV + (size_t)warp * DM_BUFS * TILE;        // [buffer]
 
+  // ---- the piece of a pair that is being walked ---------------------------------------------------------------------------
+  int t, pos, kvh, lo, lo_v, k_begin, k_end, own_tile, n_mine, key_head;
+  const int* tab;
+  size_t v_off;
+  auto take_piece = [&](const DmPiece& p) {
+    t = p.t, pos = p.pos, kvh = p.kvh;
+    const KfHeadMap hm = kf_head_map(kvh * G, kvh, nh, nkv, vsplit);   // with the rotation inside (qkv given) vsplit is 0
+    key_head = hm.key;
+    // Kept first tokens: keys [0, kept) are seen behind the window.  The keys are walked by a running index u in
+    // [lo_v, pos]: u >= lo is key u itself, u in [lo_v, lo) is key u - lo_v, so the walk below does not know of the gap.
+    lo = kf_first_key(pos, window);
+    lo_v = lo - (window > 0 ? min(keep_first, lo) : 0);
+    k_begin = lo_v + p.tile0 * DM_KEYS;
+    k_end = min(pos + 1, k_begin + p.n_tiles * DM_KEYS);
+    // the tile that holds the row's own key: an earlier kernel of this step writes that key (or this block does)
+    own_tile = pos < k_end ? (pos - k_begin) / DM_KEYS : -1;
+    tab = table + (size_t)p.req * table_stride;
+    v_off = (size_t)(hm.n_stored + hm.value - hm.key) * head_stride;
+    // A warp walks its tiles (warp, warp + DM_WARPS, ...) as the sequence K0 V0 K1 V1 ...: item n is the keys (n even) or
+    // the values (n odd) of its tile n / 2 and lands in buffer n % DM_BUFS.
+    n_mine = p.n_tiles > warp ? (p.n_tiles - warp + DM_WARPS - 1) / DM_WARPS : 0;
+  };
   const int n_stored = vsplit > 0 ? nkv / vsplit : nkv;
   long row_base = -1;                                             // lanes 0..15: where key j0 + lane of the item's tile lies
   auto load_item = [&](int n, int buf) {
@@ -643,6 +624,7 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
     for (int n = 0; n < DM_BUFS; ++n)
       if (n < 2 * n_mine && (warp + (n >> 1) * DM_WARPS == own_tile) == own) load_item(n, n);
   };
+  take_piece(s_piece[0]);
   request_first(false);
   if (qkv != nullptr)
     for (int idx = G * CH + tid; idx < 16 * CH; idx += blockDim.x)
@@ -651,6 +633,7 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
   q = kf_produced(q), qkv = kf_produced(qkv), cos_t = kf_produced(cos_t), sin_t = kf_produced(sin_t);
 
   for (int walk = 0;; walk ^= 1) {
+  const DmPiece& piece = s_piece[walk];
   const int h_first = kvh * G;
   __nv_bfloat16* orow = out + (size_t)t * nh * D;
   if (qkv != nullptr) {
@@ -718,10 +701,8 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
     }
   }
   __syncthreads();                                                // Q in place; the new key and value are in the page
-  if constexpr (RUNS) {
-    if (tid == DM_WARPS * 32 - 32 && s_piece[walk].more) plan(s_piece[walk ^ 1]);   // in the last warp, which has a tile less if any has
-    __syncwarp();
-  }
+  if (tid == DM_WARPS * 32 - 32 && piece.more) plan(s_piece[walk ^ 1]);   // in the last warp, which has a tile less if any has
+  __syncwarp();
   // the own-key tile, if it is one of this warp's first tiles; then all first items are one group, and empty groups
   // keep the count of one group per item that the loop below relies on
   request_first(true);
@@ -865,13 +846,13 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
 #pragma unroll
       for (int n = 0; n < NT_O; ++n)
         *reinterpret_cast<float2*>(sm_o + ((size_t)warp * G + row) * D + n * 8 + tq * 2) = make_float2(o_acc[n][2 * r], o_acc[n][2 * r + 1]);
-      if (tq == 0) { sm_ml[warp][row][0] = SIG ? 0.f : m_run[r]; sm_ml[warp][row][1] = SIG ? (warp == 0 && first_part) : l_run[r]; }
+      if (tq == 0) { sm_ml[warp][row][0] = SIG ? 0.f : m_run[r]; sm_ml[warp][row][1] = SIG ? (warp == 0 && piece.tile0 == 0) : l_run[r]; }
     }
   }
   __syncthreads();
-  const bool alone = RUNS ? s_piece[walk].alone : n_splits == 1, more = RUNS && s_piece[walk].more;
-  const bool sink_here = sink && first_part;
-  float* rec0 = partial + (RUNS ? (size_t)(blockIdx.x + pair) : (size_t)pair * n_splits + blockIdx.y) * G * PSTRIDE;
+  const bool alone = piece.alone, more = piece.more;
+  const bool sink_here = sink && piece.tile0 == 0;
+  float* rec0 = partial + (size_t)(blockIdx.x + piece.pair) * G * PSTRIDE;
   if (more && apart) {                                             // the next piece's first tiles, while this one is merged
     take_piece(s_piece[walk ^ 1]);
     request_first(false);
@@ -903,37 +884,25 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
     request_first(false);
   }
   }
-  auto merge = [&](int records, size_t first_record, __nv_bfloat16* o_first) {
-    __threadfence();                                               // maxima here are base-2 scaled
-    if (records > 8 && (size_t)G * records * PSTRIDE * sizeof(float) <= (size_t)DM_WARPS * DM_BUFS * TILE * sizeof(__nv_bfloat16))
-      merge_splits_shared<D>(partial, first_record, G, records, o_first, reinterpret_cast<float*>(sKV));
-    else
-      merge_splits<D, true>(partial, first_record, G, records, 1, G, o_first);
-  };
-  if constexpr (RUNS) {
-    const int n_open = s_run.n_open;
-    if (n_open == 0) return;
-    __threadfence();
-    __syncthreads();
-    if (tid < n_open) s_last[tid] = atomicAdd(&counters[s_open[tid].pair], 1) == s_open[tid].records - 1;
-    __syncthreads();
+  const int n_open = s_run.n_open;
+  if (n_open == 0) return;
+  __threadfence();
+  __syncthreads();
+  if (tid < n_open) s_last[tid] = atomicAdd(&counters[s_open[tid].pair], 1) == s_open[tid].records - 1;
+  __syncthreads();
 #pragma unroll 1
-    for (int o = 0; o < n_open; ++o) {
-      if (!s_last[o]) continue;
-      const DmOpen open = s_open[o];
-      merge(open.records, (size_t)(open.first_block + open.pair) * G, out + ((size_t)open.t * nh + (size_t)(open.pair % nkv) * G) * D);
-      if (tid == 0) counters[open.pair] = 0;
-      __syncthreads();
-    }
-  } else {
-    if (n_splits == 1) return;
-    __threadfence();
+  for (int o = 0; o < n_open; ++o) {
+    if (!s_last[o]) continue;
+    __threadfence();                                               // maxima here are base-2 scaled
+    const DmOpen open = s_open[o];
+    const size_t first_record = (size_t)(open.first_block + open.pair) * G;
+    __nv_bfloat16* o_first = out + ((size_t)open.t * nh + (size_t)(open.pair % nkv) * G) * D;
+    if (open.records > 8 && (size_t)G * open.records * PSTRIDE * sizeof(float) <= (size_t)DM_WARPS * DM_BUFS * TILE * sizeof(__nv_bfloat16))
+      merge_splits_shared<D>(partial, first_record, G, open.records, o_first, reinterpret_cast<float*>(sKV));
+    else
+      merge_splits<D, true>(partial, first_record, G, open.records, 1, G, o_first);
+    if (tid == 0) counters[open.pair] = 0;
     __syncthreads();
-    if (tid == 0) s_last[0] = atomicAdd(&counters[pair], 1) == n_splits - 1;
-    __syncthreads();
-    if (!s_last[0]) return;
-    merge(n_splits, (size_t)pair * n_splits * G, out + ((size_t)t * nh + kvh * G) * D);
-    if (tid == 0) counters[pair] = 0;
   }
 }
 
@@ -941,16 +910,16 @@ constexpr size_t dm_smem_bytes(int d, int warps) { return (size_t)(16 * d + warp
 
 // Blocks of the tensor-core decode kernel that one SM holds at a time (shared memory or registers, whichever binds), as
 // the runtime reports it; also sets the kernel's shared-memory limit.  0 if that fails.
-template <int D, bool SIG, int DM_WARPS, bool RUNS = false>
+template <int D, bool SIG, int DM_WARPS>
 int decode_mma_blocks_per_sm() {
   static int cached = -1;
   if (cached >= 0) return cached;
   const size_t smem = dm_smem_bytes(D, DM_WARPS);
   cudaFuncAttributes fa;
   int n = 0;
-  if (cudaFuncGetAttributes(&fa, attn_decode_mma_kernel<D, SIG, DM_WARPS, RUNS>) != cudaSuccess ||
-      cudaFuncSetAttribute(attn_decode_mma_kernel<D, SIG, DM_WARPS, RUNS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_decode_mma_kernel<D, SIG, DM_WARPS, RUNS>, DM_WARPS * 32, smem) != cudaSuccess) {
+  if (cudaFuncGetAttributes(&fa, attn_decode_mma_kernel<D, SIG, DM_WARPS>) != cudaSuccess ||
+      cudaFuncSetAttribute(attn_decode_mma_kernel<D, SIG, DM_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_decode_mma_kernel<D, SIG, DM_WARPS>, DM_WARPS * 32, smem) != cudaSuccess) {
     kf_record_cuda_error(cudaGetLastError());
     return 0;
   }
@@ -959,63 +928,63 @@ int decode_mma_blocks_per_sm() {
 }
 
 // Whether the warps' results of G heads get shared memory of their own: where that costs no resident block.
-template <int D, bool SIG, int DM_WARPS, bool RUNS>
+template <int D, bool SIG, int DM_WARPS>
 bool decode_mma_apart(int G) {
   static signed char cached[17] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
   if (cached[G] < 0) {
     int n = 0;
     cudaFuncAttributes fa;
     const size_t smem = dm_smem_bytes(D, DM_WARPS) + (size_t)DM_WARPS * G * D * sizeof(float);
-    if (cudaFuncGetAttributes(&fa, attn_decode_mma_kernel<D, SIG, DM_WARPS, RUNS>) != cudaSuccess || smem + fa.sharedSizeBytes > 227 * 1024 ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_decode_mma_kernel<D, SIG, DM_WARPS, RUNS>, DM_WARPS * 32, smem) != cudaSuccess) {
+    if (cudaFuncGetAttributes(&fa, attn_decode_mma_kernel<D, SIG, DM_WARPS>) != cudaSuccess || smem + fa.sharedSizeBytes > 227 * 1024 ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_decode_mma_kernel<D, SIG, DM_WARPS>, DM_WARPS * 32, smem) != cudaSuccess) {
       cudaGetLastError();
       n = 0;
     }
-    cached[G] = n >= decode_mma_blocks_per_sm<D, SIG, DM_WARPS, RUNS>();
+    cached[G] = n >= decode_mma_blocks_per_sm<D, SIG, DM_WARPS>();
   }
   return cached[G] != 0;
 }
 
 constexpr int MOST_BLOCKS_PER_SM = 8;
 
-// RUNS, n_splits -k: as many blocks as the GPU holds, but no more than k - 1 for each pair, so that the records (one per block and
-// one per pair, at most) fit what k records for each pair take.
-template <int D, bool SIG, int DM_WARPS, bool RUNS>
+// n_splits 1: a block per pair.  More: as many blocks as the GPU holds, but no more than the caller's n_splits - 1 for each pair,
+// so that the records (one per block and one per pair, at most) fit what n_splits records for each pair take.
+template <int D, bool SIG, int DM_WARPS>
 int launch_decode_mma_warps(const float* qkv, const float* cos_t, const float* sin_t, int rot, int write_kv,
                       const void* q, const void* pages, const int* items, int n_items, const int* positions,
                       const int* row_req, const int* table, int table_stride, int page_size, int nh, int nkv, float scale,
                       float softcap, int window, int vsplit, int keep_first, int sink, const float* sig_bias, int n_splits,
                       float* partial, int* counters, void* out, cudaStream_t stream) {
-  int per_sm = decode_mma_blocks_per_sm<D, SIG, DM_WARPS, RUNS>();
+  int per_sm = decode_mma_blocks_per_sm<D, SIG, DM_WARPS>();
   if (per_sm < 1) return KF_ERR_SETUP;
   if (per_sm > MOST_BLOCKS_PER_SM) per_sm = MOST_BLOCKS_PER_SM;
   const int G = nh / nkv;
-  const bool apart = RUNS && decode_mma_apart<D, SIG, DM_WARPS, RUNS>(G);
+  const bool apart = decode_mma_apart<D, SIG, DM_WARPS>(G);
   const size_t smem = dm_smem_bytes(D, DM_WARPS) + (apart ? (size_t)DM_WARPS * G * D * sizeof(float) : 0);
   const long pairs = (long)n_items * nkv, most = (long)kf_sm_count() * per_sm;
-  const long wanted = pairs * (-n_splits - 1);
-  const dim3 grid = RUNS ? dim3((unsigned)(wanted < most ? wanted : most)) : dim3((unsigned)pairs, n_splits);
-  kf_launch(attn_decode_mma_kernel<D, SIG, DM_WARPS, RUNS>, grid, dim3(DM_WARPS * 32), smem, stream,
+  const long blocks = n_splits <= 1 ? pairs : pairs * (n_splits - 1) < most ? pairs * (n_splits - 1) : most;
+  kf_launch(attn_decode_mma_kernel<D, SIG, DM_WARPS>, dim3((unsigned)blocks), dim3(DM_WARPS * 32), smem, stream,
             (const __nv_bfloat16*)q, qkv, cos_t, sin_t, rot, write_kv, (__nv_bfloat16*)const_cast<void*>(pages), items, n_items,
             positions, row_req, table, table_stride, page_size, nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias,
-            n_splits, apart ? 1 : 0, partial, counters, (__nv_bfloat16*)out);
+            n_splits <= 1 ? 1 : 0, apart ? 1 : 0, partial, counters, (__nv_bfloat16*)out);
   KF_CHECK_LAUNCH();
   return KF_OK;
 }
 
-// n_splits: 1 or more parts of every pair; 0, one part in blocks of DM_WARPS_SHORT warps; below 0, equal runs.
+// n_splits 0: one split in blocks of DM_WARPS_SHORT warps.
 template <int D, bool SIG>
 int launch_decode_mma(const float* qkv, const float* cos_t, const float* sin_t, int rot, int write_kv,
                       const void* q, const void* pages, const int* items, int n_items, const int* positions,
                       const int* row_req, const int* table, int table_stride, int page_size, int nh, int nkv, float scale,
                       float softcap, int window, int vsplit, int keep_first, int sink, const float* sig_bias, int n_splits,
                       float* partial, int* counters, void* out, cudaStream_t stream) {
-#define KF_WARP_ARGS(SPLITS) qkv, cos_t, sin_t, rot, write_kv, q, pages, items, n_items, positions, row_req, table, table_stride, page_size, nh, nkv, \
-                     scale, softcap, window, vsplit, keep_first, sink, sig_bias, SPLITS, partial, counters, out, stream
-  if (n_splits < 0) return launch_decode_mma_warps<D, SIG, DM_WARPS_SHORT, true>(KF_WARP_ARGS(n_splits));
-  if (n_splits == 0) return launch_decode_mma_warps<D, SIG, DM_WARPS_SHORT, false>(KF_WARP_ARGS(1));
-  return launch_decode_mma_warps<D, SIG, DM_WARPS, false>(KF_WARP_ARGS(n_splits));
-#undef KF_WARP_ARGS
+  if (n_splits == 0)
+    return launch_decode_mma_warps<D, SIG, DM_WARPS_SHORT>(
+        qkv, cos_t, sin_t, rot, write_kv, q, pages, items, n_items, positions, row_req, table, table_stride, page_size,
+        nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias, 1, partial, counters, out, stream);
+  return launch_decode_mma_warps<D, SIG, DM_WARPS>(
+        qkv, cos_t, sin_t, rot, write_kv, q, pages, items, n_items, positions, row_req, table, table_stride, page_size,
+        nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias, n_splits, partial, counters, out, stream);
 }
 
 template <int D, int HT>
@@ -1051,34 +1020,25 @@ static int g_forced_splits = 0;
 KF_API void kf_set_attention_decode_splits(int splits) { g_forced_splits = splits; }
 #endif
 
-// Blocks of one kind that the GPU holds at heads of d elements.
-template <int WARPS, bool RUNS>
-static long decode_mma_resident(int d) {
-  long per_sm = d == 256 ? decode_mma_blocks_per_sm<256, false, WARPS, RUNS>() : d == 128 ? decode_mma_blocks_per_sm<128, false, WARPS, RUNS>()
-              : d == 64 ? decode_mma_blocks_per_sm<64, false, WARPS, RUNS>() : d == 32 ? decode_mma_blocks_per_sm<32, false, WARPS, RUNS>()
-              : d == 16 ? decode_mma_blocks_per_sm<16, false, WARPS, RUNS>() : 0;
-  if (per_sm > MOST_BLOCKS_PER_SM) per_sm = MOST_BLOCKS_PER_SM;
-  return kf_sm_count() * (per_sm < 1 ? 1 : per_sm);
-}
-
-// splits_out: how many parts a row's keys are cut into; 0 for one part in blocks of fewer warps (short rows, more of them than
-// the GPU holds blocks); -k for equal runs with k records a pair on average (`launch_decode_mma_warps`): where a block per pair and
-// part would leave SMs idle or give them rows of unequal length, because the pairs are more than half of the blocks that
-// the GPU holds.  kf_attention_decode (ht = 0) and kf_attention_decode_fused take it as it is.
+// splits_out: 1 for a block per (row, kv head) pair; 0 for the same in blocks of fewer warps (short rows, more of them than the
+// GPU holds blocks); otherwise the pairs' keys are cut evenly between the blocks that the GPU holds, and splits_out is how
+// many records a pair needs on average (`launch_decode_mma_warps`).  kf_attention_decode (ht = 0) and
+// kf_attention_decode_fused take it as it is.
 KF_API int kf_attention_decode_mma_plan(int n_items, int nh, int nkv, int d, int max_keys, int* splits_out) {
   if (g_forced_splits > 0) { *splits_out = g_forced_splits; return KF_OK; }
-  const long pairs = (long)n_items * nkv, resident = decode_mma_resident<DM_WARPS, false>(d);
-  int splits = (int)(resident / pairs);                           // fill one wave
-  const int by_len = (max_keys + 255) / 256;
-  if (splits > by_len) splits = by_len;
-  if (splits > MERGE_MAX_SPLITS) splits = MERGE_MAX_SPLITS;
-  if (splits < 1) splits = 1;
-  if (pairs > resident && max_keys <= DM_KEYS_SHORT) splits = 0;
-  else if (pairs * 2 > resident && max_keys > DM_LEAST * DM_KEYS) {
-    const long blocks = decode_mma_resident<DM_WARPS_SHORT, true>(d), by_keys = pairs * kf_ceil_div(max_keys, DM_LEAST * DM_KEYS);
-    splits = -(1 + kf_ceil_div(blocks < by_keys ? blocks : by_keys, pairs));
+  const long pairs = (long)n_items * nkv;
+  long per_sm = d == 256 ? decode_mma_blocks_per_sm<256, false, DM_WARPS>() : d == 128 ? decode_mma_blocks_per_sm<128, false, DM_WARPS>()
+              : d == 64 ? decode_mma_blocks_per_sm<64, false, DM_WARPS>() : d == 32 ? decode_mma_blocks_per_sm<32, false, DM_WARPS>()
+              : d == 16 ? decode_mma_blocks_per_sm<16, false, DM_WARPS>() : 0;
+  if (per_sm > MOST_BLOCKS_PER_SM) per_sm = MOST_BLOCKS_PER_SM;
+  if (per_sm < 1) per_sm = 1;
+  const long resident = kf_sm_count() * per_sm, by_len = pairs * kf_ceil_div(max_keys, DM_LEAST * DM_KEYS);
+  if (pairs > resident && max_keys <= DM_KEYS_SHORT) *splits_out = 0;
+  else if (max_keys <= DM_LEAST * DM_KEYS) *splits_out = 1;
+  else {
+    const int splits = 1 + kf_ceil_div(resident < by_len ? resident : by_len, pairs);
+    *splits_out = splits > MERGE_MAX_SPLITS ? MERGE_MAX_SPLITS : splits;
   }
-  *splits_out = splits;
   return KF_OK;
 }
 
@@ -1110,8 +1070,8 @@ KF_API int kf_attention_decode(const void* q, void* out, const void* pages, cons
   if (n_items <= 0) return KF_OK;
   if ((keep_first > 0 || sink || sig_bias) && ht != 0) return KF_ERR_SIZE;   // kept first tokens, the sink, sigmoid weights: tensor-core variant only
   if (window <= 0) keep_first = 0;
-  if (nkv < 1 || nh % nkv != 0 || page_size < 1 || n_splits < (ht == 0 ? -MERGE_MAX_SPLITS : 1) || n_splits == -1 || !kf_head_map_ok(nh, nkv, vsplit)) return KF_ERR_SIZE;
-  if ((n_splits > 1 || n_splits < 0) && (!partial || !counters)) return KF_ERR_SIZE;
+  if (nkv < 1 || nh % nkv != 0 || page_size < 1 || n_splits < (ht == 0 ? 0 : 1) || !kf_head_map_ok(nh, nkv, vsplit)) return KF_ERR_SIZE;
+  if (n_splits > 1 && (!partial || !counters)) return KF_ERR_SIZE;
   if (n_splits > MERGE_MAX_SPLITS || ht > MERGE_MAX_HEADS) return KF_ERR_SIZE;
   if (ht == 0) {                                     // tensor-core variant
     if (nh / nkv > 16) return KF_ERR_SIZE;
@@ -1149,9 +1109,9 @@ KF_API int kf_attention_decode_fused(const float* qkv, const float* cos_t, const
                                      float softcap, int window, int n_splits, float* partial, int* counters,
                                      cudaStream_t stream) {
   if (n_items <= 0) return KF_OK;
-  if (!qkv || nkv < 1 || nh % nkv != 0 || nh / nkv > 16 || page_size < 1 || n_splits < -MERGE_MAX_SPLITS || n_splits == -1) return KF_ERR_SIZE;
+  if (!qkv || nkv < 1 || nh % nkv != 0 || nh / nkv > 16 || page_size < 1 || n_splits < 0) return KF_ERR_SIZE;
   if (rot < 0 || rot > d || (rot & 1) || (rot > 0 && (!cos_t || !sin_t))) return KF_ERR_SIZE;
-  if ((n_splits > 1 || n_splits < 0) && (!partial || !counters)) return KF_ERR_SIZE;
+  if (n_splits > 1 && (!partial || !counters)) return KF_ERR_SIZE;
   if (n_splits > MERGE_MAX_SPLITS) return KF_ERR_SIZE;
 #define KF_MMA_ARGS qkv, cos_t, sin_t, rot, write_kv, nullptr, pages, items, n_items, positions, row_req, table, table_stride, page_size, nh, nkv, scale, softcap, window, 0, 0, 0, nullptr, n_splits, partial, counters, out, stream
   switch (d) {
