@@ -70,21 +70,21 @@ constexpr int MERGE_MAX_SPLITS = 64;
 // and then every thread sums four elements over the splits with sixteen 16-byte loads in flight.  Splits are summed in index order.
 template <int D, bool BASE2>
 __device__ __forceinline__ void merge_splits(const float* __restrict__ partial, size_t first_record, int n_heads,
-                                             int n_splits, int head_step, int split_step, __nv_bfloat16* __restrict__ o_first) {
+                                             int n_splits, __nv_bfloat16* __restrict__ o_first) {
   constexpr int PS = KF_PSTRIDE(D);
   __shared__ float s_w[MERGE_MAX_HEADS][MERGE_MAX_SPLITS];
-  const float* rec0 = partial + first_record * PS;              // record (h, s) at rec0 + (h * head_step + s * split_step) * PS
+  const float* rec0 = partial + first_record * PS;              // record (h, s) at rec0 + (h * n_splits + s) * PS
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n_warps = blockDim.x >> 5;
   if (n_splits <= 8) {
     for (int e = tid; e < n_heads * (D / 4); e += blockDim.x) {
       const int h = e / (D / 4), i4 = e - h * (D / 4);
-      const float* src = rec0 + (size_t)h * head_step * PS;
+      const float* src = rec0 + (size_t)h * n_splits * PS;
       float ms[8], ls[8];
       float4 v[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const bool in = u < n_splits;
-        const float* rec = src + (size_t)(in ? u : 0) * split_step * PS;
+        const float* rec = src + (size_t)(in ? u : 0) * PS;
         ms[u] = in ? __ldcg(rec + D) : -INFINITY;
         ls[u] = in ? __ldcg(rec + D + 1) : 0.f;
         v[u] = in ? __ldcg(reinterpret_cast<const float4*>(rec + i4 * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -112,9 +112,8 @@ __device__ __forceinline__ void merge_splits(const float* __restrict__ partial, 
   __shared__ float s_l[MERGE_MAX_HEADS][MERGE_MAX_SPLITS];
   for (int idx = tid; idx < n_heads * n_splits; idx += blockDim.x) {
     const int h = idx / n_splits, sp = idx - h * n_splits;
-    const float* rec = rec0 + ((size_t)h * head_step + (size_t)sp * split_step) * PS + D;
-    s_w[h][sp] = __ldcg(rec);
-    s_l[h][sp] = __ldcg(rec + 1);
+    s_w[h][sp] = __ldcg(rec0 + (size_t)idx * PS + D);
+    s_l[h][sp] = __ldcg(rec0 + (size_t)idx * PS + D + 1);
   }
   __syncthreads();
   for (int h = warp; h < n_heads; h += n_warps) {
@@ -137,13 +136,13 @@ __device__ __forceinline__ void merge_splits(const float* __restrict__ partial, 
   __syncthreads();
   for (int e = tid; e < n_heads * (D / 4); e += blockDim.x) {
     const int h = e / (D / 4), i4 = e - h * (D / 4);
-    const float* src = rec0 + (size_t)h * head_step * PS + i4 * 4;
+    const float* src = rec0 + (size_t)h * n_splits * PS + i4 * 4;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int sp = 0; sp < n_splits; sp += 16) {              // sixteen 16-byte loads in flight
       float4 v[16];
 #pragma unroll
       for (int u = 0; u < 16; ++u)
-        v[u] = sp + u < n_splits ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)(sp + u) * split_step * PS)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[u] = sp + u < n_splits ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)(sp + u) * PS)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int u = 0; u < 16; ++u) {
         const float c = sp + u < n_splits ? s_w[h][sp + u] : 0.f;
@@ -158,7 +157,7 @@ __device__ __forceinline__ void merge_splits(const float* __restrict__ partial, 
   }
 }
 
-// The same merge of a few records through shared memory: the records, part by part and head by head, lie behind one another, so all of
+// The same merge of a few records through shared memory: the records of a row's heads lie behind one another, so all of
 // them are asked for at once (16-byte cp.async) and the weights and sums are made from shared memory: one trip to L2 where
 // the loop above takes one for the maxima and another for every sixteen splits.  `buf` holds n_heads * n_splits records.
 // With the loads of the rotation in one trip too (below), a decode step of the 2B model at 8,192 tokens: one request 1.720 ->
@@ -168,38 +167,37 @@ __device__ __forceinline__ void merge_splits_shared(const float* __restrict__ pa
                                                     int n_splits, __nv_bfloat16* __restrict__ o_first, float* buf) {
   constexpr int PS = KF_PSTRIDE(D);
   const float* rec0 = partial + first_record * PS;
-  const int step = n_heads * PS;                                // from a part's record of a head to the next part's
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n_warps = blockDim.x >> 5;
   for (int i = tid; i < n_heads * n_splits * (PS / 4); i += blockDim.x) kf_mma::cp_async16(buf + 4 * i, rec0 + 4 * i, true);
   kf_mma::cp_async_commit();
   kf_mma::cp_async_wait<0>();
   __syncthreads();
   for (int h = warp; h < n_heads; h += n_warps) {
-    float* rec = buf + h * PS + D;              // maximum, sum; the maximum's place takes the weight
+    float* rec = buf + (size_t)h * n_splits * PS + D;              // maximum, sum; the maximum's place takes the weight
     float m = -INFINITY;
-    for (int sp = lane; sp < n_splits; sp += 32) m = fmaxf(m, rec[sp * step]);
+    for (int sp = lane; sp < n_splits; sp += 32) m = fmaxf(m, rec[sp * PS]);
     m = kf_warp_max(m);
     float l = 0.f;
     for (int sp = lane; sp < n_splits; sp += 32) {
-      const float ms = rec[sp * step];
+      const float ms = rec[sp * PS];
       const float c = (ms == -INFINITY) ? 0.f : exp2f(ms - m);
-      l += rec[sp * step + 1] * c;
-      rec[sp * step] = c;
+      l += rec[sp * PS + 1] * c;
+      rec[sp * PS] = c;
     }
     l = kf_warp_sum(l);                                            // a fixed order: lanes hold interleaved splits
     const float inv = l > 0.f ? 1.f / l : 0.f;
     __syncwarp();
-    for (int sp = lane; sp < n_splits; sp += 32) rec[sp * step] *= inv;
+    for (int sp = lane; sp < n_splits; sp += 32) rec[sp * PS] *= inv;
   }
   __syncthreads();
   for (int e = tid; e < n_heads * (D / 4); e += blockDim.x) {
     const int h = e / (D / 4), i4 = e - h * (D / 4);
-    const float* rec = buf + h * PS;
+    const float* rec = buf + (size_t)h * n_splits * PS;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
     for (int sp = 0; sp < n_splits; ++sp) {
-      const float4 v = *reinterpret_cast<const float4*>(rec + sp * step + i4 * 4);
-      const float c = rec[sp * step + D];
+      const float4 v = *reinterpret_cast<const float4*>(rec + sp * PS + i4 * 4);
+      const float c = rec[sp * PS + D];
       a.x += v.x * c; a.y += v.y * c; a.z += v.z * c; a.w += v.w * c;
     }
     uint2 packed;
@@ -392,23 +390,17 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  merge_splits<D, false>(partial, ((size_t)t * nh + h_first) * n_splits, h_count, n_splits, n_splits, 1, orow + (size_t)h_first * D);
+  merge_splits<D, false>(partial, ((size_t)t * nh + h_first) * n_splits, h_count, n_splits, orow + (size_t)h_first * D);
   if (threadIdx.x == 0) counters[cidx] = 0;
 }
 
 // ---- the tensor-core variant -----------------------------------------------------------------------------------
-// The query heads that share a kv head (up to 16) are the rows of one m16n8k16 tile, so a key costs a handful of
-// instructions instead of a warp's worth of shuffles.  Each of a block's warps walks its own 16-key tiles: the tile's key
-// and value rows are gathered from the pages into warp-private shared memory by cp.async, S = Q K^T (16 heads x 16 keys) and
-// O += P V run on mma.sync with 32-bit accumulators, the online softmax is the one of the prompt kernel.  Warps are merged
-// through shared memory in warp order, the parts of a row by the block that arrives last.
-//
-// The work is the tiles of all pairs (row, kv head), one pair behind the other.  Each block takes an equal run of them,
-// counted from the rows' own lengths on the device (a replayed step is planned for the longest context there may be), and
-// walks the pairs or parts of pairs in it; it requests the next one's first tiles before it merges its warps.  A part of a
-// pair leaves a record at place (block + pair), so a pair's records lie behind one another.  A run is DM_LEAST tiles or
-// more (fewer blocks then work), and long enough that a pair has at most MERGE_MAX_SPLITS records.
-// With whole pairs (n_splits 1) a block takes the pair of its own number.
+// Same work split (item, kv head, key split), but the query heads that share the kv head (up to 16) are the rows
+// of one m16n8k16 tile, so a key costs a handful of instructions instead of a warp's worth of shuffles.  Each of the
+// 4 warps walks its own 16-key tiles of the split: the tile's key and value rows are gathered from the pages into
+// warp-private shared memory by cp.async (double-buffered, so the next tile is in flight while this one is used),
+// S = Q K^T (16 heads x 16 keys) and O += P V run on mma.sync with 32-bit accumulators, the online softmax is the
+// one of the prompt kernel.  Warps are merged through shared memory in warp order, splits by the last block.
 constexpr int DM_WARPS = 8;                       // two per scheduler: a warp's tile is one chain of dependent instructions
 // More (row, kv head) pairs than blocks of eight warps fit the GPU, and short rows: a block then is mostly its start and its
 // merge, and blocks of four warps, two to an SM at heads of 256, cover each other's.  64 rows of 8 heads over 4 of 256, alone:
@@ -417,7 +409,6 @@ constexpr int DM_WARPS_SHORT = 4;
 constexpr int DM_KEYS_SHORT = 512;
 constexpr int DM_BUFS = 3;                        // buffers of one key tile or one value tile per warp: one in use, two in flight
 constexpr int DM_KEYS = 16;                       // keys per warp tile
-constexpr int DM_LEAST = 8;                       // tiles of a block's run, at least
 
 // With `qkv` given (the 32-bit q|k|v rows of the step, a row = [nh*D | nkv*D | nkv*D]) the kernel also does what the
 // rotate-and-append kernel would: it rotates its query heads itself, and the block whose key range holds the row's own
@@ -427,27 +418,14 @@ constexpr int DM_LEAST = 8;                       // tiles of a block's run, at 
 //
 // SIG: no softmax.  Key j counts with sigmoid(s_j + sig_bias[h]) and the weights are not normalized: the weighted sum is
 // what is stored.  In the merges this is a maximum of 0 everywhere and a sum of 1 that the first split holds.
-// Blocks per SM that registers must leave room for: as many as shared memory holds at heads of 128 and more, what the
-// sums of a thread allow at smaller ones.
-constexpr int dm_blocks_per_sm(int d, int warps) {
-  return warps == DM_WARPS ? (d >= 256 ? 1 : d >= 64 ? 2 : 3) : (d >= 256 ? 2 : d >= 128 ? 3 : d >= 64 ? 4 : 5);
-}
-
-// A block's run of tiles [at, end) of `total`, and the item it has reached, whose first tile is number `item_at`; the piece
-// of a pair that one walk takes; a pair that other blocks have parts of.  All in shared memory: one thread plans, and
-// registers are what limits the blocks per SM.
-struct DmRun { long total; int at, end, item, item_at, n_blocks, n_open; };
-struct DmPiece { int t, req, pos, kvh, pair, tile0, n_tiles, alone, more; };
-struct DmOpen { int pair, records, first_block, t; };
-
 template <int D, bool SIG, int DM_WARPS>
-__global__ void __launch_bounds__(DM_WARPS * 32, dm_blocks_per_sm(D, DM_WARPS))
+__global__ void __launch_bounds__(DM_WARPS * 32)
 attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restrict__ qkv, const float* __restrict__ cos_t,
                        const float* __restrict__ sin_t, int rot, int write_kv, __nv_bfloat16* pages,
                        const int* __restrict__ items, int n_items, const int* __restrict__ positions,
                        const int* __restrict__ row_req, const int* __restrict__ table, int table_stride, int page_size,
                        int nh, int nkv, float scale, float softcap, int window, int vsplit, int keep_first, int sink,
-                       const float* __restrict__ sig_bias, int whole_pairs, int apart, float* __restrict__ partial, int* __restrict__ counters,
+                       const float* __restrict__ sig_bias, int n_splits, float* __restrict__ partial, int* __restrict__ counters,
                        __nv_bfloat16* __restrict__ out) {
   using namespace kf_mma;
   kf_pdl_trigger();
@@ -460,136 +438,49 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
   __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(dm_smem);  // [16][D]
   __nv_bfloat16* sKV = sQ + 16 * D;                               // [warp][buffer][16][D]
   __shared__ float sm_ml[DM_WARPS][16][2];
-  __shared__ int s_last[2];
-  __shared__ DmRun s_run;
-  __shared__ DmPiece s_piece[2];
-  __shared__ DmOpen s_open[2];
+  __shared__ int s_last;
 
   // ---- the step's integers: written before the step's first kernel, so readable at once -------------------------------
+  const int item = blockIdx.x / nkv, kvh = blockIdx.x - item * nkv;
+  const int split = blockIdx.y;
   const int G = nh / nkv;
+  const int h_first = kvh * G;
+  const KfHeadMap hm = kf_head_map(h_first, kvh, nh, nkv, vsplit);   // with the rotation inside (qkv given) vsplit is 0
+  const int t = items ? items[item] : item;
+  const int req = row_req[t];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, tq = lane & 3;
-  auto row_of = [&](int item) { return items ? items[item] : item; };
-  // the tiles that each of a row's kv heads walks; 0 for rows of no request
-  auto tiles_of = [&](int item) {
-    const int t = row_of(item);
-    const int req = row_req[t], pos = positions[t], lo = kf_first_key(pos, window);
-    return req < 0 ? 0 : (pos + 1 - lo + (window > 0 ? min(keep_first, lo) : 0) + DM_KEYS - 1) / DM_KEYS;
-  };
-  // rows of no request: zeros
-  for (int item = whole_pairs ? blockIdx.x / nkv : blockIdx.x; item < n_items; item += gridDim.x) {
-    const int t = row_of(item);
-    if (row_req[t] < 0) {
-      kf_pdl_wait();
-      const int first = whole_pairs ? blockIdx.x % nkv * G * D : 0, n = whole_pairs ? G * D : nh * D;
-      for (int e = tid; e < n; e += blockDim.x) out[(size_t)t * nh * D + first + e] = __float2bfloat16_rn(0.f);
-    }
-    if (whole_pairs) break;
+  __nv_bfloat16* orow = out + (size_t)t * nh * D;
+  if (req < 0) {
+    kf_pdl_wait();
+    if (split == 0)
+      for (int e = tid; e < G * D; e += blockDim.x) orow[(size_t)h_first * D + e] = __float2bfloat16_rn(0.f);
+    return;
   }
+  const int pos = positions[t];
+  const int lo = kf_first_key(pos, window);
+  // Kept first tokens: keys [0, kept) are seen behind the window.  The keys are walked by a running index u in
+  // [lo_v, pos]: u >= lo is key u itself, u in [lo_v, lo) is key u - lo_v, so the walk below does not know of the gap.
+  const int kept = window > 0 ? min(keep_first, lo) : 0;
+  const int lo_v = lo - kept;
+  const int n_keys = pos + 1 - lo_v;
+  int per = (n_keys + n_splits - 1) / n_splits;
+  per = (per + 63) & ~63;
+  const int k_begin = lo_v + split * per;
+  const int k_end = min(pos + 1, k_begin + per);
+  const int n_tiles = k_end > k_begin ? (k_end - k_begin + DM_KEYS - 1) / DM_KEYS : 0;
+  // the tile that holds the row's own key: an earlier kernel of this step writes that key (or this block does)
+  const int own_tile = (pos >= k_begin && pos < k_end) ? (pos - k_begin) / DM_KEYS : -1;
 
-  // the piece from the run's place on, to the end of its pair or of the run, whichever comes first
-  auto plan = [&](DmPiece& p) {
-    DmRun r = s_run;
-    int nt = tiles_of(r.item);
-    while (r.at >= r.item_at + nt * nkv) {
-      r.item_at += nt * nkv;
-      nt = tiles_of(++r.item);
-    }
-    p.t = row_of(r.item);
-    p.req = row_req[p.t];
-    p.pos = positions[p.t];
-    p.kvh = (r.at - r.item_at) / nt;
-    p.pair = r.item * nkv + p.kvh;
-    p.tile0 = r.at - r.item_at - p.kvh * nt;
-    p.n_tiles = min(nt - p.tile0, r.end - r.at);
-    p.alone = p.n_tiles == nt;
-    if (!p.alone) {                                                // the blocks whose runs the pair's first and last tile are in
-      const int pair_at = r.at - p.tile0;
-      const int first = (int)(((long)(pair_at + 1) * r.n_blocks - 1) / r.total);
-      s_open[r.n_open++] = {p.pair, (int)(((long)(pair_at + nt) * r.n_blocks - 1) / r.total) - first + 1, first, p.t};   // at most two
-    }
-    r.at += p.n_tiles;
-    p.more = r.at < r.end;
-    s_run = r;
-  };
-  if (warp == 0) {
-    DmRun r = {};
-    if (whole_pairs) {
-      r.item = blockIdx.x / nkv;
-      const int nt = tiles_of(r.item);
-      r.at = blockIdx.x % nkv * nt;
-      r.end = r.at + nt;
-    } else {
-      int sum = 0, most = 0;
-      for (int i = lane; i < n_items; i += 32) {
-        const int n = tiles_of(i);
-        sum += n;
-        most = max(most, n);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
-      }
-      r.total = (long)sum * nkv;
-      const int least = max(DM_LEAST, (most + MERGE_MAX_SPLITS - 3) / (MERGE_MAX_SPLITS - 2));
-      r.n_blocks = (int)max(1l, min((long)gridDim.x, r.total / least));
-      if (blockIdx.x < r.n_blocks) {
-        r.at = (int)(r.total * blockIdx.x / r.n_blocks);
-        r.end = (int)(r.total * (blockIdx.x + 1) / r.n_blocks);
-      }
-      for (int i0 = 0; i0 < n_items && r.at < r.end; i0 += 32) {   // the item that tile `at` belongs to
-        const int own = i0 + lane < n_items ? tiles_of(i0 + lane) * nkv : 0;
-        int n = own;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, n, o);
-          if (lane >= o) n += v;
-        }
-        const unsigned in = __ballot_sync(0xffffffffu, r.item_at + n > r.at);
-        if (in) {
-          r.item = i0 + __ffs(in) - 1;
-          r.item_at += __shfl_sync(0xffffffffu, n - own, __ffs(in) - 1);
-          break;
-        }
-        r.item_at += __shfl_sync(0xffffffffu, n, 31);
-      }
-    }
-    if (lane == 0) {
-      s_run = r;
-      s_piece[0].n_tiles = 0;
-      if (r.at < r.end) plan(s_piece[0]);
-    }
-  }
-  __syncthreads();
-  if (s_piece[0].n_tiles == 0) return;
-
+  const int* tab = table + (size_t)req * table_stride;
   const size_t head_stride = (size_t)page_size * D;
+  const size_t v_off = (size_t)(hm.n_stored + hm.value - hm.key) * head_stride;
   __nv_bfloat16* my = sKV + (size_t)warp * DM_BUFS * TILE;        // [buffer]
 
-  // ---- the piece of a pair that is being walked ---------------------------------------------------------------------------
-  int t, pos, kvh, lo, lo_v, k_begin, k_end, own_tile, n_mine, key_head;
-  const int* tab;
-  size_t v_off;
-  auto take_piece = [&](const DmPiece& p) {
-    t = p.t, pos = p.pos, kvh = p.kvh;
-    const KfHeadMap hm = kf_head_map(kvh * G, kvh, nh, nkv, vsplit);   // with the rotation inside (qkv given) vsplit is 0
-    key_head = hm.key;
-    // Kept first tokens: keys [0, kept) are seen behind the window.  The keys are walked by a running index u in
-    // [lo_v, pos]: u >= lo is key u itself, u in [lo_v, lo) is key u - lo_v, so the walk below does not know of the gap.
-    lo = kf_first_key(pos, window);
-    lo_v = lo - (window > 0 ? min(keep_first, lo) : 0);
-    k_begin = lo_v + p.tile0 * DM_KEYS;
-    k_end = min(pos + 1, k_begin + p.n_tiles * DM_KEYS);
-    // the tile that holds the row's own key: an earlier kernel of this step writes that key (or this block does)
-    own_tile = pos < k_end ? (pos - k_begin) / DM_KEYS : -1;
-    tab = table + (size_t)p.req * table_stride;
-    v_off = (size_t)(hm.n_stored + hm.value - hm.key) * head_stride;
-    // A warp walks its tiles (warp, warp + DM_WARPS, ...) as the sequence K0 V0 K1 V1 ...: item n is the keys (n even) or
-    // the values (n odd) of its tile n / 2 and lands in buffer n % DM_BUFS.
-    n_mine = p.n_tiles > warp ? (p.n_tiles - warp + DM_WARPS - 1) / DM_WARPS : 0;
-  };
-  const int n_stored = vsplit > 0 ? nkv / vsplit : nkv;
+  // A warp walks its tiles (warp, warp + DM_WARPS, ...) as the sequence K0 V0 K1 V1 ...: item n is the keys (n even) or
+  // the values (n odd) of its tile n / 2 and lands in buffer n % DM_BUFS.
+  const int n_mine = n_tiles > warp ? (n_tiles - warp + DM_WARPS - 1) / DM_WARPS : 0;
+  const int n_loads = 2 * n_mine;
   long row_base = -1;                                             // lanes 0..15: where key j0 + lane of the item's tile lies
   auto load_item = [&](int n, int buf) {
     const int tile = warp + (n >> 1) * DM_WARPS;
@@ -601,7 +492,7 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
       if (u < k_end) {
         const int j = u >= lo ? u : u - lo_v;
         const int page = tab[j / page_size];
-        if (page >= 0) row_base = ((long)page * 2 * n_stored + key_head) * (long)head_stride + (long)(j % page_size) * D;
+        if (page >= 0) row_base = ((long)page * 2 * hm.n_stored + hm.key) * (long)head_stride + (long)(j % page_size) * D;
       }
     }
     __nv_bfloat16* dst = my + (size_t)buf * TILE;
@@ -618,24 +509,16 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
     }
   };
 
-  // the first items of this warp: those of the tile with the row's own key, or the others (keys of earlier steps)
-  auto request_first = [&](bool own) {
+  // the first items of this warp, except those of the tile with the row's own key: keys of earlier steps
 #pragma unroll
-    for (int n = 0; n < DM_BUFS; ++n)
-      if (n < 2 * n_mine && (warp + (n >> 1) * DM_WARPS == own_tile) == own) load_item(n, n);
-  };
-  take_piece(s_piece[0]);
-  request_first(false);
+  for (int n = 0; n < DM_BUFS; ++n)
+    if (n < n_loads && warp + (n >> 1) * DM_WARPS != own_tile) load_item(n, n);
   if (qkv != nullptr)
     for (int idx = G * CH + tid; idx < 16 * CH; idx += blockDim.x)
       *reinterpret_cast<uint4*>(tile_ptr<D>(sQ, idx / CH, idx % CH)) = make_uint4(0, 0, 0, 0);
   kf_pdl_wait();
   q = kf_produced(q), qkv = kf_produced(qkv), cos_t = kf_produced(cos_t), sin_t = kf_produced(sin_t);
 
-  for (int walk = 0;; walk ^= 1) {
-  const DmPiece& piece = s_piece[walk];
-  const int h_first = kvh * G;
-  __nv_bfloat16* orow = out + (size_t)t * nh * D;
   if (qkv != nullptr) {
     // ---- Q: rotated here; rows 0..G-1 are the heads of this kv head, the rest of the 16 rows are zero (written above) -----
     const float* in = qkv + (size_t)t * (nh + 2 * nkv) * D;
@@ -692,23 +575,23 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
     }
   } else {
     // ---- Q as the rotate-and-append kernel left it ---------------------------------------------------------------------
-    const KfHeadMap hq = kf_head_map(h_first, kvh, nh, nkv, vsplit);
     for (int idx = tid; idx < 16 * CH; idx += blockDim.x) {
       const int r = idx / CH, c = idx - r * CH;
       uint4 v = make_uint4(0, 0, 0, 0);
-      if (r < G) v = *reinterpret_cast<const uint4*>(q + ((size_t)t * hq.n_query + hq.query + r) * D + c * 8);
+      if (r < G) v = *reinterpret_cast<const uint4*>(q + ((size_t)t * hm.n_query + hm.query + r) * D + c * 8);
       *reinterpret_cast<uint4*>(tile_ptr<D>(sQ, r, c)) = v;
     }
   }
   __syncthreads();                                                // Q in place; the new key and value are in the page
-  if (tid == DM_WARPS * 32 - 32 && piece.more) plan(s_piece[walk ^ 1]);   // in the last warp, which has a tile less if any has
-  __syncwarp();
-  // the own-key tile, if it is one of this warp's first tiles; then all first items are one group, and empty groups
-  // keep the count of one group per item that the loop below relies on
-  request_first(true);
+  {
+    // the own-key tile, if it is one of this warp's first tiles; then all first items are one group, and empty groups
+    // keep the count of one group per item that the loop below relies on
 #pragma unroll
-  for (int n = 0; n < DM_BUFS; ++n) cp_async_commit();
-  const int n_loads = 2 * n_mine;
+    for (int n = 0; n < DM_BUFS; ++n)
+      if (n < n_loads && warp + (n >> 1) * DM_WARPS == own_tile) load_item(n, n);
+#pragma unroll
+    for (int n = 0; n < DM_BUFS; ++n) cp_async_commit();
+  }
 
   float o_acc[NT_O][4];
 #pragma unroll
@@ -837,29 +720,27 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
     l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
     l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 2);
   }
-  __syncthreads();                                                // the ring and Q have been read by everyone
-  float* sm_o = reinterpret_cast<float*>(sKV) + (apart ? (size_t)DM_WARPS * DM_BUFS * TILE / 2 : 0);      // [warp][G][D]
+  __syncthreads();
+  float* sm_o = reinterpret_cast<float*>(sKV);                     // [warp][G][D]
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const int row = g + r * 8;
     if (row < G) {
 #pragma unroll
-      for (int n = 0; n < NT_O; ++n)
-        *reinterpret_cast<float2*>(sm_o + ((size_t)warp * G + row) * D + n * 8 + tq * 2) = make_float2(o_acc[n][2 * r], o_acc[n][2 * r + 1]);
-      if (tq == 0) { sm_ml[warp][row][0] = SIG ? 0.f : m_run[r]; sm_ml[warp][row][1] = SIG ? (warp == 0 && piece.tile0 == 0) : l_run[r]; }
+      for (int n = 0; n < NT_O; ++n) {
+        float* dst = sm_o + ((size_t)warp * G + row) * D + n * 8 + tq * 2;
+        dst[0] = o_acc[n][2 * r];
+        dst[1] = o_acc[n][2 * r + 1];
+      }
+      if (tq == 0) { sm_ml[warp][row][0] = SIG ? 0.f : m_run[r]; sm_ml[warp][row][1] = SIG ? (warp == 0 && split == 0) : l_run[r]; }
     }
   }
   __syncthreads();
-  const bool alone = piece.alone, more = piece.more;
-  const bool sink_here = sink && piece.tile0 == 0;
-  float* rec0 = partial + (size_t)(blockIdx.x + piece.pair) * G * PSTRIDE;
-  if (more && apart) {                                             // the next piece's first tiles, while this one is merged
-    take_piece(s_piece[walk ^ 1]);
-    request_first(false);
-  }
+  const size_t rec_base = (((size_t)t * nh + h_first) * n_splits + split) * PSTRIDE;
   for (int e = tid; e < G * D; e += blockDim.x) {
     const int h = e / D, i = e - h * D;
-    // the sink (a key of score 0 without a value) joins the first part like one more warp: maximum 0, sum 1, no row
+    // the sink (a key of score 0 without a value) joins the first split like one more warp: maximum 0, sum 1, no row
+    const bool sink_here = sink && split == 0;
     float m = sink_here ? 0.f : -INFINITY;
     for (int w = 0; w < DM_WARPS; ++w) m = fmaxf(m, sm_ml[w][h][0]);
     float l = sink_here ? exp2f(-m) : 0.f, a = 0.f;
@@ -869,44 +750,28 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
       l += sm_ml[w][h][1] * c;
       a += sm_o[((size_t)w * G + h) * D + i] * c;
     }
-    if (alone) {
+    if (n_splits == 1) {
       orow[(size_t)(h_first + h) * D + i] = __float2bfloat16_rn(l > 0.f ? a / l : 0.f);
     } else {
-      float* rec = rec0 + (size_t)h * PSTRIDE;
+      float* rec = partial + rec_base + (size_t)h * n_splits * PSTRIDE;
       rec[i] = a;
       if (i == 0) { rec[D] = m; rec[D + 1] = l; }
     }
   }
-  if (!more) break;
-  if (!apart) {
-    __syncthreads();
-    take_piece(s_piece[walk ^ 1]);
-    request_first(false);
-  }
-  }
-  const int n_open = s_run.n_open;
-  if (n_open == 0) return;
+  if (n_splits == 1) return;
   __threadfence();
   __syncthreads();
-  if (tid < n_open) s_last[tid] = atomicAdd(&counters[s_open[tid].pair], 1) == s_open[tid].records - 1;
+  const int cidx = item * nkv + kvh;
+  if (tid == 0) s_last = (atomicAdd(&counters[cidx], 1) == n_splits - 1);
   __syncthreads();
-#pragma unroll 1
-  for (int o = 0; o < n_open; ++o) {
-    if (!s_last[o]) continue;
-    __threadfence();                                               // maxima here are base-2 scaled
-    const DmOpen open = s_open[o];
-    const size_t first_record = (size_t)(open.first_block + open.pair) * G;
-    __nv_bfloat16* o_first = out + ((size_t)open.t * nh + (size_t)(open.pair % nkv) * G) * D;
-    if (open.records > 8 && (size_t)G * open.records * PSTRIDE * sizeof(float) <= (size_t)DM_WARPS * DM_BUFS * TILE * sizeof(__nv_bfloat16))
-      merge_splits_shared<D>(partial, first_record, G, open.records, o_first, reinterpret_cast<float*>(sKV));
-    else
-      merge_splits<D, true>(partial, first_record, G, open.records, 1, G, o_first);
-    if (tid == 0) counters[open.pair] = 0;
-    __syncthreads();
-  }
+  if (!s_last) return;
+  __threadfence();                                               // maxima here are base-2 scaled
+  if (n_splits > 8 && (size_t)G * n_splits * PSTRIDE * sizeof(float) <= (size_t)DM_WARPS * DM_BUFS * TILE * sizeof(__nv_bfloat16))
+    merge_splits_shared<D>(partial, ((size_t)t * nh + h_first) * n_splits, G, n_splits, orow + (size_t)h_first * D, sm_o);
+  else
+    merge_splits<D, true>(partial, ((size_t)t * nh + h_first) * n_splits, G, n_splits, orow + (size_t)h_first * D);
+  if (tid == 0) counters[cidx] = 0;
 }
-
-constexpr size_t dm_smem_bytes(int d, int warps) { return (size_t)(16 * d + warps * DM_BUFS * DM_KEYS * d) * 2; }
 
 // Blocks of the tensor-core decode kernel that one SM holds at a time (shared memory or registers, whichever binds), as
 // the runtime reports it; also sets the kernel's shared-memory limit.  0 if that fails.
@@ -914,11 +779,9 @@ template <int D, bool SIG, int DM_WARPS>
 int decode_mma_blocks_per_sm() {
   static int cached = -1;
   if (cached >= 0) return cached;
-  const size_t smem = dm_smem_bytes(D, DM_WARPS);
-  cudaFuncAttributes fa;
+  const size_t smem = (size_t)(16 * D + DM_WARPS * DM_BUFS * DM_KEYS * D) * 2;
   int n = 0;
-  if (cudaFuncGetAttributes(&fa, attn_decode_mma_kernel<D, SIG, DM_WARPS>) != cudaSuccess ||
-      cudaFuncSetAttribute(attn_decode_mma_kernel<D, SIG, DM_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes) != cudaSuccess ||
+  if (cudaFuncSetAttribute(attn_decode_mma_kernel<D, SIG, DM_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_decode_mma_kernel<D, SIG, DM_WARPS>, DM_WARPS * 32, smem) != cudaSuccess) {
     kf_record_cuda_error(cudaGetLastError());
     return 0;
@@ -927,46 +790,18 @@ int decode_mma_blocks_per_sm() {
   return n;
 }
 
-// Whether the warps' results of G heads get shared memory of their own: where that costs no resident block.
-template <int D, bool SIG, int DM_WARPS>
-bool decode_mma_apart(int G) {
-  static signed char cached[17] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
-  if (cached[G] < 0) {
-    int n = 0;
-    cudaFuncAttributes fa;
-    const size_t smem = dm_smem_bytes(D, DM_WARPS) + (size_t)DM_WARPS * G * D * sizeof(float);
-    if (cudaFuncGetAttributes(&fa, attn_decode_mma_kernel<D, SIG, DM_WARPS>) != cudaSuccess || smem + fa.sharedSizeBytes > 227 * 1024 ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_decode_mma_kernel<D, SIG, DM_WARPS>, DM_WARPS * 32, smem) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-    cached[G] = n >= decode_mma_blocks_per_sm<D, SIG, DM_WARPS>();
-  }
-  return cached[G] != 0;
-}
-
-constexpr int MOST_BLOCKS_PER_SM = 8;
-
-// n_splits 1: a block per pair.  More: as many blocks as the GPU holds, but no more than the caller's n_splits - 1 for each pair,
-// so that the records (one per block and one per pair, at most) fit what n_splits records for each pair take.
 template <int D, bool SIG, int DM_WARPS>
 int launch_decode_mma_warps(const float* qkv, const float* cos_t, const float* sin_t, int rot, int write_kv,
                       const void* q, const void* pages, const int* items, int n_items, const int* positions,
                       const int* row_req, const int* table, int table_stride, int page_size, int nh, int nkv, float scale,
                       float softcap, int window, int vsplit, int keep_first, int sink, const float* sig_bias, int n_splits,
                       float* partial, int* counters, void* out, cudaStream_t stream) {
-  int per_sm = decode_mma_blocks_per_sm<D, SIG, DM_WARPS>();
-  if (per_sm < 1) return KF_ERR_SETUP;
-  if (per_sm > MOST_BLOCKS_PER_SM) per_sm = MOST_BLOCKS_PER_SM;
-  const int G = nh / nkv;
-  const bool apart = decode_mma_apart<D, SIG, DM_WARPS>(G);
-  const size_t smem = dm_smem_bytes(D, DM_WARPS) + (apart ? (size_t)DM_WARPS * G * D * sizeof(float) : 0);
-  const long pairs = (long)n_items * nkv, most = (long)kf_sm_count() * per_sm;
-  const long blocks = n_splits <= 1 ? pairs : pairs * (n_splits - 1) < most ? pairs * (n_splits - 1) : most;
-  kf_launch(attn_decode_mma_kernel<D, SIG, DM_WARPS>, dim3((unsigned)blocks), dim3(DM_WARPS * 32), smem, stream,
+  const size_t smem = (size_t)(16 * D + DM_WARPS * DM_BUFS * DM_KEYS * D) * 2;
+  if (decode_mma_blocks_per_sm<D, SIG, DM_WARPS>() < 1) return KF_ERR_SETUP;
+  kf_launch(attn_decode_mma_kernel<D, SIG, DM_WARPS>, dim3(n_items * nkv, n_splits), dim3(DM_WARPS * 32), smem, stream,
             (const __nv_bfloat16*)q, qkv, cos_t, sin_t, rot, write_kv, (__nv_bfloat16*)const_cast<void*>(pages), items, n_items,
-            positions, row_req, table, table_stride, page_size, nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias,
-            n_splits <= 1 ? 1 : 0, apart ? 1 : 0, partial, counters, (__nv_bfloat16*)out);
+            positions, row_req, table, table_stride, page_size, nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias, n_splits,
+            partial, counters, (__nv_bfloat16*)out);
   KF_CHECK_LAUNCH();
   return KF_OK;
 }
@@ -1020,25 +855,23 @@ static int g_forced_splits = 0;
 KF_API void kf_set_attention_decode_splits(int splits) { g_forced_splits = splits; }
 #endif
 
-// splits_out: 1 for a block per (row, kv head) pair; 0 for the same in blocks of fewer warps (short rows, more of them than the
-// GPU holds blocks); otherwise the pairs' keys are cut evenly between the blocks that the GPU holds, and splits_out is how
-// many records a pair needs on average (`launch_decode_mma_warps`).  kf_attention_decode (ht = 0) and
-// kf_attention_decode_fused take it as it is.
+// splits_out: how many parts a row's keys are cut into; 0 for one part in blocks of fewer warps (short rows, more of them than
+// the GPU holds blocks), which kf_attention_decode (ht = 0) and kf_attention_decode_fused take as it is.
 KF_API int kf_attention_decode_mma_plan(int n_items, int nh, int nkv, int d, int max_keys, int* splits_out) {
   if (g_forced_splits > 0) { *splits_out = g_forced_splits; return KF_OK; }
-  const long pairs = (long)n_items * nkv;
+  const long blocks = (long)n_items * nkv;
+  // fill one wave: as many splits as resident blocks allow
   long per_sm = d == 256 ? decode_mma_blocks_per_sm<256, false, DM_WARPS>() : d == 128 ? decode_mma_blocks_per_sm<128, false, DM_WARPS>()
               : d == 64 ? decode_mma_blocks_per_sm<64, false, DM_WARPS>() : d == 32 ? decode_mma_blocks_per_sm<32, false, DM_WARPS>()
               : d == 16 ? decode_mma_blocks_per_sm<16, false, DM_WARPS>() : 0;
-  if (per_sm > MOST_BLOCKS_PER_SM) per_sm = MOST_BLOCKS_PER_SM;
+  if (per_sm > 8) per_sm = 8;
   if (per_sm < 1) per_sm = 1;
-  const long resident = kf_sm_count() * per_sm, by_len = pairs * kf_ceil_div(max_keys, DM_LEAST * DM_KEYS);
-  if (pairs > resident && max_keys <= DM_KEYS_SHORT) *splits_out = 0;
-  else if (max_keys <= DM_LEAST * DM_KEYS) *splits_out = 1;
-  else {
-    const int splits = 1 + kf_ceil_div(resident < by_len ? resident : by_len, pairs);
-    *splits_out = splits > MERGE_MAX_SPLITS ? MERGE_MAX_SPLITS : splits;
-  }
+  int splits = (int)((kf_sm_count() * per_sm) / blocks);
+  const int by_len = (max_keys + 255) / 256;
+  if (splits > by_len) splits = by_len;
+  if (splits > 64) splits = 64;
+  if (splits < 1) splits = blocks > kf_sm_count() * per_sm && max_keys <= DM_KEYS_SHORT ? 0 : 1;
+  *splits_out = splits;
   return KF_OK;
 }
 
