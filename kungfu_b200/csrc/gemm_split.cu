@@ -18,8 +18,8 @@
 // and leaves the parts' sums in memory for `sum_parts_kernel`.  Either way an output's sum is the chunks of a part in
 // ascending k and the parts in ascending order, whatever T is, so a row does not depend on the rows beside it.
 //
-// A row of x or of w that holds an infinity or NaN (or nothing but numbers below 2^-90, whose lower planes would leave
-// bfloat16's range) is multiplied with plain FMAs instead, by the threads that own its outputs.
+// A sum that is not finite, or below 2^-60 and not zero, is made again with plain FMAs by the thread that owns it: an infinity
+// has no planes (its product with a plane of zeros would be NaN), and lower planes of numbers below 2^-110 leave bfloat16's range.
 #include "common.cuh"
 #include "tc_common.cuh"
 
@@ -31,11 +31,9 @@ constexpr int CK = 64;                                          // k of a chunk:
 constexpr int W_STAGE = BM * CK * 4;                            // 32 KB: two boxes of 128 rows x 32 floats
 constexpr int A_COLS = 3 * CK / 2;                              // tensor-memory columns of a chunk's three weight planes
 constexpr int CUTTERS = 256;                                    // threads that cut weights: two per feature
-constexpr int FLAG_SETS = 8;                                    // units by which converters may be ahead of the sums, and more
 constexpr int SMALL_T = 16, LARGE_T = 160;                      // rows of a tile, at most
-constexpr uint32_t TINY = 0x12800000u;                          // 2^-90
 
-__device__ __forceinline__ bool odd_range(uint32_t largest) { return largest >= 0x7f800000u || (largest != 0u && largest < TINY); }
+__device__ __forceinline__ bool plain_needed(float v) { return !(fabsf(v) >= 8.67361738e-19f && fabsf(v) <= 3.4e38f) && v != 0.f; }   // 2^-60
 
 // Two neighbours cut into three words of bfloat16 pairs; the cuts are exact.
 __device__ __forceinline__ void cut_pair(float a, float b, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
@@ -48,38 +46,22 @@ __device__ __forceinline__ void cut_pair(float a, float b, uint32_t& p1, uint32_
   p3 = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 
-// The three planes [3][T][pitch] of x [T, K], K a multiple of 4, zeros from K to the pitch, and per row and part of K whether
-// it needs the plain product (row_odd [parts][T]).  A block per row.
+// The three planes [3][T][pitch] of x [T, K], K a multiple of 4, zeros from K to the pitch.  A block per row.
 __global__ void __launch_bounds__(256)
-split_rows_kernel(const float* x, __nv_bfloat16* planes, int* row_odd, int T, int K, int pitch, int parts) {
+split_rows_kernel(const float* x, __nv_bfloat16* planes, int T, int K, int pitch) {
   kf_pdl_trigger();
   kf_pdl_wait();
-  const int t = blockIdx.x, chunks = (K + CK - 1) / CK;
+  const int t = blockIdx.x;
   const float4* src = reinterpret_cast<const float4*>(x + (size_t)t * K);
-  __shared__ uint32_t s_largest[8];
-  if (threadIdx.x < 8) s_largest[threadIdx.x] = 0u;
-  __syncthreads();
-  uint32_t largest = 0;
-  int part = 0;
 #pragma unroll 4
   for (int i = threadIdx.x; i < pitch / 4; i += 256) {
-    const int z = min(parts - 1, ((4 * i / CK + 1) * parts - 1) / chunks);
-    if (z != part) {
-      if (largest) atomicMax(&s_largest[part], largest);
-      largest = 0, part = z;
-    }
     const float4 v = 4 * i < K ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     uint2 p[3];
     cut_pair(v.x, v.y, p[0].x, p[1].x, p[2].x);
     cut_pair(v.z, v.w, p[0].y, p[1].y, p[2].y);
-    largest = max(max(largest, __float_as_uint(fabsf(v.x))), __float_as_uint(fabsf(v.y)));
-    largest = max(max(largest, __float_as_uint(fabsf(v.z))), __float_as_uint(fabsf(v.w)));
 #pragma unroll
     for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(planes + ((size_t)j * T + t) * pitch + 4 * i) = p[j];
   }
-  if (largest) atomicMax(&s_largest[part], largest);
-  __syncthreads();
-  if (threadIdx.x < parts) row_odd[(size_t)threadIdx.x * T + t] = odd_range(s_largest[threadIdx.x]);
 }
 
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
@@ -121,7 +103,6 @@ struct SplitArgs {
   const float* w;
   void* out;
   float* partial;                                                // [parts][T][N], where a launch leaves the parts' sums
-  const int* row_odd;
   int* error_flag;
   float softcap;
   int T, N, K, parts, bn, w_stages;                              // bn: rows of a tile, 16 or a multiple of 32
@@ -158,8 +139,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   uint64_t* acc_free = done + 2;                                  // [2] its accumulator has been read
   uint32_t* tmem_slot = (uint32_t*)(acc_free + 2);
   volatile int* s_abort = (volatile int*)(tmem_slot + 1);
-  uint32_t* s_rows = tmem_slot + 2;                               // rows of x with: something not finite, 2^-90 or more, not zero
-  volatile uint8_t* s_odd = (volatile uint8_t*)(tmem_slot + 6);   // [FLAG_SETS][CUTTERS] features that need the plain product
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int chunks = (a.K + CK - 1) / CK;
@@ -171,7 +150,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     for (int s = 0; s < S::X_STAGES; ++s) { mbar_init(&x_full[s], LARGE ? 1 : 128); mbar_init(&x_empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&a_full[b], CUTTERS); mbar_init(&done[b], 1); mbar_init(&acc_free[b], 128 * S::SUM_GROUPS); }
     *s_abort = 0;
-    s_rows[0] = s_rows[1] = s_rows[2] = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -279,13 +257,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     // ---- weights: two threads per feature, 32 k each at a time from shared memory into three planes of tensor memory ----------
     const int quarter = warp & 3, half = (warp - 2) >> 2, r = quarter * 32 + lane;
     const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
-    int c = 0, slot = 0, set = 0;
+    int c = 0, slot = 0;
     uint32_t ph = 0;
     bool ok = true;
     for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
       int first, last;
       range(unit, first, last);
-      uint32_t largest = 0;
       for (int i = first; i < last; ++i, ++c) {
         const int b = c & 1;
         ok = mbar_wait(&w_full[slot], ph) && (c < 2 || mbar_wait(&done[b], (uint32_t)((c >> 1) - 1) & 1)) && !*s_abort;
@@ -297,8 +274,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
 #pragma unroll
         for (int j = 0; j < 8; ++j) {                             // 16-byte piece j of a row stands at j ^ (row % 8)
           const float4 v = *reinterpret_cast<const float4*>(row + ((j ^ (r & 7)) << 4));
-          largest = max(max(largest, __float_as_uint(fabsf(v.x))), __float_as_uint(fabsf(v.y)));
-          largest = max(max(largest, __float_as_uint(fabsf(v.z))), __float_as_uint(fabsf(v.w)));
           cut_pair(v.x, v.y, p1[2 * j], p2[2 * j], p3[2 * j]);
           cut_pair(v.z, v.w, p1[2 * j + 1], p2[2 * j + 1], p3[2 * j + 1]);
         }
@@ -306,13 +281,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         tmem_st16(dst + CK / 2, p2);
         tmem_st16(dst + CK, p3);
         mbar_arrive(&w_empty[slot]);
-        if (i + 1 == last) s_odd[set * CUTTERS + threadIdx.x - 64] = odd_range(largest);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         mbar_arrive(&a_full[b]);
         if (++slot == ws) { slot = 0; ph ^= 1; }
       }
-      set = (set + 1) % FLAG_SETS;
     }
     __syncwarp();
   } else {
@@ -321,21 +294,23 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     const int fl = quarter * 32 + lane;
     const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
     const int cols = bn / S::SUM_GROUPS, col0 = group * cols;
-    int c = 0, set = 0;
+    int c = 0;
     bool ok = true;
-    kf_pdl_wait();                                                // before anything is written, and for x or the rows' flags
+    kf_pdl_wait();                                                // before anything is written, and for x
     // The small tile: these 128 threads cut x.  Thread i has 4 floats at k 4 (i % 16) of rows i / 16 and i / 16 + 8; a chunk's
     // stage is its accumulator's number, free when its products are done; the next chunk's floats are on their way meanwhile.
     const int ct = threadIdx.x - 64 - CUTTERS, cj = ct & 15;
     int xu = blockIdx.x, xc = 0, xl = 0;
-    float4 xv[2];
-    uint32_t told = 0;                                            // what this thread has told of its rows
+    float4 xv[2], xn[2];                                          // the next chunk's floats and those of the one after
+    int au = blockIdx.x, ac = 0, al = 0;                          // where the asking is
     auto ask_x = [&]() {
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const int t = (ct >> 4) + 8 * u, k = xc * CK + 4 * cj;
-        xv[u] = xu < n_units && t < a.T && k < a.K ? *reinterpret_cast<const float4*>(a.x + (size_t)t * a.K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const int t = (ct >> 4) + 8 * u, k = ac * CK + 4 * cj;
+        xv[u] = xn[u];
+        xn[u] = au < n_units && t < a.T && k < a.K ? *reinterpret_cast<const float4*>(a.x + (size_t)t * a.K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
+      if (au < n_units && ++ac == al) { au += gridDim.x; if (au < n_units) range(au, ac, al); }
     };
     auto cut_x = [&](int stage) {
       if (xu >= n_units) return;
@@ -345,14 +320,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         uint2 q[3];
         cut_pair(xv[u].x, xv[u].y, q[0].x, q[1].x, q[2].x);
         cut_pair(xv[u].z, xv[u].w, q[0].y, q[1].y, q[2].y);
-        const uint32_t big = max(max(__float_as_uint(fabsf(xv[u].x)), __float_as_uint(fabsf(xv[u].y))),
-                                 max(__float_as_uint(fabsf(xv[u].z)), __float_as_uint(fabsf(xv[u].w))));
-        const uint32_t news = ((big >= 0x7f800000u ? 1u : 0u) | (big >= TINY ? 2u : 0u) | (big != 0u ? 4u : 0u)) << (3 * u);
-        if (news & ~told) {
-          told |= news;
-#pragma unroll
-          for (int e = 0; e < 3; ++e) if (news >> (3 * u + e) & 1u) atomicOr(&s_rows[e], 1u << t);
-        }
         uint8_t* dst = sx + (size_t)stage * x_stage + t * 128 + (((cj >> 1) ^ (t & 7)) << 4) + (cj & 1) * 8;
 #pragma unroll
         for (int e = 0; e < 3; ++e) *reinterpret_cast<uint2*>(dst + e * (SMALL_T * CK * 2)) = q[e];
@@ -364,6 +331,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     };
     if (!LARGE) {
       if (xu < n_units) range(xu, xc, xl);
+      ac = xc, al = xl;
+      ask_x();
       ask_x();
       cut_x(0);
       cut_x(1);
@@ -402,16 +371,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       // ---- the unit's outputs: the parts of a product in a cluster through shared memory, else to memory -----------------------
       const int z = unit % a.parts, t0 = (unit / a.parts % n_tt) * bn, f = unit / a.parts / n_tt * BM + fl;
       const int k0 = first * CK, k1 = min(a.K, last * CK);
-      const int at = set * CUTTERS + ((quarter + 2) & 3) * 32 + lane;   // the cutting threads of this feature: warps 2-5 and 6-9
-      const bool f_odd = (s_odd[at] | s_odd[at + 128]) != 0;
-      set = (set + 1) % FLAG_SETS;
-      uint32_t t_odd[(S::COLS + 31) / 32];
-#pragma unroll
-      for (int q = 0; q < (S::COLS + 31) / 32; ++q) {
-        const int t = t0 + col0 + 32 * q + lane;
-        t_odd[q] = LARGE ? __ballot_sync(0xffffffffu, 32 * q + lane < cols && t < a.T && __ldcg(a.row_odd + (size_t)z * a.T + t) != 0)
-                         : *(volatile uint32_t*)&s_rows[0] | (*(volatile uint32_t*)&s_rows[2] & ~*(volatile uint32_t*)&s_rows[1]);
-      }
       const bool in_cluster = !LARGE && a.parts > 1;
       float* red = reinterpret_cast<float*>(sw);                  // [16][128]: the ring is free by then
       auto put = [&](int j, float v) {
@@ -422,20 +381,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
           else kf_store((TO*)a.out, (size_t)t * a.N + f, kf_softcap(v, a.softcap));
         }
       };
+      unsigned long long again = 0ull;                            // columns whose sums are made again: rare
 #pragma unroll
       for (int j = 0; j < S::COLS; ++j)
-        if ((j & ~7) < cols) put(j, sum[j]);
-      bool rows_odd = false;
-#pragma unroll
-      for (int q = 0; q < (S::COLS + 31) / 32; ++q) rows_odd |= t_odd[q] != 0u;
-      if ((f_odd || rows_odd) && f < a.N) {                       // rare: these sums again, by plain FMAs
-        for (int j = 0; j < cols; ++j) {
-          uint32_t m = 0;
-#pragma unroll
-          for (int q = 0; q < (S::COLS + 31) / 32; ++q) m = (j >> 5) == q ? t_odd[q] : m;
-          if (t0 + col0 + j < a.T && (f_odd || (m >> (j & 31) & 1u)))
-            put(j, plain_sum(a.x + (size_t)(t0 + col0 + j) * a.K + k0, a.w + (size_t)f * a.K + k0, k1 - k0));
+        if ((j & ~7) < cols) {
+          put(j, sum[j]);
+          if (plain_needed(sum[j])) again |= 1ull << j;
         }
+      if (again && f < a.N) {
+#pragma unroll 1
+        for (int j = 0; j < cols; ++j)
+          if ((again >> j & 1ull) && t0 + col0 + j < a.T)
+            put(j, plain_sum(a.x + (size_t)(t0 + col0 + j) * a.K + k0, a.w + (size_t)f * a.K + k0, k1 - k0));
       }
     }
     __syncwarp();
@@ -519,7 +476,7 @@ template <bool LARGE, typename TO>
 int launch_split(const CUtensorMap& tw, const CUtensorMap& tx, SplitArgs a, cudaStream_t stream) {
   using S = SplitShape<LARGE>;
   constexpr size_t LIMIT = LARGE ? SMEM_LIMIT : 112 * 1024;       // two CTAs of the small one share an SM
-  const size_t fixed = (size_t)S::X_STAGES * 3 * a.bn * CK * 2 + 1024 + 256 + FLAG_SETS * CUTTERS;
+  const size_t fixed = (size_t)S::X_STAGES * 3 * a.bn * CK * 2 + 1024 + 256;
   a.w_stages = (int)((LIMIT - fixed) / W_STAGE);
   if (a.w_stages > 6) a.w_stages = 6;
   const size_t smem = fixed + (size_t)a.w_stages * W_STAGE;
@@ -570,13 +527,12 @@ int linear_split(const float* x, const float* w, TO* out, int T, int N, int K, f
   const int n_tt = kf_ceil_div(T, large ? LARGE_T : SMALL_T);
   a.bn = large ? (kf_ceil_div(T, n_tt) + 31) & ~31 : SMALL_T;
   __nv_bfloat16* planes = (__nv_bfloat16*)scratch;
-  a.row_odd = (int*)(scratch + plane_floats(T, K));
-  a.partial = scratch + plane_floats(T, K) + ((a.parts * T + 3) & ~3);
+  a.partial = scratch + plane_floats(T, K);
   CUtensorMap tw, tx;
   if (!tensor_map_f32(w, N, K, BM, &tw)) return KF_ERR_SETUP;
   if (!large) return launch_split<false, TO>(tw, tw, a, stream);
   if (!tensor_map(planes, 3l * T, pitch, a.bn, &tx)) return KF_ERR_SETUP;
-  kf_launch(split_rows_kernel, dim3(T), dim3(256), 0, stream, x, planes, (int*)a.row_odd, T, K, pitch, a.parts);
+  kf_launch(split_rows_kernel, dim3(T), dim3(256), 0, stream, x, planes, T, K, pitch);
   KF_CHECK_LAUNCH();
   const int s = launch_split<true, TO>(tw, tx, a, stream);
   if (s != KF_OK || a.parts == 1) return s;
@@ -597,7 +553,7 @@ KF_API int kf_linear_split_supported(const void* x, const void* w, int N, int K)
 // Floats of scratch that a call needs, and the kernels that it launches.
 KF_API long kf_linear_split_scratch(int T, int N, int K) {
   const int parts = split_parts(N, K);
-  return T <= SMALL_T ? 0 : plane_floats(T, K) + (((long)parts * T + 3) & ~3l) + (parts > 1 ? (long)parts * T * N : 0);
+  return T <= SMALL_T ? 0 : plane_floats(T, K) + (parts > 1 ? (long)parts * T * N : 0);
 }
 KF_API int kf_linear_split_launches(int T, int N, int K) { return T <= SMALL_T ? 1 : split_parts(N, K) > 1 ? 3 : 2; }
 

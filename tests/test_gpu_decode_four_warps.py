@@ -1,5 +1,5 @@
-"""Decode attention whose blocks take equal runs of the step's keys: runs that end inside a pair, hold several whole pairs, or begin
-and end in two; rows of no request between the others; lengths around a tile of 16 keys; more rows than a warp counts at a time."""
+"""Decode attention in blocks of four warps planned for more keys than there are: rows taken by their rank in length (as many as fill one
+block on every SM, up to twice as many, more, and rows of equal length), three parts a pair, rows of no request between the others."""
 import pytest
 import torch
 
@@ -9,10 +9,13 @@ DEV = "cuda:0"
 RAGGED = [1100, 1, 15, 16, 17, 128, 129, 500, 33, 700]
 
 
-@pytest.mark.parametrize("nh,nkv,d,lens,most", [(8, 4, 256, RAGGED, 1100), (16, 1, 256, RAGGED, 4000), (16, 4, 128, RAGGED, 1100), (6, 2, 64, RAGGED * 7, 1100),
-                                                (8, 4, 256, [9000, 3], 9000), (4, 4, 16, [5] * 40, 2000), (8, 4, 256, [40 + 13 * i for i in range(64)], 900)])
+# heads of 256 (148 and 296 blocks on the GPU): 64 rows of 4 heads, 78 of them (more than two a block of every SM), 20 rows in three parts;
+# heads of 128 and 16; one head of keys (as many rows ranked as SMs), and few rows, which stay in blocks of eight warps
+@pytest.mark.parametrize("nh,nkv,d,lens,most", [(8, 4, 256, [40 + 13 * i for i in range(50)] + [77] * 4, 1900), (8, 4, 256, RAGGED * 7, 1100), (8, 4, 256, RAGGED + [900] * 8, 3000),
+                                                (16, 4, 128, [5 + (i * 97) % 600 for i in range(90)], 900), (4, 4, 16, [5, 300] * 130, 2000),
+                                                (4, 1, 256, [(i * 31) % 250 + 1 for i in range(200)], 700), (16, 4, 128, RAGGED, 1100)])
 @pytest.mark.parametrize("window,keep,sink,sig", [(None, 0, False, False), (200, 21, True, False), (None, 0, False, True)])
-def test_runs_of_ragged_rows(nh, nkv, d, lens, most, window, keep, sink, sig):
+def test_rows_of_unequal_length(nh, nkv, d, lens, most, window, keep, sink, sig):
     from kungfu_b200 import ops
     from test_gpu_kernels import _Ctx, _View, _paged_setup
     pages, table, ks, vs = _paged_setup(torch.bfloat16, nh, nkv, d, 64, lens, seed=len(lens))
