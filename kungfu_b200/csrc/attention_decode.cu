@@ -450,7 +450,7 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
   // `ranked` rows fill one block on every SM.  Those blocks take the longest rows, the longest first, and the ones that join
   // them on their SMs the others, the shortest first: an SM then streams about as much as any other.
   if (DM_WARPS == DM_WARPS_SHORT && ranked) {
-    __shared__ int s_len[DM_RANKED], s_item;
+    int* s_len = reinterpret_cast<int*>(dm_smem);                  // the ring is not in use yet; more shared memory would cost a block
     for (int i = tid; i < n_items; i += DM_WARPS * 32) {
       const int row = items ? items[i] : i, p = positions[row];
       s_len[i] = row_req[row] < 0 ? 0 : p + 1 - kf_first_key(p, window);
@@ -461,10 +461,10 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
       const int own = s_len[i];
       int before = 0;
       for (int j = 0; j < n_items; ++j) before += s_len[j] > own || (s_len[j] == own && j < i);
-      if (before == rank) s_item = i;
+      if (before == rank) s_last = i;
     }
     __syncthreads();
-    item = s_item;
+    item = s_last;
   }
   const int split = blockIdx.y;
   const int G = nh / nkv;
