@@ -3,16 +3,15 @@
 // A 32-bit number is the exact sum of three bfloat16 ones (its significand cut after 8, 16 and 24 bits; bfloat16 has the same
 // exponents), and a product of two bfloat16 numbers is exact in 32 bits.  With x = x1 + x2 + x3 and w = w1 + w2 + w3 the six
 // products x1 w1, x1 w2, x2 w1, x2 w2, x1 w3, x3 w1 hold all but 2^-21 of x w (the other three are left out).  What a
-// tensor core adds up it may cut off instead of rounding, so an accumulator lives for 64 k only, of every 32 k the small
-// products first; the sums of those chunks are added in registers, rounded to nearest.
+// tensor core adds up it may cut off instead of rounding, so an accumulator lives for 64 k only, small products first; the
+// sums of those chunks are added in registers, rounded to nearest.
 //
 // Shape of the kernel (gemm_split_kernel): weights are the MMA's A operand (128 features = 128 lanes), rows of x its N.
 //   warp 0      TMA: weights as they are, 128 x 64 floats a stage, and the three planes of x (cut by `split_rows_kernel`; up to
 //               16 rows the summing warps cut x themselves, into shared memory, two chunks ahead)
 //   warps 2-9   read the weights of a stage, cut them in registers and put the three planes into tensor memory (the MMA
 //               takes A from there), so that the weights cross the memory system once, in 32 bits, and no copy is kept
-//   warp 1      24 MMAs a chunk (six products of four steps of 16 k) into one of two accumulators; four warps cut the first half of
-//               every chunk and four the second, each into two buffers of their own, so that the MMAs rarely wait for them
+//   warp 1      24 MMAs a chunk (six products of four steps of 16 k) into one of two accumulators
 //   warps 10-.. add a finished accumulator to their sums in registers while the next is being filled
 // K is cut into parts (`split_parts`, from N and K alone) so that the feature tiles fill the SMs.  Up to 16 rows the parts of
 // a tile are a cluster of CTAs, two of them to an SM, and meet in shared memory; beyond, a CTA walks (tile, part) units
@@ -30,7 +29,7 @@ using namespace kf_tc;
 
 constexpr int CK = 64;                                          // k of a chunk: the life of an accumulator
 constexpr int W_STAGE = BM * CK * 4;                            // 32 KB: two boxes of 128 rows x 32 floats
-constexpr int A_COLS = 3 * CK / 4;                              // tensor-memory columns of half a chunk's three weight planes
+constexpr int A_COLS = 3 * CK / 2;                              // tensor-memory columns of a chunk's three weight planes
 constexpr int CUTTERS = 256;                                    // threads that cut weights: two per feature
 constexpr int SMALL_T = 16, LARGE_T = 160;                      // rows of a tile, at most
 
@@ -120,7 +119,7 @@ struct SplitShape {
   static constexpr int TMEM = LARGE ? 512 : 256;
   static constexpr int X_STAGES = 2;
 };
-static_assert(4 * A_COLS + 2 * LARGE_T <= 512 && 4 * A_COLS + 2 * SMALL_T <= 256, "weight planes and accumulators fit tensor memory");
+static_assert(2 * A_COLS + 2 * LARGE_T <= 512 && 2 * A_COLS + 2 * SMALL_T <= 256, "weight planes and accumulators fit tensor memory");
 
 template <bool LARGE, typename TO>
 __global__ void __launch_bounds__(SplitShape<LARGE>::THREADS_, LARGE ? 1 : 2)
@@ -135,9 +134,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   uint64_t* w_empty = w_full + ws;
   uint64_t* x_full = w_empty + ws;
   uint64_t* x_empty = x_full + S::X_STAGES;
-  uint64_t* a_full = x_empty + S::X_STAGES;                       // [4] weight planes of a half chunk are in tensor memory
-  uint64_t* a_free = a_full + 4;                                  // [4] its MMAs have ended
-  uint64_t* done = a_free + 4;                                    // [2] all MMAs of a chunk have ended
+  uint64_t* a_full = x_empty + S::X_STAGES;                       // [2] weight planes of a chunk are in tensor memory
+  uint64_t* done = a_full + 2;                                    // [2] its MMAs have ended
   uint64_t* acc_free = done + 2;                                  // [2] its accumulator has been read
   uint32_t* tmem_slot = (uint32_t*)(acc_free + 2);
   volatile int* s_abort = (volatile int*)(tmem_slot + 1);
@@ -150,8 +148,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   if (threadIdx.x == 0) {
     for (int s = 0; s < ws; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], CUTTERS); }
     for (int s = 0; s < S::X_STAGES; ++s) { mbar_init(&x_full[s], LARGE ? 1 : 128); mbar_init(&x_empty[s], 1); }
-    for (int b = 0; b < 4; ++b) { mbar_init(&a_full[b], CUTTERS / 2); mbar_init(&a_free[b], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&done[b], 1); mbar_init(&acc_free[b], 128 * S::SUM_GROUPS); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&a_full[b], CUTTERS); mbar_init(&done[b], 1); mbar_init(&acc_free[b], 128 * S::SUM_GROUPS); }
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -236,26 +233,19 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         range(unit, first, last);
         for (int i = first; i < last; ++i, ++c) {
           const int b = c & 1;
-          const uint32_t ph = (uint32_t)(c >> 1) & 1;
-          if (!mbar_wait(&x_full[x_slot], x_ph) || (c >= 2 && !mbar_wait(&acc_free[b], ph ^ 1))) { give_up(ERR_WAIT_FULL); ok = false; break; }
-          const uint32_t acc = tmem + 4 * A_COLS + b * S::MAX_T;
+          if (!mbar_wait(&a_full[b], (uint32_t)(c >> 1) & 1) || !mbar_wait(&x_full[x_slot], x_ph) ||
+              (c >= 2 && !mbar_wait(&acc_free[b], (uint32_t)((c >> 1) - 1) & 1))) { give_up(ERR_WAIT_FULL); ok = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t wa = tmem + b * A_COLS, acc = tmem + 2 * A_COLS + b * S::MAX_T;
           const uint64_t dx = dx0 + (uint64_t)((uint32_t)(x_slot * x_stage) >> 4);
           const uint32_t plane = (uint32_t)(bn * CK * 2) >> 4;
           // small products first: (w plane, x plane)
           constexpr int order[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (!mbar_wait(&a_full[2 * b + h], ph)) { give_up(ERR_WAIT_FULL); ok = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t wa = tmem + (2 * b + h) * A_COLS;
+          for (int q = 0; q < 6; ++q)
 #pragma unroll
-            for (int q = 0; q < 6; ++q)
-#pragma unroll
-              for (int k = 0; k < CK / 2 / UMMA_K; ++k)
-                umma_ts(acc, wa + order[q][0] * (CK / 4) + k * (UMMA_K / 2), dx + order[q][1] * plane + 4 * h + 2 * k, idesc, (h > 0 || q > 0 || k > 0) ? 1u : 0u);
-            umma_commit(&a_free[2 * b + h]);
-          }
-          if (!ok) break;
+            for (int k = 0; k < CK / UMMA_K; ++k)
+              umma_ts(acc, wa + order[q][0] * (CK / 2) + k * (UMMA_K / 2), dx + order[q][1] * plane + 2 * k, idesc, (q > 0 || k > 0) ? 1u : 0u);
           umma_commit(&x_empty[x_slot]);
           umma_commit(&done[b]);
           if (++x_slot == S::X_STAGES) { x_slot = 0; x_ph ^= 1; }
@@ -275,11 +265,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       range(unit, first, last);
       for (int i = first; i < last; ++i, ++c) {
         const int b = c & 1;
-        ok = mbar_wait(&w_full[slot], ph) && (c < 2 || mbar_wait(&a_free[2 * b + half], (uint32_t)((c >> 1) - 1) & 1)) && !*s_abort;
+        ok = mbar_wait(&w_full[slot], ph) && (c < 2 || mbar_wait(&done[b], (uint32_t)((c >> 1) - 1) & 1)) && !*s_abort;
         if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) give_up(ERR_WAIT_FULL); ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint8_t* row = sw + (size_t)slot * W_STAGE + half * (W_STAGE / 2) + r * 128;
-        const uint32_t dst = lane_addr + (2 * b + half) * A_COLS;
+        const uint32_t dst = lane_addr + b * A_COLS + half * 16;
         uint32_t p1[16], p2[16], p3[16];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {                             // 16-byte piece j of a row stands at j ^ (row % 8)
@@ -288,12 +278,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
           cut_pair(v.z, v.w, p1[2 * j + 1], p2[2 * j + 1], p3[2 * j + 1]);
         }
         tmem_st16(dst, p1);
-        tmem_st16(dst + CK / 4, p2);
-        tmem_st16(dst + CK / 2, p3);
+        tmem_st16(dst + CK / 2, p2);
+        tmem_st16(dst + CK, p3);
         mbar_arrive(&w_empty[slot]);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        mbar_arrive(&a_full[2 * b + half]);
+        mbar_arrive(&a_full[b]);
         if (++slot == ws) { slot = 0; ph ^= 1; }
       }
     }
@@ -359,7 +349,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) give_up(ERR_WAIT_ACC); ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (!LARGE) cut_x(b);
-        const uint32_t acc = lane_addr + 4 * A_COLS + b * S::MAX_T + col0;
+        const uint32_t acc = lane_addr + 2 * A_COLS + b * S::MAX_T + col0;
 #pragma unroll
         for (int j0 = 0; j0 < S::COLS; j0 += S::BATCH) {
           uint32_t v[S::BATCH];
@@ -486,7 +476,7 @@ template <bool LARGE, typename TO>
 int launch_split(const CUtensorMap& tw, const CUtensorMap& tx, SplitArgs a, cudaStream_t stream) {
   using S = SplitShape<LARGE>;
   constexpr size_t LIMIT = LARGE ? SMEM_LIMIT : 112 * 1024;       // two CTAs of the small one share an SM
-  const size_t fixed = (size_t)S::X_STAGES * 3 * a.bn * CK * 2 + 1024 + 320;
+  const size_t fixed = (size_t)S::X_STAGES * 3 * a.bn * CK * 2 + 1024 + 256;
   a.w_stages = (int)((LIMIT - fixed) / W_STAGE);
   if (a.w_stages > 6) a.w_stages = 6;
   const size_t smem = fixed + (size_t)a.w_stages * W_STAGE;

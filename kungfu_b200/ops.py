@@ -409,9 +409,10 @@ def _linear_split(x, weight, out, N: int, softcap: float) -> bool:
 @_dispatch("linear")
 def linear(x, weight, out, softcap: float = 0.0) -> None:
     """out[T, N] = x[T, K] . weight[N, K]^T, 32-bit accumulation; softcap > 0 applies cap*tanh(v/cap).
-    bfloat16 operands run on the tensor cores (tcgen05) when rows are multiples of 16 bytes; everything else runs 32-bit FMA
-    kernels: the whole 32-bit path the one in packed tiles, mixed types a generic one, a few 32-bit rows of a short K on
-    bfloat16 weights one of their own."""
+    bfloat16 operands run on the tensor cores (tcgen05) when rows are multiples of 16 bytes, and so do 32-bit ones with 4 Mi
+    weights or more, each number cut into three bfloat16 ones; everything else runs 32-bit FMA kernels: the rest of the
+    32-bit path the one in packed tiles, mixed types a generic one, a few 32-bit rows of a short K on bfloat16 weights one
+    of their own."""
     T, K = x.shape
     N = weight.shape[0]
     if weight.shape[1] != K or tuple(out.shape) != (T, N):
