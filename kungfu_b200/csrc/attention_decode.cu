@@ -403,10 +403,8 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 // one of the prompt kernel.  Warps are merged through shared memory in warp order, splits by the last block.
 constexpr int DM_WARPS = 8;                       // two per scheduler: a warp's tile is one chain of dependent instructions
 // Blocks of four warps, two to an SM at heads of 256: while one starts or merges its warps, the other one's keys keep coming in.
-// They need enough pairs (row, kv head) for all of those blocks, and then are the better ones at any length.  Heads of 256, 8 over 4,
-// planned for 2,000 to 4,000 tokens more than there are, in us a launch, blocks of eight warps -> of four:
-//   64 rows of 64 keys 13.6 -> 7.5, of 256 19.5 -> 14.1, of 1,024 50.3 -> 42.6, of 2,048 88.2 -> 80.1 (floor 82 at 6,544 GB/s)
-//   20 rows of 1,500 keys, in three parts each, 32.3 -> 25.1;   40 rows of 160 to 1,600 (160 blocks) 39.0 -> 58.7
+// They need enough pairs (row, kv head) for all of those blocks, and then are the better ones at any length.  A block of four
+// takes in 24 GB/s whatever its neighbour does, so a row well above the average is cut in two.
 constexpr int DM_WARPS_SHORT = 4;
 constexpr int DM_KEYS_SHORT = 512;
 constexpr int DM_RANKED = 256;                    // rows that a block ranks by their length, at most
@@ -441,32 +439,39 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
   __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(dm_smem);  // [16][D]
   __nv_bfloat16* sKV = sQ + 16 * D;                               // [warp][buffer][16][D]
   __shared__ float sm_ml[DM_WARPS][16][2];
-  __shared__ int s_last;
+  __shared__ int s_last, sm_cut;
 
   // ---- the step's integers: written before the step's first kernel, so readable at once -------------------------------
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  int item = blockIdx.x / nkv;
-  const int kvh = blockIdx.x - item * nkv;
-  // `ranked` rows fill one block on every SM.  Those blocks take the longest rows, the longest first, and the ones that join
-  // them on their SMs the others, the shortest first: an SM then streams about as much as any other.
-  if (DM_WARPS == DM_WARPS_SHORT && ranked) {
+  // `ranked`: the rows in the order of their lengths, the longest first, and two blocks a pair, of which the second one leaves
+  // unless the row is a quarter longer than the average
+  const bool by_rank = DM_WARPS == DM_WARPS_SHORT && ranked;
+  const int split = by_rank ? blockIdx.x & 1 : blockIdx.y;
+  const int place = by_rank ? blockIdx.x >> 1 : blockIdx.x;
+  int item = place / nkv, cut = 0;
+  const int kvh = place - item * nkv;
+  if (by_rank) {
     int* s_len = reinterpret_cast<int*>(dm_smem);                  // the ring is not in use yet; more shared memory would cost a block
     for (int i = tid; i < n_items; i += DM_WARPS * 32) {
       const int row = items ? items[i] : i, p = positions[row];
       s_len[i] = row_req[row] < 0 ? 0 : p + 1 - kf_first_key(p, window);
     }
     __syncthreads();
-    const int rank = item < ranked ? item : n_items <= 2 * ranked ? n_items - 1 - (item - ranked) : item;
     for (int i = tid; i < n_items; i += DM_WARPS * 32) {
       const int own = s_len[i];
-      int before = 0;
-      for (int j = 0; j < n_items; ++j) before += s_len[j] > own || (s_len[j] == own && j < i);
-      if (before == rank) s_last = i;
+      int before = 0, sum = 0, n = 0;
+      for (int j = 0; j < n_items; ++j) {
+        const int len = s_len[j];
+        before += len > own || (len == own && j < i);
+        sum += len;
+        n += len > 0;
+      }
+      if (before == item) s_last = i, sm_cut = n ? (int)((long)sum * 5 / (4 * n)) : 0;
     }
     __syncthreads();
     item = s_last;
+    cut = sm_cut;
   }
-  const int split = blockIdx.y;
   const int G = nh / nkv;
   const int h_first = kvh * G;
   const KfHeadMap hm = kf_head_map(h_first, kvh, nh, nkv, vsplit);   // with the rotation inside (qkv given) vsplit is 0
@@ -487,7 +492,10 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
   const int kept = window > 0 ? min(keep_first, lo) : 0;
   const int lo_v = lo - kept;
   const int n_keys = pos + 1 - lo_v;
-  int per = (n_keys + n_splits - 1) / n_splits;
+  // parts of this row: what the launch is planned for; blocks of four warps are planned for longer rows than there may be
+  const int parts = DM_WARPS != DM_WARPS_SHORT ? n_splits : by_rank ? (n_keys > cut ? 2 : 1) : min(n_splits, (n_keys + 127) / 128);
+  if (split >= parts) return;
+  int per = (n_keys + parts - 1) / parts;
   per = (per + 63) & ~63;
   const int k_begin = lo_v + split * per;
   const int k_end = min(pos + 1, k_begin + per);
@@ -759,7 +767,7 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
     }
   }
   __syncthreads();
-  const size_t rec_base = (((size_t)t * nh + h_first) * n_splits + split) * PSTRIDE;
+  const size_t rec_base = (((size_t)t * nh + h_first) * parts + split) * PSTRIDE;
   for (int e = tid; e < G * D; e += blockDim.x) {
     const int h = e / D, i = e - h * D;
     // the sink (a key of score 0 without a value) joins the first split like one more warp: maximum 0, sum 1, no row
@@ -773,26 +781,26 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
       l += sm_ml[w][h][1] * c;
       a += sm_o[((size_t)w * G + h) * D + i] * c;
     }
-    if (n_splits == 1) {
+    if (parts == 1) {
       orow[(size_t)(h_first + h) * D + i] = __float2bfloat16_rn(l > 0.f ? a / l : 0.f);
     } else {
-      float* rec = partial + rec_base + (size_t)h * n_splits * PSTRIDE;
+      float* rec = partial + rec_base + (size_t)h * parts * PSTRIDE;
       rec[i] = a;
       if (i == 0) { rec[D] = m; rec[D + 1] = l; }
     }
   }
-  if (n_splits == 1) return;
+  if (parts == 1) return;
   __threadfence();
   __syncthreads();
   const int cidx = item * nkv + kvh;
-  if (tid == 0) s_last = (atomicAdd(&counters[cidx], 1) == n_splits - 1);
+  if (tid == 0) s_last = (atomicAdd(&counters[cidx], 1) == parts - 1);
   __syncthreads();
   if (!s_last) return;
   __threadfence();                                               // maxima here are base-2 scaled
-  if (n_splits > 8 && (size_t)G * n_splits * PSTRIDE * sizeof(float) <= (size_t)DM_WARPS * DM_BUFS * TILE * sizeof(__nv_bfloat16))
-    merge_splits_shared<D>(partial, ((size_t)t * nh + h_first) * n_splits, G, n_splits, orow + (size_t)h_first * D, sm_o);
+  if (parts > 8 && (size_t)G * parts * PSTRIDE * sizeof(float) <= (size_t)DM_WARPS * DM_BUFS * TILE * sizeof(__nv_bfloat16))
+    merge_splits_shared<D>(partial, ((size_t)t * nh + h_first) * parts, G, parts, orow + (size_t)h_first * D, sm_o);
   else
-    merge_splits<D, true>(partial, ((size_t)t * nh + h_first) * n_splits, G, n_splits, orow + (size_t)h_first * D);
+    merge_splits<D, true>(partial, ((size_t)t * nh + h_first) * parts, G, parts, orow + (size_t)h_first * D);
   if (tid == 0) counters[cidx] = 0;
 }
 
@@ -821,16 +829,17 @@ int launch_decode_mma_warps(const float* qkv, const float* cos_t, const float* s
                       float* partial, int* counters, void* out, cudaStream_t stream) {
   const size_t smem = (size_t)(16 * D + DM_WARPS * DM_BUFS * DM_KEYS * D) * 2;
   if (decode_mma_blocks_per_sm<D, SIG, DM_WARPS>() < 1) return KF_ERR_SETUP;
-  const int ranked = DM_WARPS == DM_WARPS_SHORT && n_splits == 1 && n_items <= DM_RANKED ? kf_sm_count() / nkv : 0;
-  kf_launch(attn_decode_mma_kernel<D, SIG, DM_WARPS>, dim3(n_items * nkv, n_splits), dim3(DM_WARPS * 32), smem, stream,
+  const bool ranked = DM_WARPS == DM_WARPS_SHORT && n_splits == 2 && n_items <= DM_RANKED;
+  const dim3 grid = ranked ? dim3(2 * n_items * nkv) : dim3(n_items * nkv, n_splits);
+  kf_launch(attn_decode_mma_kernel<D, SIG, DM_WARPS>, grid, dim3(DM_WARPS * 32), smem, stream,
             (const __nv_bfloat16*)q, qkv, cos_t, sin_t, rot, write_kv, (__nv_bfloat16*)const_cast<void*>(pages), items, n_items,
             positions, row_req, table, table_stride, page_size, nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias, n_splits,
-            ranked, partial, counters, (__nv_bfloat16*)out);
+            ranked ? 1 : 0, partial, counters, (__nv_bfloat16*)out);
   KF_CHECK_LAUNCH();
   return KF_OK;
 }
 
-// n_splits 0: one split in blocks of DM_WARPS_SHORT warps; below 0: -n_splits of them.
+// n_splits 0: one split in blocks of DM_WARPS_SHORT warps; below 0: up to -n_splits of them (-2: by the rows' ranks).
 template <int D, bool SIG>
 int launch_decode_mma(const float* qkv, const float* cos_t, const float* sin_t, int rot, int write_kv,
                       const void* q, const void* pages, const int* items, int n_items, const int* positions,
@@ -889,7 +898,7 @@ static long decode_mma_resident(int d) {
   return kf_sm_count() * (per_sm < 1 ? 1 : per_sm);
 }
 
-// splits_out: how many parts a row's keys are cut into; 0 or below for blocks of fewer warps, 0 for one part and -k for k parts.
+// splits_out: how many parts a row's keys are cut into; 0 or below for blocks of fewer warps, 0 for one part and -k for up to k.
 // kf_attention_decode (ht = 0) and kf_attention_decode_fused take it as it is.
 KF_API int kf_attention_decode_mma_plan(int n_items, int nh, int nkv, int d, int max_keys, int* splits_out) {
   if (g_forced_splits > 0) { *splits_out = g_forced_splits; return KF_OK; }
@@ -902,7 +911,8 @@ KF_API int kf_attention_decode_mma_plan(int n_items, int nh, int nkv, int d, int
   if (splits < 1) splits = 1;
   // Blocks of four warps where they can be as many as the GPU holds, but for a fifth: one a pair, or, where a block of eight
   // warps a pair would leave up to half of the SMs without, three.  In between (99 to 230 pairs at heads of 256) they are too few.
-  if ((blocks > resident && max_keys <= DM_KEYS_SHORT) || blocks * 5 >= of_four * 4) splits = 0;
+  if (blocks * 5 >= of_four * 4) splits = n_items <= DM_RANKED && max_keys > 128 ? -2 : 0;
+  else if (blocks > resident && max_keys <= DM_KEYS_SHORT) splits = 0;
   else if (splits == 1 && blocks < resident && blocks * 3 <= of_four && max_keys > 2 * DM_KEYS_SHORT) splits = -3;
   *splits_out = splits;
   return KF_OK;
