@@ -3,16 +3,18 @@
 // A 32-bit number is the exact sum of three bfloat16 ones (its significand cut after 8, 16 and 24 bits; bfloat16 has the same
 // exponents), and a product of two bfloat16 numbers is exact in 32 bits.  With x = x1 + x2 + x3 and w = w1 + w2 + w3 the six
 // products x1 w1, x1 w2, x2 w1, x2 w2, x1 w3, x3 w1 hold all but 2^-21 of x w (the other three are left out).  What a
-// tensor core adds up it may cut off instead of rounding, so an accumulator lives for 64 k only, small products first; the
-// sums of those chunks are added in registers, rounded to nearest.
+// tensor core adds up it may cut off instead of rounding, so an accumulator lives for 64 k only, and products of one size share
+// one (x1 w1; x1 w2 + x2 w1; the other three); the sums are added in registers, rounded to nearest.
 //
 // Shape of the kernel (gemm_split_kernel): weights are the MMA's A operand (128 features = 128 lanes), rows of x its N.
 //   warp 0      TMA: weights as they are, 128 x 64 floats a stage, and the three planes of x (cut by `split_rows_kernel`; up to
 //               16 rows the summing warps cut x themselves, into shared memory, two chunks ahead)
 //   warps 2-9   read the weights of a stage, cut them in registers and put the three planes into tensor memory (the MMA
 //               takes A from there), so that the weights cross the memory system once, in 32 bits, and no copy is kept
-//   warp 1      24 MMAs a chunk (six products of four steps of 16 k) into one of two accumulators
-//   warps 10-.. add a finished accumulator to their sums in registers while the next is being filled
+//   warp 1      12 MMAs a chunk: the planes of x lie behind one another in shared memory as the accumulators do in tensor memory,
+//               so that w1 meets all three planes of x in one MMA, w2 the first two and w3 the first.  An MMA with A in tensor
+//               memory takes about 110 cycles however few rows it has, so their number is what counts
+//   warps 10-.. add the finished accumulators to their sums in registers
 // K is cut into parts (`split_parts`, from N and K alone) so that the feature tiles fill the SMs.  Up to 16 rows the parts of
 // a tile are a cluster of CTAs, two of them to an SM, and meet in shared memory; beyond, a CTA walks (tile, part) units
 // and leaves the parts' sums in memory for `sum_parts_kernel`.  Either way an output's sum is the chunks of a part in
@@ -31,7 +33,7 @@ constexpr int CK = 64;                                          // k of a chunk:
 constexpr int W_STAGE = BM * CK * 4;                            // 32 KB: two boxes of 128 rows x 32 floats
 constexpr int A_COLS = 3 * CK / 2;                              // tensor-memory columns of a chunk's three weight planes
 constexpr int CUTTERS = 256;                                    // threads that cut weights: two per feature
-constexpr int SMALL_T = 16, LARGE_T = 160;                      // rows of a tile, at most
+constexpr int SMALL_T = 16, LARGE_T = 80;                      // rows of a tile, at most
 
 __device__ __forceinline__ bool plain_needed(float v) { return !(fabsf(v) >= 8.67361738e-19f && fabsf(v) <= 3.4e38f) && v != 0.f; }   // 2^-60
 
@@ -105,21 +107,21 @@ struct SplitArgs {
   float* partial;                                                // [parts][T][N], where a launch leaves the parts' sums
   int* error_flag;
   float softcap;
-  int T, N, K, parts, bn, w_stages;                              // bn: rows of a tile, 16 or a multiple of 32
+  int T, N, K, parts, bn, w_stages;                              // bn: rows of a tile, a multiple of 16
 };
 
-// LARGE: a CTA per SM, up to 160 rows, the sums in sixteen warps.  Otherwise two CTAs per SM, 16 rows, the sums in four.
+// LARGE: a CTA per SM, up to 80 rows (the MMA takes 240), the sums in eight warps.  Otherwise two CTAs per SM, 16 rows, the sums in four.
 template <bool LARGE>
 struct SplitShape {
   static constexpr int MAX_T = LARGE ? LARGE_T : SMALL_T;
-  static constexpr int SUM_GROUPS = LARGE ? 4 : 1;
+  static constexpr int SUM_GROUPS = LARGE ? 2 : 1;
   static constexpr int COLS = MAX_T / SUM_GROUPS;                // accumulator columns of a thread, at most
-  static constexpr int BATCH = LARGE ? COLS / 5 : 16;             // columns per wait on tensor memory
+  static constexpr int BATCH = 8;                                // columns of every accumulator per wait on tensor memory
   static constexpr int THREADS_ = 64 + CUTTERS + 128 * SUM_GROUPS;
   static constexpr int TMEM = LARGE ? 512 : 256;
   static constexpr int X_STAGES = 2;
 };
-static_assert(2 * A_COLS + 2 * LARGE_T <= 512 && 2 * A_COLS + 2 * SMALL_T <= 256, "weight planes and accumulators fit tensor memory");
+static_assert(2 * A_COLS + 3 * LARGE_T <= 512 && 3 * LARGE_T <= 256 && 2 * A_COLS + 3 * SMALL_T <= 256, "weight planes and accumulators fit tensor memory");
 
 template <bool LARGE, typename TO>
 __global__ void __launch_bounds__(SplitShape<LARGE>::THREADS_, LARGE ? 1 : 2)
@@ -136,8 +138,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   uint64_t* x_empty = x_full + S::X_STAGES;
   uint64_t* a_full = x_empty + S::X_STAGES;                       // [2] weight planes of a chunk are in tensor memory
   uint64_t* done = a_full + 2;                                    // [2] its MMAs have ended
-  uint64_t* acc_free = done + 2;                                  // [2] its accumulator has been read
-  uint32_t* tmem_slot = (uint32_t*)(acc_free + 2);
+  uint64_t* acc_free = done + 2;                                  // its accumulators have been read
+  uint32_t* tmem_slot = (uint32_t*)(acc_free + 1);
   volatile int* s_abort = (volatile int*)(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -148,7 +150,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   if (threadIdx.x == 0) {
     for (int s = 0; s < ws; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], CUTTERS); }
     for (int s = 0; s < S::X_STAGES; ++s) { mbar_init(&x_full[s], LARGE ? 1 : 128); mbar_init(&x_empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&a_full[b], CUTTERS); mbar_init(&done[b], 1); mbar_init(&acc_free[b], 128 * S::SUM_GROUPS); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&a_full[b], CUTTERS); mbar_init(&done[b], 1); }
+    mbar_init(acc_free, 128 * S::SUM_GROUPS);
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -223,7 +226,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   } else if (warp == 1) {
     // ---- MMA issuer -------------------------------------------------------------------------------------------------------
     if (lane == 0) {
-      const uint32_t idesc = umma_idesc(bn);
+      const uint32_t idesc[3] = {umma_idesc(3 * bn), umma_idesc(2 * bn), umma_idesc(bn)};
       const uint64_t dx0 = umma_desc(sx);
       int c = 0, x_slot = 0;
       uint32_t x_ph = 0;
@@ -234,18 +237,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         for (int i = first; i < last; ++i, ++c) {
           const int b = c & 1;
           if (!mbar_wait(&a_full[b], (uint32_t)(c >> 1) & 1) || !mbar_wait(&x_full[x_slot], x_ph) ||
-              (c >= 2 && !mbar_wait(&acc_free[b], (uint32_t)((c >> 1) - 1) & 1))) { give_up(ERR_WAIT_FULL); ok = false; break; }
+              (c >= 1 && !mbar_wait(acc_free, (uint32_t)(c - 1) & 1))) { give_up(ERR_WAIT_FULL); ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t wa = tmem + b * A_COLS, acc = tmem + 2 * A_COLS + b * S::MAX_T;
+          const uint32_t wa = tmem + b * A_COLS, acc = tmem + 2 * A_COLS;
           const uint64_t dx = dx0 + (uint64_t)((uint32_t)(x_slot * x_stage) >> 4);
-          const uint32_t plane = (uint32_t)(bn * CK * 2) >> 4;
-          // small products first: (w plane, x plane)
-          constexpr int order[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
 #pragma unroll
-          for (int q = 0; q < 6; ++q)
+          for (int k = 0; k < CK / UMMA_K; ++k)
 #pragma unroll
-            for (int k = 0; k < CK / UMMA_K; ++k)
-              umma_ts(acc, wa + order[q][0] * (CK / 2) + k * (UMMA_K / 2), dx + order[q][1] * plane + 2 * k, idesc, (q > 0 || k > 0) ? 1u : 0u);
+            for (int q = 0; q < 3; ++q)                           // plane q of the weights, into the accumulators from number q on
+              umma_ts(acc + q * bn, wa + q * (CK / 2) + k * (UMMA_K / 2), dx + 2 * k, idesc[q], (q > 0 || k > 0) ? 1u : 0u);
           umma_commit(&x_empty[x_slot]);
           umma_commit(&done[b]);
           if (++x_slot == S::X_STAGES) { x_slot = 0; x_ph ^= 1; }
@@ -349,23 +349,22 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) give_up(ERR_WAIT_ACC); ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (!LARGE) cut_x(b);
-        const uint32_t acc = lane_addr + 2 * A_COLS + b * S::MAX_T + col0;
+        const uint32_t acc = lane_addr + 2 * A_COLS + col0;
 #pragma unroll
         for (int j0 = 0; j0 < S::COLS; j0 += S::BATCH) {
-          uint32_t v[S::BATCH];
+          if (j0 >= cols) break;
+          uint32_t v[3][S::BATCH];
 #pragma unroll
-          for (int j = 0; j < S::BATCH; j += 8)
-            if (j0 + j < cols) tmem_ld8_async(acc + j0 + j, v + j);
+          for (int q = 0; q < 3; ++q) tmem_ld8_async(acc + q * bn + j0, v[q]);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int j = 0; j < S::BATCH; ++j)
-            if (j0 + (j & ~7) < cols) {
-              asm volatile("" : "+r"(v[j]));                      // not before the wait
-              sum[j0 + j] += __uint_as_float(v[j]);
-            }
+          for (int j = 0; j < S::BATCH; ++j) {
+            asm volatile("" : "+r"(v[0][j]), "+r"(v[1][j]), "+r"(v[2][j]));      // not before the wait
+            sum[j0 + j] += __uint_as_float(v[0][j]) + (__uint_as_float(v[1][j]) + __uint_as_float(v[2][j]));
+          }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        mbar_arrive(&acc_free[b]);
+        mbar_arrive(acc_free);
       }
       if (!ok) break;
       // ---- the unit's outputs: the parts of a product in a cluster through shared memory, else to memory -----------------------
@@ -525,7 +524,7 @@ int linear_split(const float* x, const float* w, TO* out, int T, int N, int K, f
   a.parts = split_parts(N, K);
   const bool large = T > SMALL_T;
   const int n_tt = kf_ceil_div(T, large ? LARGE_T : SMALL_T);
-  a.bn = large ? (kf_ceil_div(T, n_tt) + 31) & ~31 : SMALL_T;
+  a.bn = (kf_ceil_div(T, n_tt) + 15) & ~15;
   __nv_bfloat16* planes = (__nv_bfloat16*)scratch;
   a.partial = scratch + plane_floats(T, K);
   CUtensorMap tw, tx;

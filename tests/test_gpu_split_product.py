@@ -20,7 +20,7 @@ def _case(N, K, T, seed=1):
 
 
 # one, two, four and eight parts of K; features around a tile of 128; a k tail of 4, 8 and 60 and a chunk that ends in its first half;
-# rows at the edges of the small tile (16), of the tiles beyond (multiples of 16 up to 160) and of two and three of them
+# rows at the edges of the small tile (16), of the tiles beyond (multiples of 16 up to 80) and of two to five of them
 @pytest.mark.parametrize("N,K", [(18433, 228), (8000, 600), (16500, 260), (4095, 1084), (2304, 2052), (1100, 4128), (70000, 64)])
 def test_rows_against_64_bits_and_alone(ops, N, K):
     assert ops.library().kf_linear_split_supported(0, 0, N, K)
@@ -34,7 +34,7 @@ def test_rows_against_64_bits_and_alone(ops, N, K):
     assert bool(((whole - ref).abs() <= bound).all())
     # and on the whole no worse than a chain of rounded 32-bit sums of K / 2 terms, whose error grows as sqrt(K / 2) 2^-25
     assert float((whole - ref).norm() / ref.norm()) <= (K / 2) ** 0.5 * 2.0 ** -25 + 2.0 ** -23
-    for T in (1, 15, 16, 17, 32, 33, 159, 160, 161, 321):
+    for T in (1, 15, 16, 17, 32, 33, 79, 80, 81, 160, 161, 321):
         out = torch.full((T + 1, N), float("nan"), device=DEV)
         ops.linear(x[:T], w, out[:T])
         assert torch.equal(out[:T], whole[:T]), T                # a row does not depend on the others, to the bit
