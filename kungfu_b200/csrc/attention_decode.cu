@@ -404,10 +404,15 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 constexpr int DM_WARPS = 8;                       // two per scheduler: a warp's tile is one chain of dependent instructions
 // Blocks of four warps, two to an SM at heads of 256: while one starts or merges its warps, the other one's keys keep coming in.
 // They need enough pairs (row, kv head) for all of those blocks, and then are the better ones at any length.  A block of four
-// takes in 24 GB/s whatever its neighbour does, so a row well above the average is cut in two.
+// takes in 24 GB/s whatever its neighbour does, so a row well above the average is cut in two.  Heads of 256, 8 over 4, planned
+// for 2,000 tokens more than there are, us a launch, blocks of eight warps -> of four:
+//   64 rows of 64 keys 13.6 -> 10.9, of 256 19.5 -> 16.7, of 1,024 50.3 -> 45.2, of 2,048 88.2 -> 82.5 (floor 82.0 at 6,544 GB/s),
+//   of 100 to 1,024 41.1 -> 36.1; 78 rows of 90 to 900 42.4 -> 39.2; 20 rows (80 pairs) of 1,500 keys, in three parts, 32.5 -> 26.0;
+//   too few: 40 rows of 160 to 1,600, 39 -> 59.  Heads of 128, 16 over 4, not ranked: 96 rows of 60 to 600 25.5 -> 23.8
+// (ranking 128 rows of at most 300 keys took 20 -> 24; without it 17.6).
 constexpr int DM_WARPS_SHORT = 4;
 constexpr int DM_KEYS_SHORT = 512;
-constexpr int DM_RANKED = 256;                    // rows that a block ranks by their length, at most
+constexpr int DM_RANKED = 96;                     // rows that a block ranks by their length, at most: it compares each with each
 constexpr int DM_BUFS = 3;                        // buffers of one key tile or one value tile per warp: one in use, two in flight
 constexpr int DM_KEYS = 16;                       // keys per warp tile
 
@@ -911,7 +916,7 @@ KF_API int kf_attention_decode_mma_plan(int n_items, int nh, int nkv, int d, int
   if (splits < 1) splits = 1;
   // Blocks of four warps where they can be as many as the GPU holds, but for a fifth: one a pair, or, where a block of eight
   // warps a pair would leave up to half of the SMs without, three.  In between (99 to 230 pairs at heads of 256) they are too few.
-  if (blocks * 5 >= of_four * 4) splits = n_items <= DM_RANKED && max_keys > 128 ? -2 : 0;
+  if (blocks * 5 >= of_four * 4) splits = d == 256 && n_items <= DM_RANKED && max_keys > 128 ? -2 : 0;
   else if (blocks > resident && max_keys <= DM_KEYS_SHORT) splits = 0;
   else if (splits == 1 && blocks < resident && blocks * 3 <= of_four && max_keys > 2 * DM_KEYS_SHORT) splits = -3;
   *splits_out = splits;
