@@ -138,20 +138,20 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   uint64_t* x_empty = x_full + S::X_STAGES;
   uint64_t* a_full = x_empty + S::X_STAGES;                       // [2] weight planes of a chunk are in tensor memory
   uint64_t* done = a_full + 2;                                    // [2] its MMAs have ended
-  uint64_t* acc_free = done + 2;                                  // its accumulators have been read
-  uint32_t* tmem_slot = (uint32_t*)(acc_free + 1);
+  uint64_t* acc_free = done + 2;                                  // [2] its accumulators have been read
+  uint32_t* tmem_slot = (uint32_t*)(acc_free + 2);
   volatile int* s_abort = (volatile int*)(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int chunks = (a.K + CK - 1) / CK;
+  const int sets = 2 * A_COLS + 6 * bn <= S::TMEM ? 2 : 1;          // of accumulators, as tensor memory has room
   const int n_tt = (a.T + bn - 1) / bn, n_ft = (a.N + BM - 1) / BM;
   const int n_units = n_ft * n_tt * a.parts;                      // unit = ((feature tile) * n_tt + row tile) * parts + part
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < ws; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], CUTTERS); }
     for (int s = 0; s < S::X_STAGES; ++s) { mbar_init(&x_full[s], LARGE ? 1 : 128); mbar_init(&x_empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&a_full[b], CUTTERS); mbar_init(&done[b], 1); }
-    mbar_init(acc_free, 128 * S::SUM_GROUPS);
+    for (int b = 0; b < 2; ++b) { mbar_init(&a_full[b], CUTTERS); mbar_init(&done[b], 1); mbar_init(&acc_free[b], 128 * S::SUM_GROUPS); }
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -237,9 +237,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         for (int i = first; i < last; ++i, ++c) {
           const int b = c & 1;
           if (!mbar_wait(&a_full[b], (uint32_t)(c >> 1) & 1) || !mbar_wait(&x_full[x_slot], x_ph) ||
-              (c >= 1 && !mbar_wait(acc_free, (uint32_t)(c - 1) & 1))) { give_up(ERR_WAIT_FULL); ok = false; break; }
+              (c >= sets && !mbar_wait(&acc_free[c & (sets - 1)], (uint32_t)(c / sets - 1) & 1))) { give_up(ERR_WAIT_FULL); ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t wa = tmem + b * A_COLS, acc = tmem + 2 * A_COLS;
+          const uint32_t wa = tmem + b * A_COLS, acc = tmem + 2 * A_COLS + (c & (sets - 1)) * 3 * bn;
           const uint64_t dx = dx0 + (uint64_t)((uint32_t)(x_slot * x_stage) >> 4);
 #pragma unroll
           for (int k = 0; k < CK / UMMA_K; ++k)
@@ -301,16 +301,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     // stage is its accumulator's number, free when its products are done; the next chunk's floats are on their way meanwhile.
     const int ct = threadIdx.x - 64 - CUTTERS, cj = ct & 15;
     int xu = blockIdx.x, xc = 0, xl = 0;
-    float4 xv[2], xn[2];                                          // the next chunk's floats and those of the one after
-    int au = blockIdx.x, ac = 0, al = 0;                          // where the asking is
+    float4 xv[2];
     auto ask_x = [&]() {
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const int t = (ct >> 4) + 8 * u, k = ac * CK + 4 * cj;
-        xv[u] = xn[u];
-        xn[u] = au < n_units && t < a.T && k < a.K ? *reinterpret_cast<const float4*>(a.x + (size_t)t * a.K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const int t = (ct >> 4) + 8 * u, k = xc * CK + 4 * cj;
+        xv[u] = xu < n_units && t < a.T && k < a.K ? *reinterpret_cast<const float4*>(a.x + (size_t)t * a.K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      if (au < n_units && ++ac == al) { au += gridDim.x; if (au < n_units) range(au, ac, al); }
     };
     auto cut_x = [&](int stage) {
       if (xu >= n_units) return;
@@ -331,8 +328,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     };
     if (!LARGE) {
       if (xu < n_units) range(xu, xc, xl);
-      ac = xc, al = xl;
-      ask_x();
       ask_x();
       cut_x(0);
       cut_x(1);
@@ -348,8 +343,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         ok = mbar_wait(&done[b], (uint32_t)(c >> 1) & 1) && !*s_abort;
         if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) give_up(ERR_WAIT_ACC); ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (!LARGE) cut_x(b);
-        const uint32_t acc = lane_addr + 2 * A_COLS + col0;
+        const uint32_t acc = lane_addr + 2 * A_COLS + (c & (sets - 1)) * 3 * bn + col0;
 #pragma unroll
         for (int j0 = 0; j0 < S::COLS; j0 += S::BATCH) {
           if (j0 >= cols) break;
@@ -364,7 +358,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        mbar_arrive(acc_free);
+        mbar_arrive(&acc_free[c & (sets - 1)]);
+        if (!LARGE) cut_x(b);                                     // for the chunk after next, while the next one's MMAs run
       }
       if (!ok) break;
       // ---- the unit's outputs: the parts of a product in a cluster through shared memory, else to memory -----------------------
