@@ -170,7 +170,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     first = (int)((long)z * chunks / a.parts);
     last = (int)((long)(z + 1) * chunks / a.parts);
   };
-  auto give_up = [&](int code) { atomicExch(a.error_flag, code); *s_abort = 1; };
+  auto give_up = [&](int code) { atomicExch(a.error_flag, 32 + code); *s_abort = 1; };
 
   if (warp == 0) {
     // ---- TMA: weights run ahead of x by as many stages as there are, and begin before the kernel ahead has ended ------------

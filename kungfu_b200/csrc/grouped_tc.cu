@@ -73,7 +73,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
   const int bytes = NACC * A_BYTES + (pair ? B_BYTES : B_BYTES / 2);
-  auto give_up = [&](int code) { atomicExch(p.error_flag, code); *s_abort = 1; };
+  auto give_up = [&](int code) { atomicExch(p.error_flag, 48 + code); *s_abort = 1; };
 
   if (warp == 0) {
     if (lane == 0) {

@@ -352,7 +352,7 @@ def raise_on_device_error(device=None) -> None:
     code = device_error(device)
     if code:
         raise KernelError(f"a kernel gave up waiting (code {code}: 1 = operands never arrived, 2 = stage never freed, "
-                          f"3 = accumulator never completed)")
+                          f"3 = accumulator never completed; 32 more in a 32-bit product, 48 more in a mixture's experts)")
 
 
 _rope_plans: dict = {}            # (rows, K, heads, kv heads, head size, rotated) -> whether the fused q,k,v product takes them
