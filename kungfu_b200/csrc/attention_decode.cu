@@ -402,17 +402,11 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 // S = Q K^T (16 heads x 16 keys) and O += P V run on mma.sync with 32-bit accumulators, the online softmax is the
 // one of the prompt kernel.  Warps are merged through shared memory in warp order, splits by the last block.
 constexpr int DM_WARPS = 8;                       // two per scheduler: a warp's tile is one chain of dependent instructions
-// Blocks of four warps, two to an SM at heads of 256: while one starts or merges its warps, the other one's keys keep coming in.
-// They need enough pairs (row, kv head) for all of those blocks, and then are the better ones at any length.  A block of four
-// takes in 24 GB/s whatever its neighbour does, so a row well above the average is cut in two.  Heads of 256, 8 over 4, planned
-// for 2,000 tokens more than there are, us a launch, blocks of eight warps -> of four:
-//   64 rows of 64 keys 13.6 -> 10.9, of 256 19.5 -> 16.7, of 1,024 50.3 -> 45.2, of 2,048 88.2 -> 82.5 (floor 82.0 at 6,544 GB/s),
-//   of 100 to 1,024 41.1 -> 36.1; 78 rows of 90 to 900 42.4 -> 39.2; 20 rows (80 pairs) of 1,500 keys, in three parts, 32.5 -> 26.0;
-//   too few: 40 rows of 160 to 1,600, 39 -> 59.  Heads of 128, 16 over 4, not ranked: 96 rows of 60 to 600 25.5 -> 23.8
-// (ranking 128 rows of at most 300 keys took 20 -> 24; without it 17.6).
+// More (row, kv head) pairs than blocks of eight warps fit the GPU, and short rows: a block then is mostly its start and its
+// merge, and blocks of four warps, two to an SM at heads of 256, cover each other's.  64 rows of 8 heads over 4 of 256, alone:
+// 64 keys 22.6 -> 16.4 us, 256 keys 30.8 -> 24.6, 577 keys 49.2 either way, 1,024 keys 67.6 -> 69.6.
 constexpr int DM_WARPS_SHORT = 4;
 constexpr int DM_KEYS_SHORT = 512;
-constexpr int DM_RANKED = 96;                     // rows that a block ranks by their length, at most: it compares each with each
 constexpr int DM_BUFS = 3;                        // buffers of one key tile or one value tile per warp: one in use, two in flight
 constexpr int DM_KEYS = 16;                       // keys per warp tile
 
@@ -431,7 +425,7 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
                        const int* __restrict__ items, int n_items, const int* __restrict__ positions,
                        const int* __restrict__ row_req, const int* __restrict__ table, int table_stride, int page_size,
                        int nh, int nkv, float scale, float softcap, int window, int vsplit, int keep_first, int sink,
-                       const float* __restrict__ sig_bias, int n_splits, int ranked, float* __restrict__ partial, int* __restrict__ counters,
+                       const float* __restrict__ sig_bias, int n_splits, float* __restrict__ partial, int* __restrict__ counters,
                        __nv_bfloat16* __restrict__ out) {
   using namespace kf_mma;
   kf_pdl_trigger();
@@ -444,44 +438,17 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
   __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(dm_smem);  // [16][D]
   __nv_bfloat16* sKV = sQ + 16 * D;                               // [warp][buffer][16][D]
   __shared__ float sm_ml[DM_WARPS][16][2];
-  __shared__ int s_last, sm_cut;
+  __shared__ int s_last;
 
   // ---- the step's integers: written before the step's first kernel, so readable at once -------------------------------
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // `ranked`: the rows in the order of their lengths, the longest first, and two blocks a pair, of which the second one leaves
-  // unless the row is a quarter longer than the average
-  const bool by_rank = DM_WARPS == DM_WARPS_SHORT && ranked;
-  const int split = by_rank ? blockIdx.x & 1 : blockIdx.y;
-  const int place = by_rank ? blockIdx.x >> 1 : blockIdx.x;
-  int item = place / nkv, cut = 0;
-  const int kvh = place - item * nkv;
-  if (by_rank) {
-    int* s_len = reinterpret_cast<int*>(dm_smem);                  // the ring is not in use yet; more shared memory would cost a block
-    for (int i = tid; i < n_items; i += DM_WARPS * 32) {
-      const int row = items ? items[i] : i, p = positions[row];
-      s_len[i] = row_req[row] < 0 ? 0 : p + 1 - kf_first_key(p, window);
-    }
-    __syncthreads();
-    for (int i = tid; i < n_items; i += DM_WARPS * 32) {
-      const int own = s_len[i];
-      int before = 0, sum = 0, n = 0;
-      for (int j = 0; j < n_items; ++j) {
-        const int len = s_len[j];
-        before += len > own || (len == own && j < i);
-        sum += len;
-        n += len > 0;
-      }
-      if (before == item) s_last = i, sm_cut = n ? (int)((long)sum * 5 / (4 * n)) : 0;
-    }
-    __syncthreads();
-    item = s_last;
-    cut = sm_cut;
-  }
+  const int item = blockIdx.x / nkv, kvh = blockIdx.x - item * nkv;
+  const int split = blockIdx.y;
   const int G = nh / nkv;
   const int h_first = kvh * G;
   const KfHeadMap hm = kf_head_map(h_first, kvh, nh, nkv, vsplit);   // with the rotation inside (qkv given) vsplit is 0
   const int t = items ? items[item] : item;
   const int req = row_req[t];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, tq = lane & 3;
   __nv_bfloat16* orow = out + (size_t)t * nh * D;
   if (req < 0) {
@@ -497,10 +464,7 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
   const int kept = window > 0 ? min(keep_first, lo) : 0;
   const int lo_v = lo - kept;
   const int n_keys = pos + 1 - lo_v;
-  // parts of this row: what the launch is planned for; blocks of four warps are planned for longer rows than there may be
-  const int parts = DM_WARPS != DM_WARPS_SHORT ? n_splits : by_rank ? (n_keys > cut ? 2 : 1) : min(n_splits, (n_keys + 127) / 128);
-  if (split >= parts) return;
-  int per = (n_keys + parts - 1) / parts;
+  int per = (n_keys + n_splits - 1) / n_splits;
   per = (per + 63) & ~63;
   const int k_begin = lo_v + split * per;
   const int k_end = min(pos + 1, k_begin + per);
@@ -772,7 +736,7 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
     }
   }
   __syncthreads();
-  const size_t rec_base = (((size_t)t * nh + h_first) * parts + split) * PSTRIDE;
+  const size_t rec_base = (((size_t)t * nh + h_first) * n_splits + split) * PSTRIDE;
   for (int e = tid; e < G * D; e += blockDim.x) {
     const int h = e / D, i = e - h * D;
     // the sink (a key of score 0 without a value) joins the first split like one more warp: maximum 0, sum 1, no row
@@ -786,26 +750,26 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const float* __restr
       l += sm_ml[w][h][1] * c;
       a += sm_o[((size_t)w * G + h) * D + i] * c;
     }
-    if (parts == 1) {
+    if (n_splits == 1) {
       orow[(size_t)(h_first + h) * D + i] = __float2bfloat16_rn(l > 0.f ? a / l : 0.f);
     } else {
-      float* rec = partial + rec_base + (size_t)h * parts * PSTRIDE;
+      float* rec = partial + rec_base + (size_t)h * n_splits * PSTRIDE;
       rec[i] = a;
       if (i == 0) { rec[D] = m; rec[D + 1] = l; }
     }
   }
-  if (parts == 1) return;
+  if (n_splits == 1) return;
   __threadfence();
   __syncthreads();
   const int cidx = item * nkv + kvh;
-  if (tid == 0) s_last = (atomicAdd(&counters[cidx], 1) == parts - 1);
+  if (tid == 0) s_last = (atomicAdd(&counters[cidx], 1) == n_splits - 1);
   __syncthreads();
   if (!s_last) return;
   __threadfence();                                               // maxima here are base-2 scaled
-  if (parts > 8 && (size_t)G * parts * PSTRIDE * sizeof(float) <= (size_t)DM_WARPS * DM_BUFS * TILE * sizeof(__nv_bfloat16))
-    merge_splits_shared<D>(partial, ((size_t)t * nh + h_first) * parts, G, parts, orow + (size_t)h_first * D, sm_o);
+  if (n_splits > 8 && (size_t)G * n_splits * PSTRIDE * sizeof(float) <= (size_t)DM_WARPS * DM_BUFS * TILE * sizeof(__nv_bfloat16))
+    merge_splits_shared<D>(partial, ((size_t)t * nh + h_first) * n_splits, G, n_splits, orow + (size_t)h_first * D, sm_o);
   else
-    merge_splits<D, true>(partial, ((size_t)t * nh + h_first) * parts, G, parts, orow + (size_t)h_first * D);
+    merge_splits<D, true>(partial, ((size_t)t * nh + h_first) * n_splits, G, n_splits, orow + (size_t)h_first * D);
   if (tid == 0) counters[cidx] = 0;
 }
 
@@ -834,27 +798,25 @@ int launch_decode_mma_warps(const float* qkv, const float* cos_t, const float* s
                       float* partial, int* counters, void* out, cudaStream_t stream) {
   const size_t smem = (size_t)(16 * D + DM_WARPS * DM_BUFS * DM_KEYS * D) * 2;
   if (decode_mma_blocks_per_sm<D, SIG, DM_WARPS>() < 1) return KF_ERR_SETUP;
-  const bool ranked = DM_WARPS == DM_WARPS_SHORT && n_splits == 2 && n_items <= DM_RANKED;
-  const dim3 grid = ranked ? dim3(2 * n_items * nkv) : dim3(n_items * nkv, n_splits);
-  kf_launch(attn_decode_mma_kernel<D, SIG, DM_WARPS>, grid, dim3(DM_WARPS * 32), smem, stream,
+  kf_launch(attn_decode_mma_kernel<D, SIG, DM_WARPS>, dim3(n_items * nkv, n_splits), dim3(DM_WARPS * 32), smem, stream,
             (const __nv_bfloat16*)q, qkv, cos_t, sin_t, rot, write_kv, (__nv_bfloat16*)const_cast<void*>(pages), items, n_items,
             positions, row_req, table, table_stride, page_size, nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias, n_splits,
-            ranked ? 1 : 0, partial, counters, (__nv_bfloat16*)out);
+            partial, counters, (__nv_bfloat16*)out);
   KF_CHECK_LAUNCH();
   return KF_OK;
 }
 
-// n_splits 0: one split in blocks of DM_WARPS_SHORT warps; below 0: up to -n_splits of them (-2: by the rows' ranks).
+// n_splits 0: one split in blocks of DM_WARPS_SHORT warps.
 template <int D, bool SIG>
 int launch_decode_mma(const float* qkv, const float* cos_t, const float* sin_t, int rot, int write_kv,
                       const void* q, const void* pages, const int* items, int n_items, const int* positions,
                       const int* row_req, const int* table, int table_stride, int page_size, int nh, int nkv, float scale,
                       float softcap, int window, int vsplit, int keep_first, int sink, const float* sig_bias, int n_splits,
                       float* partial, int* counters, void* out, cudaStream_t stream) {
-  if (n_splits <= 0)
+  if (n_splits == 0)
     return launch_decode_mma_warps<D, SIG, DM_WARPS_SHORT>(
         qkv, cos_t, sin_t, rot, write_kv, q, pages, items, n_items, positions, row_req, table, table_stride, page_size,
-        nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias, n_splits ? -n_splits : 1, partial, counters, out, stream);
+        nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias, 1, partial, counters, out, stream);
   return launch_decode_mma_warps<D, SIG, DM_WARPS>(
         qkv, cos_t, sin_t, rot, write_kv, q, pages, items, n_items, positions, row_req, table, table_stride, page_size,
         nh, nkv, scale, softcap, window, vsplit, keep_first, sink, sig_bias, n_splits, partial, counters, out, stream);
@@ -893,32 +855,22 @@ static int g_forced_splits = 0;
 KF_API void kf_set_attention_decode_splits(int splits) { g_forced_splits = splits; }
 #endif
 
-// Blocks of one kind that the GPU holds at heads of d elements.
-template <int WARPS>
-static long decode_mma_resident(int d) {
-  long per_sm = d == 256 ? decode_mma_blocks_per_sm<256, false, WARPS>() : d == 128 ? decode_mma_blocks_per_sm<128, false, WARPS>()
-              : d == 64 ? decode_mma_blocks_per_sm<64, false, WARPS>() : d == 32 ? decode_mma_blocks_per_sm<32, false, WARPS>()
-              : d == 16 ? decode_mma_blocks_per_sm<16, false, WARPS>() : 0;
-  if (per_sm > 8) per_sm = 8;
-  return kf_sm_count() * (per_sm < 1 ? 1 : per_sm);
-}
-
-// splits_out: how many parts a row's keys are cut into; 0 or below for blocks of fewer warps, 0 for one part and -k for up to k.
-// kf_attention_decode (ht = 0) and kf_attention_decode_fused take it as it is.
+// splits_out: how many parts a row's keys are cut into; 0 for one part in blocks of fewer warps (short rows, more of them than
+// the GPU holds blocks), which kf_attention_decode (ht = 0) and kf_attention_decode_fused take as it is.
 KF_API int kf_attention_decode_mma_plan(int n_items, int nh, int nkv, int d, int max_keys, int* splits_out) {
   if (g_forced_splits > 0) { *splits_out = g_forced_splits; return KF_OK; }
-  const long blocks = (long)n_items * nkv, resident = decode_mma_resident<DM_WARPS>(d), of_four = decode_mma_resident<DM_WARPS_SHORT>(d);
+  const long blocks = (long)n_items * nkv;
   // fill one wave: as many splits as resident blocks allow
-  int splits = (int)(resident / blocks);
+  long per_sm = d == 256 ? decode_mma_blocks_per_sm<256, false, DM_WARPS>() : d == 128 ? decode_mma_blocks_per_sm<128, false, DM_WARPS>()
+              : d == 64 ? decode_mma_blocks_per_sm<64, false, DM_WARPS>() : d == 32 ? decode_mma_blocks_per_sm<32, false, DM_WARPS>()
+              : d == 16 ? decode_mma_blocks_per_sm<16, false, DM_WARPS>() : 0;
+  if (per_sm > 8) per_sm = 8;
+  if (per_sm < 1) per_sm = 1;
+  int splits = (int)((kf_sm_count() * per_sm) / blocks);
   const int by_len = (max_keys + 255) / 256;
   if (splits > by_len) splits = by_len;
-  if (splits > MERGE_MAX_SPLITS) splits = MERGE_MAX_SPLITS;
-  if (splits < 1) splits = 1;
-  // Blocks of four warps where they can be as many as the GPU holds, but for a fifth: one a pair, or, where a block of eight
-  // warps a pair would leave up to half of the SMs without, three.  In between (99 to 230 pairs at heads of 256) they are too few.
-  if (blocks * 5 >= of_four * 4) splits = d == 256 && n_items <= DM_RANKED && max_keys > 128 ? -2 : 0;
-  else if (blocks > resident && max_keys <= DM_KEYS_SHORT) splits = 0;
-  else if (splits == 1 && blocks < resident && blocks * 3 <= of_four && max_keys > 2 * DM_KEYS_SHORT) splits = -3;
+  if (splits > 64) splits = 64;
+  if (splits < 1) splits = blocks > kf_sm_count() * per_sm && max_keys <= DM_KEYS_SHORT ? 0 : 1;
   *splits_out = splits;
   return KF_OK;
 }
@@ -951,8 +903,8 @@ KF_API int kf_attention_decode(const void* q, void* out, const void* pages, cons
   if (n_items <= 0) return KF_OK;
   if ((keep_first > 0 || sink || sig_bias) && ht != 0) return KF_ERR_SIZE;   // kept first tokens, the sink, sigmoid weights: tensor-core variant only
   if (window <= 0) keep_first = 0;
-  if (nkv < 1 || nh % nkv != 0 || page_size < 1 || n_splits < (ht == 0 ? -MERGE_MAX_SPLITS : 1) || !kf_head_map_ok(nh, nkv, vsplit)) return KF_ERR_SIZE;
-  if ((n_splits > 1 || n_splits < -1) && (!partial || !counters)) return KF_ERR_SIZE;
+  if (nkv < 1 || nh % nkv != 0 || page_size < 1 || n_splits < (ht == 0 ? 0 : 1) || !kf_head_map_ok(nh, nkv, vsplit)) return KF_ERR_SIZE;
+  if (n_splits > 1 && (!partial || !counters)) return KF_ERR_SIZE;
   if (n_splits > MERGE_MAX_SPLITS || ht > MERGE_MAX_HEADS) return KF_ERR_SIZE;
   if (ht == 0) {                                     // tensor-core variant
     if (nh / nkv > 16) return KF_ERR_SIZE;
@@ -990,9 +942,9 @@ KF_API int kf_attention_decode_fused(const float* qkv, const float* cos_t, const
                                      float softcap, int window, int n_splits, float* partial, int* counters,
                                      cudaStream_t stream) {
   if (n_items <= 0) return KF_OK;
-  if (!qkv || nkv < 1 || nh % nkv != 0 || nh / nkv > 16 || page_size < 1 || n_splits < -MERGE_MAX_SPLITS) return KF_ERR_SIZE;
+  if (!qkv || nkv < 1 || nh % nkv != 0 || nh / nkv > 16 || page_size < 1 || n_splits < 0) return KF_ERR_SIZE;
   if (rot < 0 || rot > d || (rot & 1) || (rot > 0 && (!cos_t || !sin_t))) return KF_ERR_SIZE;
-  if ((n_splits > 1 || n_splits < -1) && (!partial || !counters)) return KF_ERR_SIZE;
+  if (n_splits > 1 && (!partial || !counters)) return KF_ERR_SIZE;
   if (n_splits > MERGE_MAX_SPLITS) return KF_ERR_SIZE;
 #define KF_MMA_ARGS qkv, cos_t, sin_t, rot, write_kv, nullptr, pages, items, n_items, positions, row_req, table, table_stride, page_size, nh, nkv, scale, softcap, window, 0, 0, 0, nullptr, n_splits, partial, counters, out, stream
   switch (d) {

@@ -564,7 +564,7 @@ def paged_attention(q, out, ctx, cache, n_heads: int, n_kv_heads: int, head_dim:
         if n_counters > sc["counters"].numel():
             rest, n_rest = None, T
         else:
-            partial = _partial(q.device, T * n_heads * abs(splits.value) * (head_dim + 4)) if abs(splits.value) > 1 else None
+            partial = _partial(q.device, T * n_heads * splits.value * (head_dim + 4)) if splits.value > 1 else None
             items = None if n_dec == T else ctx.dec_rows
             _check(lib.kf_attention_decode(_p(q), _p(out), _p(pages), _p(items), n_dec, *common, ht.value,
                                            splits.value, _p(partial), _p(sc["counters"]), *extras, _stream()), "attention (decode)")
@@ -640,7 +640,7 @@ def rope_append_attend(qkv, cos, sin, rot: int, out, ctx, cache, n_heads: int, n
     splits = ctypes.c_int(0)
     lib.kf_attention_decode_mma_plan(T, n_heads, n_kv_heads, head_dim, int(max_keys), ctypes.byref(splits))
     sc = _dev_scratch(qkv.device)
-    partial = _partial(qkv.device, T * n_heads * abs(splits.value) * (head_dim + 4)) if abs(splits.value) > 1 else None
+    partial = _partial(qkv.device, T * n_heads * splits.value * (head_dim + 4)) if splits.value > 1 else None
     _check(lib.kf_attention_decode_fused(_p(qkv), _p(cos), _p(sin), int(rot), int(cache.writes), _p(out), _p(cache.pages),
                                          None, T, _p(ctx.positions), _p(ctx.row_req), _p(table), table.shape[1],
                                          cache.page_size, n_heads, n_kv_heads, head_dim, _f(scale), _f(softcap),
