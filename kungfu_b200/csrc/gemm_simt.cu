@@ -1,7 +1,7 @@
 // Generic matrix product  out[T, N] = x[T, K] . w[N, K]^T  with 32-bit FMA accumulation.
 //
-// This is the 32-bit product of weights below 4 Mi numbers, of rows that are no multiple of 16 bytes and of unaligned bases
-// (others: `gemm_split.cu`, at the same precision), and the fallback for shapes and types the tensor-core kernels refuse.  Any T, N, K.  The order of an output's sum is
+// This is the true 32-bit product of the engine (no tensor-core or reduced-precision mode) and the
+// fallback for shapes and types the tensor-core kernel refuses.  Any T, N, K.  The order of an output's sum is
 // fixed by (N, K) alone, so a row's result does not depend on T or on which other rows share the launch.
 // `fma_tile_kernel` where both operands are 32-bit; `gemm_simt_kernel` (64 x 64 tiles, k ascending in one thread) for
 // bfloat16 operands; `cols_kernel`, with the same bits, for a few 32-bit rows of a short K on bfloat16 weights.  Reference counterpart: the 32x64x64 shared-tile product in

@@ -1027,23 +1027,26 @@ EncodeTiledFn encode_fn() {
 }
 
 std::mutex g_map_mutex;
-std::map<std::tuple<const void*, long, long, int, bool>, CUtensorMap> g_maps;
+std::map<std::tuple<const void*, long, long, int>, CUtensorMap> g_maps;
 
-// A 2-D map over a row-major [rows, cols] matrix with boxes of box_rows x 128 bytes and the 128-byte swizzle.
-bool cached_map(const void* base, long rows, long cols, int box_rows, bool f32, CUtensorMap* out) {
+// A 2-D map over a row-major [rows, cols] bfloat16 matrix with boxes of [box_rows, 64] and the 128-byte swizzle.
+}  // namespace
+
+bool kf_tc::tensor_maps_available() { return encode_fn() != nullptr; }
+
+bool kf_tc::tensor_map(const void* base, long rows, long cols, int box_rows, CUtensorMap* out) {
   std::lock_guard<std::mutex> lock(g_map_mutex);
-  auto key = std::make_tuple(base, rows, cols, box_rows, f32);
+  auto key = std::make_tuple(base, rows, cols, box_rows);
   auto it = g_maps.find(key);
   if (it != g_maps.end()) { *out = it->second; return true; }
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
-  const int size = f32 ? 4 : 2;
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)cols * size};
-  cuuint32_t box[2] = {(cuuint32_t)(128 / size), (cuuint32_t)box_rows};
+  cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+  cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
   cuuint32_t elem[2] = {1, 1};
   CUtensorMap m;
-  if (fn(&m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+  if (fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return false;
@@ -1051,16 +1054,6 @@ bool cached_map(const void* base, long rows, long cols, int box_rows, bool f32, 
   g_maps[key] = m;
   *out = m;
   return true;
-}
-}  // namespace
-
-bool kf_tc::tensor_maps_available() { return encode_fn() != nullptr; }
-
-bool kf_tc::tensor_map(const void* base, long rows, long cols, int box_rows, CUtensorMap* out) {
-  return cached_map(base, rows, cols, box_rows, false, out);
-}
-bool kf_tc::tensor_map_f32(const void* base, long rows, long cols, int box_rows, CUtensorMap* out) {
-  return cached_map(base, rows, cols, box_rows, true, out);
 }
 
 namespace {

@@ -169,7 +169,6 @@ constexpr int SMEM_LIMIT = 220 * 1024;
 // A 2-D map over a row-major [rows, cols] bfloat16 matrix with boxes of [box_rows, 64] and the 128-byte swizzle
 // (cached per base address and shape).  False if the driver entry point is missing or refuses the shape.
 bool tensor_map(const void* base, long rows, long cols, int box_rows, CUtensorMap* out);
-bool tensor_map_f32(const void* base, long rows, long cols, int box_rows, CUtensorMap* out);      // 32-bit, boxes of [box_rows, 32]
 bool tensor_maps_available();
 
 }  // namespace kf_tc

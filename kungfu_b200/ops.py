@@ -47,7 +47,6 @@ def library():
                 path = _build.build()
                 lib = ctypes.CDLL(path)
                 lib.kf_last_cuda_error.restype = ctypes.c_char_p
-                lib.kf_linear_split_scratch.restype = ctypes.c_long
                 # kernels may start before their predecessor in the stream has finished (each waits for it before
                 # touching dependent memory); KUNGFU_PDL=0 switches that off
                 lib.kf_set_pdl(0 if os.environ.get("KUNGFU_PDL", "1") == "0" else 1)
@@ -352,7 +351,7 @@ def raise_on_device_error(device=None) -> None:
     code = device_error(device)
     if code:
         raise KernelError(f"a kernel gave up waiting (code {code}: 1 = operands never arrived, 2 = stage never freed, "
-                          f"3 = accumulator never completed; 32 more in a 32-bit product, 48 more in a mixture's experts)")
+                          f"3 = accumulator never completed; 48 more in a mixture's experts)")
 
 
 _rope_plans: dict = {}            # (rows, K, heads, kv heads, head size, rotated) -> whether the fused q,k,v product takes them
@@ -386,33 +385,12 @@ def _linear_tc(x, weight, out, mode: int, N: int, softcap: float, act: int) -> b
     return True
 
 
-_split_plans: dict = {}           # (rows, features, K) -> (floats of scratch, launches) of the split product
-
-
-def _linear_split(x, weight, out, N: int, softcap: float) -> bool:
-    """Launch the 32-bit product on the tensor cores if it takes these operands; False if the FMA kernels must run."""
-    T, K = x.shape
-    lib = library()
-    if not (use_tensor_cores and x.dtype == torch.float32 and weight.dtype == torch.float32 and T > 0
-            and lib.kf_linear_split_supported(_p(x), _p(weight), N, K)):
-        return False
-    plan = _split_plans.get((T, N, K))
-    if plan is None:
-        plan = _split_plans[(T, N, K)] = (lib.kf_linear_split_scratch(T, N, K), lib.kf_linear_split_launches(T, N, K))
-    sc = _dev_scratch(x.device)
-    _check(lib.kf_linear_split(_p(x), _p(weight), _p(out), _dt(out), T, N, K, _f(softcap), _p(_partial(x.device, plan[0])),
-                               _p(sc["error"]), _stream()), "linear (32-bit on tensor cores)")
-    add_launches(plan[1] - 1)
-    return True
-
-
 @_dispatch("linear")
 def linear(x, weight, out, softcap: float = 0.0) -> None:
     """out[T, N] = x[T, K] . weight[N, K]^T, 32-bit accumulation; softcap > 0 applies cap*tanh(v/cap).
-    bfloat16 operands run on the tensor cores (tcgen05) when rows are multiples of 16 bytes, and so do 32-bit ones with 4 Mi
-    weights or more, each number cut into three bfloat16 ones; everything else runs 32-bit FMA kernels: the rest of the
-    32-bit path the one in packed tiles, mixed types a generic one, a few 32-bit rows of a short K on bfloat16 weights one
-    of their own."""
+    bfloat16 operands run on the tensor cores (tcgen05) when rows are multiples of 16 bytes; everything else runs 32-bit FMA
+    kernels: the whole 32-bit path the one in packed tiles, mixed types a generic one, a few 32-bit rows of a short K on
+    bfloat16 weights one of their own."""
     T, K = x.shape
     N = weight.shape[0]
     if weight.shape[1] != K or tuple(out.shape) != (T, N):
@@ -420,8 +398,6 @@ def linear(x, weight, out, softcap: float = 0.0) -> None:
     if out.dtype == torch.float32 or softcap == 0.0:
         if _linear_tc(x, weight, out, 0 if out.dtype == torch.float32 else 1, N, softcap, 0):
             return
-    if _linear_split(x, weight, out, N, softcap):
-        return
     _check(library().kf_linear_simt(_p(x), _dt(x), _p(weight), _dt(weight), _p(out), _dt(out), T, N, K, _f(softcap),
                                     _stream()), "linear")
 
