@@ -203,6 +203,8 @@ __device__ __forceinline__ int key_of_tile(int i, int kt_first, int n_kept) {
 }
 // A launch is planned for the longest context that its step may have; a tile whose own keys are few gains nothing from being
 // cut: a key tile takes a block about 0.93 us, the partial rows and their merge as much as MERGE_TILES of them.
+// A step of 512 rows (504 of a prompt beside eight decoding requests of 2,048 keys), attention + merge a launch: 14.7 + 9.9 us with one
+// count of runs for all, 16.6 + 0.5 us by length.
 constexpr int RUNS_BY_LENGTH = -1, MERGE_TILES = 9;
 __device__ __forceinline__ int tile_runs(int n_key_tiles, int n_parts, int run_tiles) {
   if (n_parts <= 1) return 1;

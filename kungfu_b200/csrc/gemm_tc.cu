@@ -523,7 +523,9 @@ struct RopeArgs {
 };
 
 // Feature and token tile of a persistent kernel's tile number: token tiles fastest, so that the CTAs running side by side read a
-// few weight tiles and all the rows, and the weights, by far the larger operand of a prompt, come from memory once.
+// few weight tiles and all the rows, and the weights, by far the larger operand of a prompt, come from memory once.  With the early
+// release below, gated 2,048 x 2 * 9,216 x 2,304: 172.7 -> 138.9 us (MMAs 61 % of the time at work, DRAM 10 %, L2 29 %; SM clock
+// 1.63 GHz); 2,240 x 2 * 14,336 x 3,584: 464.8 -> 378.9 us.
 __device__ __forceinline__ void tile_place(int tile, int n_tt, int& ft, int& tt) {
   ft = tile / n_tt;
   tt = tile - ft * n_tt;
@@ -697,7 +699,8 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = lane_addr + buf * NACC * PN;
       // The next tile's products may begin once this thread's last columns are in registers: with one accumulator set they wait
-      // for the slowest thread, which needs not have stored.
+      // for the slowest thread, which need not have stored.  What is left of that wait: the first of the two products above takes
+      // 119 us with the wait left out of a copy of this kernel, 131 us with the stores left out, and 139 us as it is.
       auto release = [&]() {
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         mbar_arrive_cluster(map_to_rank(smem_u32(&acc_empty[buf]), 0));

@@ -4,7 +4,8 @@
 // A block owns 128 features of an expert x up to 128 of its rows (two neighbouring tiles of the plan's list): weights are the
 // MMA's A operand (128 lanes), rows its N (64 or 128), K in stages of 64 through a TMA ring, one tile per block; roles as in
 // gemm_tc.cu.  Rows that are read through the plan (one row per token) are first copied in sorted order, which costs less
-// than a row-wise gather in every feature tile.  What bounds it is what an SM takes in: 48 KB a stage for 16.8 M multiply-adds.
+// than a row-wise gather in every feature tile.  What bounds it is what an SM takes in: 48 KB a stage for 2.1 M multiply-adds.
+// Gate and up of 3,900 pairs over 32 experts of 2 * 2,048 x 2,048: 355 us on grouped.cu's kernel, 169 us here.
 #include "common.cuh"
 #include "tc_common.cuh"
 
