@@ -38,7 +38,6 @@ __global__ void __launch_bounds__(THREADS)
 grouped_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ GroupedTc p) {
   constexpr int NACC = GATED ? 2 : 1, A_BYTES = BM * BK * 2, B_BYTES = GT_ROWS * BK * 2, STAGE = NACC * A_BYTES + B_BYTES;
   constexpr int TMEM = 128 * NACC;
-  kf_pdl_trigger();
   kf_pdl_wait();                                                  // the plan and the rows come from the kernels ahead
   const int ti = blockIdx.y;
   if (ti >= *p.n_tiles) return;
@@ -73,6 +72,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  kf_pdl_trigger();                                               // after the allocation (tc_common.cuh); a block that left counts as triggered
   const int bytes = NACC * A_BYTES + (pair ? B_BYTES : B_BYTES / 2);
   auto give_up = [&](int code) { atomicExch(p.error_flag, 48 + code); *s_abort = 1; };
 

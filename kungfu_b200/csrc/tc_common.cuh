@@ -1,5 +1,10 @@
 // Device helpers shared by the tcgen05 products: mbarriers with bounded waits, TMA tile loads, shared-memory and
 // instruction descriptors, the MMA and tensor-memory instructions and the fast activations.  Everything is inline; the one host function (the cached tensor maps) lives in gemm_tc.cu.
+//
+// Order in every kernel that uses tensor memory: allocate, __syncthreads, then kf_pdl_trigger.  tcgen05.alloc waits without a
+// limit.  The next kernel's blocks become resident once every block of this one has triggered or left, and they may allocate
+// before their own wait for this kernel: were a block of this kernel still without its columns then, each could wait for the other
+// for good.  In this order a block that holds columns only ever waits for blocks that hold theirs or have freed them.
 #pragma once
 #include "common.cuh"
 #include <cuda.h>
