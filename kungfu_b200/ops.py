@@ -1245,7 +1245,8 @@ def moe_route(logits, correction, groups: int, keep: int, top: int, scale: float
 @_dispatch("moe_plan")
 def moe_plan(ids, n_experts: int, ctx) -> dict:
     """Lay the (token, choice) pairs of `ids` [T, top] out expert by expert.  Returns the device arrays the grouped
-    products and the combination read: sorted_pair, inverse, and the list of 64-row tiles per expert."""
+    products and the combination read: sorted_pair, inverse, and the list of 64-row tiles per expert; `buf` is where the
+    products take their workspace from."""
     T, top = ids.shape
     P = T * top
     max_tiles = P // 64 + n_experts
@@ -1254,7 +1255,7 @@ def moe_plan(ids, n_experts: int, ctx) -> dict:
             "tile_group": ctx.buf("moe_tile_group", (max_tiles,), torch.int32),
             "tile_row0": ctx.buf("moe_tile_row0", (max_tiles,), torch.int32),
             "tile_nrows": ctx.buf("moe_tile_nrows", (max_tiles,), torch.int32),
-            "n_tiles": ctx.buf("moe_n_tiles", (1,), torch.int32)}
+            "n_tiles": ctx.buf("moe_n_tiles", (1,), torch.int32), "buf": ctx.buf}
     _check(library().kf_moe_plan(_p(ids), P, int(n_experts), _p(plan["sorted_pair"]), _p(plan["inverse"]), _p(plan["tile_group"]),
                                  _p(plan["tile_row0"]), _p(plan["tile_nrows"]), _p(plan["n_tiles"]), _stream()), "moe_plan")
     return plan
@@ -1281,7 +1282,7 @@ def moe_linear(x, plan: dict, weight, out, *, gather: bool, gated: bool = False,
     lib = library()
     if (grouped_on_tcgen05 and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
             and lib.kf_grouped_tc_supported(_p(x), _p(weight), ctypes.c_long(plan["pairs"]), E, N, K)):
-        sorted_rows = _partial(x.device, plan["pairs"] * K // 2) if gather else None
+        sorted_rows = plan["buf"]("moe_sorted_rows", (plan["pairs"], K), torch.bfloat16) if gather else None
         _check(lib.kf_grouped_tc(_p(x), _p(plan["sorted_pair"] if gather else None), plan["top"] if gather else 1, _p(sorted_rows), _p(weight),
                                  _p(out), _dt(out), *(_p(t) for t in tiles), plan["max_tiles"], E, plan["pairs"], N, K, act, _f(limit),
                                  _p(row_scale), _p(_dev_scratch(x.device)["error"]), _stream()), "moe_linear (tcgen05)")

@@ -60,3 +60,27 @@ def test_many_rows_per_expert(counts, top, N, K, act, out):
         ops.moe_linear(x[pair // top].to(DEV), plan, w.to(DEV), again, gather=False)
         assert torch.equal(again, got[:-1])
     ops.raise_on_device_error()
+
+
+def test_the_sorted_rows_belong_to_the_plan():
+    """A gathered product writes its result and a buffer of the plan's context; the scratch that every launch of the device shares stays
+    as it is."""
+    from kungfu_b200 import ops
+    P, E, N, K = 256, 2, 128, 64
+    taken = {}
+
+    class Ctx(_Ctx):
+        def buf(self, name, shape, dtype):
+            taken[name] = super().buf(name, shape, dtype)
+            return taken[name]
+
+    plan = ops.moe_plan((torch.arange(P, device=DEV, dtype=torch.int32) % E)[:, None].contiguous(), E, Ctx())
+    x = torch.randn(P, K, device=DEV).to(torch.bfloat16)
+    w = torch.randn(E, N, K, device=DEV).to(torch.bfloat16)
+    out = torch.empty(P, N, device=DEV)
+    shared = ops._partial(torch.device(DEV), P * K)
+    shared.fill_(-3.0)
+    assert ops.library().kf_grouped_tc_supported(0, 0, P, E, N, K)
+    ops.moe_linear(x, plan, w, out, gather=True)
+    assert bool((shared == -3.0).all()) and ops._partial(torch.device(DEV), 1) is shared
+    assert torch.equal(taken["moe_sorted_rows"], x[plan["sorted_pair"].long()])
