@@ -522,13 +522,20 @@ struct RopeArgs {
   __nv_bfloat16* q_out;                                           // [T, nh * head size]
 };
 
-// Feature and token tile of a persistent kernel's tile number: token tiles fastest, so that the CTAs running side by side read a
-// few weight tiles and all the rows, and the weights, by far the larger operand of a prompt, come from memory once.  With the early
-// release below, gated 2,048 x 2 * 9,216 x 2,304: 172.7 -> 138.9 us (MMAs 61 % of the time at work, DRAM 10 %, L2 29 %; SM clock
-// 1.63 GHz); 2,240 x 2 * 14,336 x 3,584: 464.8 -> 378.9 us.
-__device__ __forceinline__ void tile_place(int tile, int n_tt, int& ft, int& tt) {
-  ft = tile / n_tt;
-  tt = tile - ft * n_tt;
+// Feature and token tile of a persistent kernel's tile number.  The CTAs running side by side should read all of the smaller operand,
+// which then stays in L2, and a few tiles of the larger one, which comes from memory once: token tiles fastest while x has no more
+// rows than the weights, feature tiles fastest beyond.  L2 flushed, one launch, feature-first -> token-first: gated 768 x 2 * 36,864 x 4,608
+// 418 -> 367 us, 2,048 x 2 * 14,336 x 3,584 355 -> 328 us, 2,048 x 2 * 9,216 x 2,304 172.5 -> 169.1 us; with more rows than weights 16,384 x 2,304 x 9,216 472
+// -> 513 us, 32,768 x 4,096 x 2,304 468 -> 501 us; where both operands fit in L2 the two are equal.  The gated product of 2,048 rows has its
+// MMAs 61 % of the time at work, DRAM 10 %, L2 29 % (SM clock 1.63 GHz).
+__device__ __forceinline__ void tile_place(int tile, int n_ft, int n_tt, bool tokens_first, int& ft, int& tt) {
+  if (tokens_first) {
+    ft = tile / n_tt;
+    tt = tile - ft * n_tt;
+  } else {
+    tt = tile / n_ft;
+    ft = tile - tt * n_ft;
+  }
 }
 
 template <int EPI, int PN>                                        // PN: tokens of the pair's tile = MMA N (256, or 128 for EPI_ROPE)
@@ -563,6 +570,7 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
   const int n_tiles = n_ft * n_tt;
   const int nkb = (K + BK - 1) / BK;
   const int second = ROPE ? BM : up_offset;                       // weight rows of the second accumulator, after the first's
+  const bool tokens_first = (long)T <= (GATED ? 2l : 1l) * n_feat;   // no more rows than the weights have
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -593,7 +601,7 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
       const uint32_t full0 = map_to_rank(smem_u32(&full[0]), 0);   // the leader's full[0], as a cluster address
       for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
         int ft, tt;
-        tile_place(tile, n_tt, ft, tt);
+        tile_place(tile, n_ft, n_tt, tokens_first, ft, tt);
         const int f0 = (ft * 2 + (int)rank) * (ROPE ? 2 * BM : BM);
         const int t0 = tt * PN + (int)rank * (PN / 2);
         for (int kb = 0; kb < nkb; ++kb) {
@@ -662,7 +670,7 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
     for (int tile = pair; tile < n_tiles; tile += n_pairs, ++ti) {
       const int buf = ti % NBUF;
       int ft, tt;
-      tile_place(tile, n_tt, ft, tt);
+      tile_place(tile, n_ft, n_tt, tokens_first, ft, tt);
       const int f0 = (ft * 2 + (int)rank) * (ROPE ? 2 * BM : BM), t0 = tt * PN;
       const int f = f0 + quarter * 32 + lane;
       // ROPE: where this warp's PN / 4 rows go (one or two rows per lane), looked up while the accumulator is still being filled:
@@ -699,8 +707,8 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = lane_addr + buf * NACC * PN;
       // The next tile's products may begin once this thread's last columns are in registers: with one accumulator set they wait
-      // for the slowest thread, which need not have stored.  What is left of that wait: the first of the two products above takes
-      // 119 us with the wait left out of a copy of this kernel, 131 us with the stores left out, and 139 us as it is.
+      // for the slowest thread, which need not have stored.  Gated 2,048 x 2 * 9,216 x 2,304, 20 launches in a graph: 172.7 us without the
+      // two rules, 138.9 with them; of that wait 119 us with it left out of a copy of this kernel, 131 with the stores left out.
       auto release = [&]() {
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         mbar_arrive_cluster(map_to_rank(smem_u32(&acc_empty[buf]), 0));
