@@ -185,7 +185,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
 }
 
 // The 64-key tiles a tile of query rows reads (and its first key), and into how many runs they are cut: `n_parts` runs for
-// every tile when `run_tiles` is 0; as many as the tile's own length is worth, up to n_parts, when it is RUNS_BY_LENGTH;
+// every tile when `run_tiles` is 0; n_parts or, where the tile's own length is not worth it, one when it is RUNS_BY_LENGTH;
 // otherwise as many runs of at most `run_tiles` key tiles as the tile needs, at most n_parts (short tiles then stay whole and
 // write their rows themselves, long ones are shared between blocks).
 // With kept first tokens (keys 0..keep_first-1 stay visible behind the window) the tiles of those keys that lie before
@@ -202,17 +202,22 @@ __device__ __forceinline__ int key_of_tile(int i, int kt_first, int n_kept) {
   return i < n_kept ? i * BKV : kt_first + (i - n_kept) * BKV;
 }
 // A launch is planned for the longest context that its step may have; a tile whose own keys are few gains nothing from being
-// cut: a key tile takes a block about 0.93 us, the partial rows and their merge as much as MERGE_TILES of them.
-// A step of 512 rows (504 of a prompt beside eight decoding requests of 2,048 keys), attention + merge a launch: 14.7 + 9.9 us with one
-// count of runs for all, 16.6 + 0.5 us by length.
-constexpr int RUNS_BY_LENGTH = -1, MERGE_TILES = 9;
-__device__ __forceinline__ int tile_runs(int n_key_tiles, int n_parts, int run_tiles) {
+// cut.  A cut saves the key tiles that other blocks take, key_tile_ns each.  It costs 2.2 us, 18 ns for every element of a head (a block's
+// partial rows) and 2.5 ns for every element of a row (their merge), less the 0.26 us that the merge's blocks of a whole tile take to
+// find that out.  These were read off launches of 1 to 8 tiles of 128 rows, 4 to 32 heads of 64, 128 and 256, 2 to 8 runs and 2 to 64 key tiles.
+// Attention and merge, planned for 16,384 keys, every tile cut -> by length: 4 tiles, 8 heads of 256, scores capped, of 8 / 14 / 24 key tiles 22.4 -> 17.1,
+// 24.5 -> 22.9, 26.8 -> 26.8 us; 1 tile, 8 heads of 64, of 4 / 8 / 24 key tiles 8.7 -> 7.6, 9.7 -> 9.7, 11.5 -> 11.5 us; nowhere more than 6 % slower.
+// Tiles cut into fewer runs than the launch has were slower (28 key tiles in seven of eight runs 27.9 -> 30.9 us), so there are the two.
+// A step of 512 rows (504 of a prompt beside eight decoding requests of 2,048 keys), attention + merge a launch: 14.7 + 9.9 us with every tile
+// cut, 16.6 + 0.5 us by length.
+constexpr int RUNS_BY_LENGTH = -1;
+template <int D>
+__device__ __forceinline__ int tile_runs(int n_key_tiles, int n_parts, int run_tiles, int nh, int n_tiles, bool capped) {
   if (n_parts <= 1) return 1;
   if (run_tiles == RUNS_BY_LENGTH) {
-    int best = 1;
-    for (int p = 2; p <= n_parts; ++p)
-      if ((n_key_tiles + p - 1) / p + MERGE_TILES < (n_key_tiles + best - 1) / best + (best > 1 ? MERGE_TILES : 0)) best = p;
-    return best;
+    const int key_tile_ns = D == 256 ? (capped ? 980 : 940) : D == 128 ? (capped ? 850 : 620) : (capped ? 830 : 580);
+    const int saved = n_key_tiles - (n_key_tiles + n_parts - 1) / n_parts;
+    return saved * key_tile_ns <= 2200 + 18 * D + 5 * nh * D / 2 - 260 * n_tiles ? 1 : n_parts;
   }
   if (run_tiles <= 0) return n_parts;
   const int p = (n_key_tiles + run_tiles - 1) / run_tiles;
@@ -302,7 +307,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   const int pos0 = positions[row0];
   int kt_first, n_kept;
   const int n_tiles_all = tile_key_tiles(row0, nrows, positions, row_req, window, keep_first, &kt_first, &n_kept);
-  const int my_parts = tile_runs(n_tiles_all, n_parts, run_tiles);
+  const int my_parts = tile_runs<D>(n_tiles_all, n_parts, run_tiles, nh, (int)(gridDim.x / (nh * n_parts)), softcap > 0.f);
   const bool idle = part >= my_parts;                     // this tile has fewer runs than the launch has blocks per tile
   const int per_part = (n_tiles_all + my_parts - 1) / my_parts;
   const int tile_begin = part * per_part;                 // this run's first tile of the walk
@@ -626,13 +631,13 @@ __global__ void __launch_bounds__(128)
 attn_prefill_merge_kernel(const float* __restrict__ partial, const int* __restrict__ tile_row0,
                           const int* __restrict__ tile_nrows, const int* __restrict__ positions,
                           const int* __restrict__ row_req, int window, int keep_first, int nh, int n_parts_max,
-                          int run_tiles, __nv_bfloat16* __restrict__ out) {
+                          int run_tiles, int capped, __nv_bfloat16* __restrict__ out) {
   kf_pdl_trigger();
   const int tile = blockIdx.x, r = blockIdx.y;                // the step's integers may be read before the wait
   const int nrows = tile_nrows[tile];
   int kt_first, n_kept;
-  const int n_parts = tile_runs(tile_key_tiles(tile_row0[tile], nrows, positions, row_req, window, keep_first,
-                                               &kt_first, &n_kept), n_parts_max, run_tiles);
+  const int n_parts = tile_runs<D>(tile_key_tiles(tile_row0[tile], nrows, positions, row_req, window, keep_first,
+                                                  &kt_first, &n_kept), n_parts_max, run_tiles, nh, gridDim.x, capped);
   kf_pdl_wait();
   if (r >= nrows || n_parts == 1) return;                     // a tile with one run wrote its rows itself
   partial = kf_produced(partial);
@@ -726,7 +731,7 @@ int launch(const CUtensorMap& tq, const CUtensorMap& tkv, const int* tile_row0, 
   KF_CHECK_LAUNCH();
   if (n_parts > 1) {
     kf_launch(attn_prefill_merge_kernel<D>, dim3(n_tiles, BMQ), dim3(128), 0, stream, (const float*)partial, tile_row0,
-              tile_nrows, positions, row_req, window, keep_first, nh, n_parts, run_tiles, (__nv_bfloat16*)out);
+              tile_nrows, positions, row_req, window, keep_first, nh, n_parts, run_tiles, (int)(softcap > 0.f), (__nv_bfloat16*)out);
     KF_CHECK_LAUNCH();
   }
   return KF_OK;
@@ -746,7 +751,7 @@ static int g_forced_parts = 0, g_forced_run_tiles = 0;
 KF_API void kf_set_attention_prefill_plan(int parts, int run_tiles) { g_forced_parts = parts, g_forced_run_tiles = run_tiles; }
 #endif
 
-// Into how many runs the keys of a tile are cut, and how long a run may be (0: every tile gets `parts` runs).
+// Into how many runs the keys of a tile are cut, and how long a run may be (0: no bound, the caller may leave short tiles whole).
 // Few blocks (tiles x heads fill less than half of the GPU): every tile may be cut so that the blocks fill it; at most 8
 // runs, never so many that a run of the longest tile has fewer than two 64-key tiles, and only if the shorter loop
 // saves more than the partial rows and their merge cost.
@@ -765,7 +770,8 @@ KF_API int kf_attention_prefill_tc_plan(int n_tiles, int nh, int max_keys, int* 
   const int key_tiles = (max_keys + BKV - 1) / BKV;
   if (parts > key_tiles / 2) parts = key_tiles / 2;
   if (parts < 1) parts = 1;
-  // A key tile takes a block about 0.93 us; partial rows, their merge kernel and its launch about 11 us together.  Of the
+  // For the longest tile: a key tile of head size 256 takes a block about 0.93 us; partial rows, their merge kernel and its launch were
+  // 11 us together at the 8 heads and 4 runs this was measured at (tile_runs has the figures for other sizes).  Of the
   // run counts that fill the GPU the one with the shortest estimate wins, so short prompts stay whole.
   int best = 1;
   float best_us = 0.93f * (float)key_tiles;
@@ -778,7 +784,8 @@ KF_API int kf_attention_prefill_tc_plan(int n_tiles, int nh, int max_keys, int* 
 
 // q, out: [T, nh*d] bfloat16; pages: [n_pages, 2, nkv, page_size, d] bfloat16.  tile_row0/tile_nrows: tiles of up to 128
 // consecutive rows of one request (consecutive positions).  n_parts > 1 cuts a tile's keys into up to that many runs
-// (every tile's when run_tiles is 0, by the tiles' own lengths when it is -1, else those of tiles with more than run_tiles key tiles);
+// (every tile's when run_tiles is 0, those of tiles that are worth it when it is -1, else those of tiles with more than run_tiles key
+// tiles);
 // `partial` then holds T * nh * n_parts * (d + 4) floats.
 KF_API int kf_attention_prefill_tc(const void* q, void* out, const void* pages, long n_pages, int T, const int* tile_row0,
                                    const int* tile_nrows, int n_tiles, const int* positions, const int* row_req,
