@@ -185,7 +185,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
 }
 
 // The 64-key tiles a tile of query rows reads (and its first key), and into how many runs they are cut: `n_parts` runs for
-// every tile when `run_tiles` is 0; n_parts or, where the tile's own length is not worth it, one when it is RUNS_BY_LENGTH;
+// every tile when `run_tiles` is 0 or RUNS_OF_ALL; n_parts or, where the tile's own length is not worth it, one when it is RUNS_BY_LENGTH;
 // otherwise as many runs of at most `run_tiles` key tiles as the tile needs, at most n_parts (short tiles then stay whole and
 // write their rows themselves, long ones are shared between blocks).
 // With kept first tokens (keys 0..keep_first-1 stay visible behind the window) the tiles of those keys that lie before
@@ -210,7 +210,7 @@ __device__ __forceinline__ int key_of_tile(int i, int kt_first, int n_kept) {
 // Tiles cut into fewer runs than the launch has were slower (28 key tiles in seven of eight runs 27.9 -> 30.9 us), so there are the two.
 // A step of 512 rows (504 of a prompt beside eight decoding requests of 2,048 keys), attention + merge a launch: 14.7 + 9.9 us with every tile
 // cut, 16.6 + 0.5 us by length.
-constexpr int RUNS_BY_LENGTH = -1;
+constexpr int RUNS_BY_LENGTH = -1, RUNS_OF_ALL = -2;
 template <int D>
 __device__ __forceinline__ int tile_runs(int n_key_tiles, int n_parts, int run_tiles, int nh, int n_tiles, bool capped) {
   if (n_parts <= 1) return 1;
@@ -747,7 +747,7 @@ KF_API int kf_attention_prefill_tc_tile_rows() { return BMQ; }
 
 static int g_forced_parts = 0, g_forced_run_tiles = 0;
 #ifdef KF_TUNING
-// Measurement hook of a tuning build: a fixed plan instead of the planner's (0, 0 gives its choice back).
+// Measurement hook of a tuning build: a fixed plan instead of the planner's (parts 0 gives its choice back; run_tiles 0: every tile).
 KF_API void kf_set_attention_prefill_plan(int parts, int run_tiles) { g_forced_parts = parts, g_forced_run_tiles = run_tiles; }
 #endif
 
@@ -761,7 +761,7 @@ KF_API void kf_set_attention_prefill_plan(int parts, int run_tiles) { g_forced_p
 // runs slower: the partial rows cost a write, a read and a second kernel.  So such launches stay uncut.
 KF_API int kf_attention_prefill_tc_plan(int n_tiles, int nh, int max_keys, int* run_tiles) {
   *run_tiles = 0;
-  if (g_forced_parts > 0) { *run_tiles = g_forced_run_tiles; return g_forced_parts; }
+  if (g_forced_parts > 0) { *run_tiles = g_forced_run_tiles > 0 ? g_forced_run_tiles : RUNS_OF_ALL; return g_forced_parts; }
   const long blocks = (long)n_tiles * nh;
   const int n_sm = kf_sm_count();
   if (blocks <= 0 || 2 * blocks > n_sm) return 1;
@@ -784,7 +784,7 @@ KF_API int kf_attention_prefill_tc_plan(int n_tiles, int nh, int max_keys, int* 
 
 // q, out: [T, nh*d] bfloat16; pages: [n_pages, 2, nkv, page_size, d] bfloat16.  tile_row0/tile_nrows: tiles of up to 128
 // consecutive rows of one request (consecutive positions).  n_parts > 1 cuts a tile's keys into up to that many runs
-// (every tile's when run_tiles is 0, those of tiles that are worth it when it is -1, else those of tiles with more than run_tiles key
+// (every tile's when run_tiles is 0 or -2, those of tiles that are worth it when it is -1, else those of tiles with more than run_tiles key
 // tiles);
 // `partial` then holds T * nh * n_parts * (d + 4) floats.
 KF_API int kf_attention_prefill_tc(const void* q, void* out, const void* pages, long n_pages, int T, const int* tile_row0,
@@ -796,7 +796,7 @@ KF_API int kf_attention_prefill_tc(const void* q, void* out, const void* pages, 
   if (window <= 0) keep_first = 0;
   if (nkv < 1 || nh % nkv != 0 || page_size % 64 != 0 || !kf_head_map_ok(nh, nkv, vsplit)) return KF_ERR_SIZE;
   const KfHeadMap hm = kf_head_map(0, 0, nh, nkv, vsplit);
-  if (n_parts < 1 || n_parts > 8 || (n_parts > 1 && !partial) || run_tiles < RUNS_BY_LENGTH) return KF_ERR_SIZE;
+  if (n_parts < 1 || n_parts > 8 || (n_parts > 1 && !partial) || run_tiles < RUNS_OF_ALL) return KF_ERR_SIZE;
   CUtensorMap tq, tkv;
   if (!tensor_map(q, T, (long)hm.n_query * d, BMQ, &tq)) return KF_ERR_SETUP;
   if (!tensor_map(pages, n_pages * 2 * hm.n_stored * page_size, d, BKV, &tkv)) return KF_ERR_SETUP;
