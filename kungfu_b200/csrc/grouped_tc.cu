@@ -5,7 +5,8 @@
 // MMA's A operand (128 lanes), rows its N (64 or 128), K in stages of 64 through a TMA ring, one tile per block; roles as in
 // gemm_tc.cu.  Rows that are read through the plan (one row per token) are first copied in sorted order, which costs less
 // than a row-wise gather in every feature tile.  What bounds it is what an SM takes in: 48 KB a stage for 2.1 M multiply-adds.
-// Gate and up of 3,900 pairs over 32 experts of 2 * 2,048 x 2,048: 355 us on grouped.cu's kernel, 169 us here.
+// 128 rows for each of 32 experts of 2,048 x 2,048, grouped.cu's kernel -> this one: gate and up 277 -> 125 us, down 133 -> 57 us.  Its results
+// are those of grouped.cu's tensor-core kernels bit for bit.
 #include "common.cuh"
 #include "tc_common.cuh"
 
@@ -33,8 +34,12 @@ __global__ void __launch_bounds__(256) sorted_rows_kernel(const uint4* src, cons
   for (int i = threadIdx.x; i < chunks; i += 256) dst[(size_t)r * chunks + i] = from[i];
 }
 
+// Warps of the epilogue.  An activation is a chain of an exponential and a division, 0.16 us a row with one warp per scheduler, which
+// nothing hides: gated products have four (the product above 168 -> 125 us, N = K = 512 of two experts of 192 rows 24 -> 13 us).
+template <int GATED> constexpr int EPI_WARPS = GATED ? 16 : 4;
+
 template <int GATED, typename TO>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(64 + 32 * EPI_WARPS<GATED>)
 grouped_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ GroupedTc p) {
   constexpr int NACC = GATED ? 2 : 1, A_BYTES = BM * BK * 2, B_BYTES = GT_ROWS * BK * 2, STAGE = NACC * A_BYTES + B_BYTES;
   constexpr int TMEM = 128 * NACC;
@@ -120,23 +125,30 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     if (!ok && lane == 0) give_up(ERR_WAIT_ACC);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (__all_sync(0xffffffffu, ok)) {
-      TO* out = (TO*)p.out;
-      for (int c0 = 0; c0 < nrows; c0 += 16) {
+      TO* out = (TO*)p.out + (size_t)r0 * p.N + f;
+      for (int c0 = (warp - 2) / 4 * 16; c0 < nrows; c0 += EPI_WARPS<GATED> / 4 * 16) {
         float v[16], u[16];
         tmem_ld16(lane_addr + c0, v);
-        if (GATED) tmem_ld16(lane_addr + GT_ROWS + c0, u);
+        if (GATED) {
+          tmem_ld16(lane_addr + GT_ROWS + c0, u);
+          if (p.row_scale)
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int r = r0 + c0 + j;
-          if (c0 + j >= nrows || f >= p.N) continue;
-          float y = v[j];
-          if (GATED) {
-            const float rs = p.row_scale ? p.row_scale[p.row_index ? p.row_index[r] : r] : 1.f;
-            const float ga = v[j] * rs, up = u[j] * rs;
-            y = p.silu ? ga / (1.f + expf(-ga)) * up : kf_clamped_swish(ga, up, p.limit);
+            for (int j = 0; j < 16; ++j) {
+              const int r = r0 + min(c0 + j, nrows - 1);
+              const float rs = p.row_scale[p.row_index ? p.row_index[r] : r];
+              v[j] *= rs, u[j] *= rs;
+            }
+          if (p.silu) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = v[j] / (1.f + expf(-v[j])) * u[j];
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = kf_clamped_swish(v[j], u[j], p.limit);
           }
-          kf_store(out, (size_t)r * p.N + f, y);
         }
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (c0 + j < nrows && f < p.N) kf_store(out, (size_t)(c0 + j) * p.N, v[j]);
       }
     }
   }
@@ -162,7 +174,7 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tx, GroupedTc p, int max_ti
     }
     configured = true;
   }
-  kf_launch(kernel, dim3(kf_ceil_div(p.N, BM), max_tiles), dim3(THREADS), smem, s, tw, tx, p);
+  kf_launch(kernel, dim3(kf_ceil_div(p.N, BM), max_tiles), dim3(64 + 32 * EPI_WARPS<GATED>), smem, s, tw, tx, p);
   KF_CHECK_LAUNCH();
   return KF_OK;
 }
@@ -174,6 +186,14 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tx, GroupedTc p, int max_ti
 // read only the experts and rows that exist, are the better ones.
 KF_API int kf_grouped_tc_supported(const void* x, const void* w, long pairs, int groups, int N, int K) {
   return pairs >= 64l * groups && N >= 128 && K > 0 && K % 8 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0 && tensor_maps_available();
+}
+
+// Whether it is also the faster one for these sizes.  A short K does not hide a block's start, the copy of gathered rows and the gated epilogue.
+// Against grouped.cu's kernels, times here over times there at 64 to 320 rows for each of 2 to 96 experts, evenly spread and on a third of the
+// experts: gathered and gated, K 256 0.6 to 2.0, 512 0.5 to 1.5, 768 0.4 to 1.0 from 384 features on (below to 1.2), 1,536 0.3 to 1.0 at any N; one of
+// the two, 768 0.4 to 0.9 (to 1.2); neither, K 64 0.6 to 1.3, 128 0.5 to 1.2, 256 0.4 to 0.9.
+KF_API int kf_grouped_tc_pays(int gathered, int gated, int N, int K) {
+  return K >= (gathered || gated ? (N >= 384 ? 768 : 1536) : 256);
 }
 
 // x: [pairs, K], or with row_index one row per row_index[r] / row_div, copied to `sorted` [pairs, K] first.  gated: 0, 1 (the

@@ -1202,7 +1202,7 @@ def _grouped(x, x_off, ldx, x_gstride, row_index, row_div, w, w_gstride, out, o_
                                        int(gated), _f(limit), _p(row_scale), int(most_rows), _stream()), what)
 
 
-grouped_on_tcgen05 = True       # False: experts of many rows run the mma.sync kernel too
+grouped_on_tcgen05 = True       # False: experts of many rows run the mma.sync kernel too; "always": also where that one is the faster
 
 
 def grouped_on_tensor_cores(on: bool) -> None:
@@ -1281,6 +1281,7 @@ def moe_linear(x, plan: dict, weight, out, *, gather: bool, gated: bool = False,
     act = (2 if activation == "silu" else 1) if gated else 0
     lib = library()
     if (grouped_on_tcgen05 and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
+            and (grouped_on_tcgen05 == "always" or lib.kf_grouped_tc_pays(int(gather), int(gated), N, K))
             and lib.kf_grouped_tc_supported(_p(x), _p(weight), ctypes.c_long(plan["pairs"]), E, N, K)):
         sorted_rows = plan["buf"]("moe_sorted_rows", (plan["pairs"], K), torch.bfloat16) if gather else None
         _check(lib.kf_grouped_tc(_p(x), _p(plan["sorted_pair"] if gather else None), plan["top"] if gather else 1, _p(sorted_rows), _p(weight),

@@ -6,6 +6,13 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
+@pytest.fixture(autouse=True)
+def every_size(monkeypatch):
+    """The kernel's edges lie at sizes at which the other one is faster."""
+    from kungfu_b200 import ops
+    monkeypatch.setattr(ops, "grouped_on_tcgen05", "always")
+
+
 class _Ctx:
     def buf(self, name, shape, dtype):
         return torch.empty(shape, dtype=dtype, device=DEV)
@@ -84,3 +91,26 @@ def test_the_sorted_rows_belong_to_the_plan():
     ops.moe_linear(x, plan, w, out, gather=True)
     assert bool((shared == -3.0).all()) and ops._partial(torch.device(DEV), 1) is shared
     assert torch.equal(taken["moe_sorted_rows"], x[plan["sorted_pair"].long()])
+
+
+@pytest.mark.parametrize("gather,gated,N,K,takes", [(True, True, 384, 768, True), (True, True, 383, 768, False), (True, True, 384, 760, False), (True, True, 128, 1536, True),
+                                                    (False, True, 128, 1528, False), (True, False, 512, 512, False), (False, False, 128, 256, True), (False, False, 128, 248, False)])
+def test_the_line_between_the_two_kernels(gather, gated, N, K, takes, monkeypatch):
+    """Which kernel a product of 64 rows an expert takes; one row fewer an expert never takes the tcgen05 one."""
+    from kungfu_b200 import ops
+    monkeypatch.setattr(ops, "grouped_on_tcgen05", True)
+    lib, seen = ops.library(), []
+
+    class Spy:
+        def __getattr__(self, name):
+            if name in ("kf_grouped_tc", "kf_grouped_linear"):
+                seen.append(name)
+            return getattr(lib, name)
+
+    monkeypatch.setattr(ops, "library", Spy)
+    x = torch.randn(128, K, device=DEV).to(torch.bfloat16)
+    w = torch.randn(2, 2 * N if gated else N, K, device=DEV).to(torch.bfloat16)
+    for rows in (128, 126):
+        plan = ops.moe_plan((torch.arange(rows, device=DEV, dtype=torch.int32) % 2)[:, None].contiguous(), 2, _Ctx())
+        ops.moe_linear(x[:rows], plan, w, torch.empty(rows, N, device=DEV), gather=gather, gated=gated, limit=1.0)
+    assert seen == ["kf_grouped_tc" if takes else "kf_grouped_linear", "kf_grouped_linear"]
