@@ -258,7 +258,7 @@ static int grouped_mma_go(const KfGroupedArgs& p, int max_tiles, int n_groups, c
 //     so that a thread holds both numbers of a feature), K in slices of 64 (128-byte pieces) through a ring of six stages:
 //     three or four blocks per SM have 120 to 160 KB of weights on their way.
 // Shared rows are 128 bytes with their 16-byte chunks XOR-swizzled by the row.  A row's sums run over k in ascending order
-// and do not depend on the other rows, nor on which of the two kernels runs: the order over k is the same.  A tile with more
+// and do not depend on the other rows, nor on which of the two kernels, or that of grouped_tc.cu, runs: the order over k is the same.  A tile with more
 // rows than 8 * NT takes several passes over its weights; with `two` = 1 neighbouring blocks take every other one, so that both
 // read the same pieces at about the same time.
 // Measured (one B200, experts of 2 x 2,048 x 2,048 and 2,048 x 2,048, eight tokens with three of 32 each, in place in a
@@ -432,7 +432,7 @@ KF_API int kf_grouped_linear(const void* x, int x_dtype, long x_off, long ldx, l
   const bool x_ok = x_dtype == KF_F32 || (ldx % 8 == 0 && x_gstride % 8 == 0 && x_off % 8 == 0 && ((uintptr_t)x & 15) == 0);
   if (g_grouped_tensor_cores && w_ok && x_ok) {
     // Few rows per group: up to 32 at most, or 16 on average.  From there on the 64-row tiles of the kernel above read the
-    // weights once and fill their MMAs.  On average only: a group of 33 to 64 rows costs two passes, side by side.  Gate and up /
+    // weights once and fill their MMAs (from 64 rows an expert on average grouped_tc.cu may have taken the product before it gets here).  On average only: a group of 33 to 64 rows costs two passes, side by side.  Gate and up /
     // down of 32 experts of 2,048 x 2,048 at 510 pairs, in us, the 64-row kernel -> this one (one after the other in brackets):
     // evenly spread 156 / 86 -> 115 / 72, a third on one expert 168 / 86 -> 119 / 66, all on three 70 / 47 -> 68 / 43 (78 / 42),
     // all on twelve, the worst found, 74 / 53 -> 82 / 43 (92 / 51).

@@ -114,3 +114,31 @@ def test_the_line_between_the_two_kernels(gather, gated, N, K, takes, monkeypatc
         plan = ops.moe_plan((torch.arange(rows, device=DEV, dtype=torch.int32) % 2)[:, None].contiguous(), 2, _Ctx())
         ops.moe_linear(x[:rows], plan, w, torch.empty(rows, N, device=DEV), gather=gather, gated=gated, limit=1.0)
     assert seen == ["kf_grouped_tc" if takes else "kf_grouped_linear", "kf_grouped_linear"]
+
+
+# 63 and 64 rows an expert on average; the second step holds the first one's tokens.  K with a last slice of 8 and of 64, one stage and many.
+@pytest.mark.parametrize("E,N,K", [(2, 128, 8), (3, 200, 520), (2, 1000, 264), (8, 512, 768), (4, 300, 2048)])
+@pytest.mark.parametrize("act", ["", "clamped_swish", "silu"])
+@pytest.mark.parametrize("out", ["bfloat16", "float32"])
+def test_a_row_has_the_same_bits_on_either_side_of_the_line(E, N, K, act, out):
+    """A token's result does not depend on what else is in the step, although from 64 rows an expert on average another kernel takes the
+    product: both sum a row's products in 32 bits over k in ascending slices of 16."""
+    from kungfu_b200 import ops
+    gated, many, few = bool(act), 64 * E, 64 * E - 1
+    g = torch.Generator().manual_seed(E + K)
+    ids = torch.randint(0, E, (many, 1), generator=g).to(torch.int32)
+    x = torch.randn(many, K, generator=g).to(torch.bfloat16).to(DEV)
+    x[::7] *= 1e4                                              # rows whose sums cancel differently in another order
+    w = (torch.randn(E, 2 * N if gated else N, K, generator=g) * K ** -0.5).to(torch.bfloat16).to(DEV)
+    scale = torch.rand(many, 1, generator=g).to(DEV) if act == "silu" else None
+    got = {}
+    for n in (few, many):
+        plan = ops.moe_plan(ids[:n].to(DEV), E, _Ctx())
+        assert bool(ops.library().kf_grouped_tc_supported(0, 0, n, E, N, K)) == (n == many)
+        y = torch.empty(n, N, dtype=getattr(torch, out), device=DEV)
+        ops.moe_linear(x[:n], plan, w, y, gather=True, gated=gated, limit=0.9, activation=act or "clamped_swish",
+                       row_scale=scale[:n] if scale is not None else None)
+        got[n] = torch.empty_like(y)
+        got[n][plan["sorted_pair"].long()] = y
+    assert torch.equal(got[few], got[many][:few])
+    ops.raise_on_device_error()
