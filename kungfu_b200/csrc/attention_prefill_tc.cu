@@ -50,9 +50,9 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int limits = 1) {
   const uint32_t addr = smem_u32(bar);
-  for (long i = 0; i < WAIT_LIMIT; ++i) {
+  for (long i = 0; i < limits * WAIT_LIMIT; ++i) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -329,7 +329,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         int page = tab[kt / page_size];
         if (page < 0) page = 0;                            // a page already given back: every key of it is masked
         const int krow = ((page * 2 + 0) * hm.n_stored + hm.key) * page_size + (kt % page_size);
-        if (i >= 2 && !mbar_wait(&k_free[s], ((i >> 1) - 1) & 1)) { atomicExch(error_flag, ERR_ATTN_WAIT + 1); *s_abort = 1; break; }
+        if (i >= 2 && !mbar_wait(&k_free[s], ((i >> 1) - 1) & 1)) { atomicCAS(error_flag, 0, ERR_ATTN_WAIT + 1); *s_abort = 1; break; }
         mbar_expect_tx(&k_full[s], KV_BYTES);
 #pragma unroll
         for (int j = 0; j < NSUB; ++j) tma_load_2d(sK + s * KV_BYTES + j * (BKV * 128), &tm_kv, &k_full[s], j * 64, krow);
@@ -345,7 +345,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         int page = tab[kt / page_size];
         if (page < 0) page = 0;
         const int vrow = ((page * 2 + 1) * hm.n_stored + hm.value) * page_size + (kt % page_size);
-        if (i >= 2 && !mbar_wait(&v_free[s], ((i >> 1) - 1) & 1)) { atomicExch(error_flag, ERR_ATTN_WAIT + 1); *s_abort = 1; break; }
+        if (i >= 2 && !mbar_wait(&v_free[s], ((i >> 1) - 1) & 1)) { atomicCAS(error_flag, 0, ERR_ATTN_WAIT + 1); *s_abort = 1; break; }
         mbar_expect_tx(&v_full[s], KV_BYTES);
 #pragma unroll
         for (int j = 0; j < NSUB; ++j) tma_load_2d(sV + s * KV_BYTES + j * (BKV * 128), &tm_kv, &v_full[s], j * 64, vrow);
@@ -371,7 +371,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         umma_commit(&s_full[s]);
         umma_commit(&k_free[s]);
       }
-      if (!ok) { atomicExch(error_flag, ERR_ATTN_WAIT + 2); *s_abort = 1; }
+      if (!ok) { atomicCAS(error_flag, 0, ERR_ATTN_WAIT + 2); *s_abort = 1; }
     }
   } else if (warp == 9) {
     // ---- issuer of O += P V -----------------------------------------------------------------------------------
@@ -392,7 +392,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         umma_commit(&v_free[s]);
         umma_commit(&pv_done[i & 1]);
       }
-      if (!ok) { atomicExch(error_flag, ERR_ATTN_WAIT + 2); *s_abort = 1; }
+      if (!ok) { atomicCAS(error_flag, 0, ERR_ATTN_WAIT + 2); *s_abort = 1; }
     }
   } else {
     // ---- softmax and epilogue: group `grp` takes every other key tile; one thread per query row -----------------------
@@ -412,10 +412,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     constexpr int HC = D / 2;                              // O columns of this thread in the epilogue
     float m_mine = -INFINITY, l_sum = 0.f;                 // this group's sum of exponentials, scaled to 2^-m_mine
     bool ok = true;
+    // Waits of two limits: an issuer or producer that gives up is then the first to say so (the error word keeps the first code).
     // A thread runs every turn of its loop and arrives at every barrier of it, also after a wait has run out (the waits
     // are then skipped and the numbers are garbage that nobody stores): nobody is left waiting for it.
     for (int i = grp; i < n_tiles; i += 2) {
-      ok = ok && mbar_wait(&s_full[grp], (i >> 1) & 1);
+      ok = ok && mbar_wait(&s_full[grp], (i >> 1) & 1, 2);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int kt = key_of_tile(tile_begin + i, kt_first, n_kept);   // first key of the tile
       float sv[64];
@@ -500,7 +501,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         }
         const float m_tile = fmaxf(fmaxf(mt[0], mt[1]), fmaxf(mt[2], mt[3]));
         // the maximum O is scaled to after tile i - 1, from the other group; this tile's goes back the same way
-        if (i > 0) ok = ok && mbar_wait(&m_done[grp ^ 1], ((i - 1) >> 1) & 1);
+        if (i > 0) ok = ok && mbar_wait(&m_done[grp ^ 1], ((i - 1) >> 1) & 1, 2);
         const float m_used = i > 0 ? s_max[r] : -INFINITY;
         raise = m_tile > m_used + RESCALE_STEP;   // also true for the first finite maximum
         const float m_new = raise ? m_tile : m_used;
@@ -523,7 +524,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         m_mine = m_new;
       }
       if (i > 0) {                                          // P V of the previous tile must be done: O is at rest, P is free
-        ok = ok && mbar_wait(&pv_done[(i - 1) & 1], ((i - 1) >> 1) & 1);
+        ok = ok && mbar_wait(&pv_done[(i - 1) & 1], ((i - 1) >> 1) & 1, 2);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (!SIG && __any_sync(0xffffffffu, raise)) {              // rescale this row of O (all lanes of the warp take part)
 #pragma unroll 1
@@ -548,8 +549,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive(p_full);
     }
-    if (ok && n_tiles > 0) ok = mbar_wait(&pv_done[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1);
-    if (!ok) { atomicExch(error_flag, ERR_ATTN_WAIT + 3); *s_abort = 1; }
+    if (ok && n_tiles > 0) ok = mbar_wait(&pv_done[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, 2);
+    if (!ok) { atomicCAS(error_flag, 0, ERR_ATTN_WAIT + 3); *s_abort = 1; }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     float m_used = 0.f;
     if constexpr (!SIG) {

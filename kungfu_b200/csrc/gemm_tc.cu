@@ -111,7 +111,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       for (int i = pre_all; i < nkb && drop < 0; ++i) {
         const int s = i % stages;
         if (!mbar_wait(&empty[s], ((i / stages) - 1) & 1)) {
-          atomicExch(error_flag, ERR_WAIT_EMPTY);
+          record_error(error_flag, ERR_WAIT_EMPTY);
           s_flags[0] = 1;
           break;
         }
@@ -134,7 +134,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       uint32_t ph = 0;
       for (int i = 0; i < nkb && ok; ++i) {
         if (!mbar_wait(&full[s], ph)) {
-          atomicExch(error_flag, ERR_WAIT_FULL);
+          record_error(error_flag, ERR_WAIT_FULL);
           s_flags[0] = 1;
           ok = false;
           break;
@@ -157,8 +157,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     kf_pdl_wait();                                                             // before any global write
     const int quarter = warp & 3;
     const int f = f0 + quarter * 32 + lane;                                    // this thread's output feature
-    const bool acc_ok = mbar_wait(acc_full, 0);
-    if (!acc_ok && lane == 0) atomicExch(error_flag, ERR_WAIT_ACC);
+    const bool acc_ok = mbar_wait(acc_full, 0, 2);
+    if (!acc_ok && lane == 0) record_error(error_flag, ERR_WAIT_ACC);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const bool good = acc_ok && s_flags[0] == 0;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
@@ -367,7 +367,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
         const int f0 = (tile % n_ft) * BM, t0 = (tile / n_ft) * BN;
         for (int kb = 0; kb < nkb; ++kb) {
           if (!mbar_wait(&empty[s], ph)) {
-            atomicExch(error_flag, ERR_WAIT_EMPTY);
+            record_error(error_flag, ERR_WAIT_EMPTY);
             *s_abort = 1;
             ok = false;
             break;
@@ -398,7 +398,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem_base + buf * ACC_COLS;
         for (int kb = 0; kb < nkb; ++kb) {
-          if (!mbar_wait(&full[s], ph)) { ok = false; break; }
+          if (!mbar_wait(&full[s], ph)) { record_error(error_flag, ERR_WAIT_FULL); *s_abort = 1; ok = false; break; }   // before the commit below
           const uint64_t so = (uint64_t)((uint32_t)s * (uint32_t)(STAGE_BYTES >> 4));   // descriptors advance by address >> 4
           const uint64_t da = da0 + so, db = db0 + so, du = du0 + so;
 #pragma unroll
@@ -412,7 +412,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
         }
         umma_commit(&acc_full[buf]);
       }
-      if (!ok) { atomicExch(error_flag, ERR_WAIT_FULL); *s_abort = 1; }
+      if (!ok) { record_error(error_flag, ERR_WAIT_FULL); *s_abort = 1; }
     }
   } else {
     // ---- epilogue: drains one accumulator set while the other is being filled -----------------------------------------
@@ -424,8 +424,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       const int buf = ti & 1;
       const int f0 = (tile % n_ft) * BM, t0 = (tile / n_ft) * BN;
       const int f = f0 + quarter * 32 + lane;
-      if (!mbar_wait(&acc_full[buf], (uint32_t)(ti >> 1) & 1) || *s_abort) {
-        if (lane == 0) atomicExch(error_flag, ERR_WAIT_ACC);
+      if (!mbar_wait(&acc_full[buf], (uint32_t)(ti >> 1) & 1, 2) || *s_abort) {
+        if (lane == 0) record_error(error_flag, ERR_WAIT_ACC);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -606,7 +606,7 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
         const int t0 = tt * PN + (int)rank * (PN / 2);
         for (int kb = 0; kb < nkb; ++kb) {
           if (!mbar_wait(&empty[s], ph)) {
-            atomicExch(error_flag, ERR_WAIT_EMPTY);
+            record_error(error_flag, ERR_WAIT_EMPTY);
             *s_abort = 1;
             ok = false;
             break;
@@ -644,7 +644,7 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem_base + buf * NACC * PN;
         for (int kb = 0; kb < nkb; ++kb) {
-          if (!mbar_wait(&full[s], ph)) { ok = false; break; }
+          if (!mbar_wait(&full[s], ph)) { record_error(error_flag, ERR_WAIT_FULL); *s_abort = 1; ok = false; break; }   // before the commit below
           const uint64_t so = (uint64_t)((uint32_t)s * (uint32_t)(STAGE_BYTES >> 4));
           const uint64_t da = da0 + so, db = db0 + so, du = du0 + so;
 #pragma unroll
@@ -658,7 +658,7 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
         }
         umma_commit_pair(&acc_full[buf]);
       }
-      if (!ok) { atomicExch(error_flag, ERR_WAIT_FULL); *s_abort = 1; }
+      if (!ok) { record_error(error_flag, ERR_WAIT_FULL); *s_abort = 1; }
     }
   } else {
     // ---- epilogue (both CTAs): each drains its own 128 lanes ------------------------------------------------------------
@@ -700,8 +700,8 @@ gemm_tc_pair_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x, void* __rest
           if (cc) meta_b = m; else meta_a = m;
         }
       }
-      if (!mbar_wait(&acc_full[buf], (uint32_t)(ti / NBUF) & 1) || *s_abort) {
-        if (lane == 0) atomicExch(error_flag, ERR_WAIT_ACC);
+      if (!mbar_wait(&acc_full[buf], (uint32_t)(ti / NBUF) & 1, 2) || *s_abort) {
+        if (lane == 0) record_error(error_flag, ERR_WAIT_ACC);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -897,7 +897,7 @@ gemm_tc_pair_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       uint32_t ph = 0;                                             // parity of `empty` when a stage has been used once
       for (int i = pre; i < nkb; ++i) {
         if (!mbar_wait(&empty[s], ph)) {
-          atomicExch(error_flag, ERR_WAIT_EMPTY);
+          record_error(error_flag, ERR_WAIT_EMPTY);
           *s_abort = 1;
           break;
         }
@@ -919,7 +919,7 @@ gemm_tc_pair_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       uint32_t ph = 0;
       bool ok = true;
       for (int kb = 0; kb < nkb; ++kb) {
-        if (!mbar_wait(&full[s], ph)) { ok = false; break; }
+        if (!mbar_wait(&full[s], ph)) { record_error(error_flag, ERR_WAIT_FULL); *s_abort = 1; ok = false; break; }   // before the commit below
         const uint64_t so = (uint64_t)((uint32_t)s * (uint32_t)(STAGE_BYTES >> 4));
         const uint64_t da = da0 + so, db = db0 + so;
 #pragma unroll
@@ -929,7 +929,7 @@ gemm_tc_pair_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
         if (++s == stages) { s = 0; ph ^= 1; }
       }
       umma_commit_pair_at(acc_full, leader);
-      if (!ok) { atomicExch(error_flag, ERR_WAIT_FULL); *s_abort = 1; }
+      if (!ok) { record_error(error_flag, ERR_WAIT_FULL); *s_abort = 1; }
     }
   } else {
     // ---- epilogue, first half: every CTA parks its own 128 lanes x 256 tokens in shared memory as [token][feature] -------
@@ -938,8 +938,8 @@ gemm_tc_pair_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     float* red = reinterpret_cast<float*>(smem);
     const int fl = quarter * 32 + lane;
-    if (!mbar_wait(acc_full, 0) || *s_abort) {
-      if (lane == 0) atomicExch(error_flag, ERR_WAIT_ACC);
+    if (!mbar_wait(acc_full, 0, 2) || *s_abort) {
+      if (lane == 0) record_error(error_flag, ERR_WAIT_ACC);
     } else {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1

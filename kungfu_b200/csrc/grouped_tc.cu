@@ -79,7 +79,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   const uint32_t tmem = *tmem_slot;
   kf_pdl_trigger();                                               // after the allocation (tc_common.cuh); a block that left counts as triggered
   const int bytes = NACC * A_BYTES + (pair ? B_BYTES : B_BYTES / 2);
-  auto give_up = [&](int code) { atomicExch(p.error_flag, 48 + code); *s_abort = 1; };
+  auto give_up = [&](int code) { record_error(p.error_flag, 48 + code); *s_abort = 1; };
 
   if (warp == 0) {
     if (lane == 0) {
@@ -121,7 +121,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   } else {
     const int quarter = warp & 3, f = f0 + quarter * 32 + lane;
     const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
-    const bool ok = mbar_wait(acc_full, 0) && !*s_abort;
+    const bool ok = mbar_wait(acc_full, 0, 2) && !*s_abort;
     if (!ok && lane == 0) give_up(ERR_WAIT_ACC);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (__all_sync(0xffffffffu, ok)) {

@@ -33,7 +33,8 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 }
 // Bounded wait: false if the phase did not complete within the limit.  try_wait itself may block for a while that
 // the hardware chooses, so the limit is a time (about two seconds on the global timer, looked at every 256 turns)
-// as well as a count.
+// as well as a count.  `limits`: that many times the limit.  An accumulator's readers wait two of them, so that a producer or issuer that
+// gives up, and lets them go, is the first to say so.
 constexpr unsigned long long WAIT_LIMIT_NS = 2000ull * 1000ull * 1000ull;
 // The limit in force (one copy per translation unit).  A test shortens it through the translation unit's hook to see a
 // wait give up; nothing else writes it.
@@ -43,10 +44,10 @@ __device__ __forceinline__ unsigned long long global_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int limits = 1) {
   const uint32_t addr = smem_u32(bar);
   unsigned long long t0 = 0;
-  for (int i = 0; i < WAIT_LIMIT; ++i) {
+  for (int i = 0; i < limits * WAIT_LIMIT; ++i) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -57,11 +58,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     if ((i & 255) == 255) {
       const unsigned long long now = global_ns();
       if (t0 == 0) t0 = now;
-      else if (now - t0 > g_wait_limit_ns) return false;
+      else if (now - t0 > limits * g_wait_limit_ns) return false;
     }
   }
   return false;
 }
+// The error word keeps the first code: whoever waits for the one that gave up follows it.
+__device__ __forceinline__ void record_error(int* flag, int code) { atomicCAS(flag, ERR_NONE, code); }
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"

@@ -331,7 +331,7 @@ def _partial(device, n_floats: int) -> torch.Tensor:
 
 
 def device_error(device=None) -> int:
-    """The error word kernels with bounded waits write (0 = none).  Reading it waits for the device."""
+    """The error word kernels with bounded waits write (0 = none; the first code stays).  Reading it waits for the device."""
     if device is None:
         device = torch.device("cuda", torch.cuda.current_device())
     sc = _scratch.get((device.type, device.index))
@@ -350,8 +350,12 @@ def clear_device_error(device=None) -> None:
 def raise_on_device_error(device=None) -> None:
     code = device_error(device)
     if code:
-        raise KernelError(f"a kernel gave up waiting (code {code}: 1 = operands never arrived, 2 = stage never freed, "
-                          f"3 = accumulator never completed; 48 more in a mixture's experts)")
+        where, what = divmod(code, 16)
+        kernel = {0: "a product", 1: "prompt attention", 3: "a mixture's experts"}.get(where, "unknown")
+        kinds = ("a stage was never freed", "operands never arrived", "scores or sums never came") if where == 1 else (
+            "operands never arrived", "a stage was never freed", "an accumulator was never completed")
+        raise KernelError(f"a kernel gave up waiting (code {code}, the first to give up: {kernel}, "
+                          f"{kinds[what - 1] if 1 <= what <= 3 else 'unknown'})")
 
 
 _rope_plans: dict = {}            # (rows, K, heads, kv heads, head size, rotated) -> whether the fused q,k,v product takes them
