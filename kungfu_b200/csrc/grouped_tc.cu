@@ -14,6 +14,9 @@ namespace {
 
 using namespace kf_tc;
 
+// A test can make the producer leave out the loads of every stage from this one on (-1: never); see kf_test_grouped_give_up.
+static __device__ int g_test_drop_from_stage = -1;
+
 constexpr int GT_ROWS = 128, GT_PLAN = 64;                      // rows of a block; of a tile of the plan
 
 struct GroupedTc {
@@ -43,7 +46,8 @@ __global__ void __launch_bounds__(64 + 32 * EPI_WARPS<GATED>)
 grouped_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ GroupedTc p) {
   constexpr int NACC = GATED ? 2 : 1, A_BYTES = BM * BK * 2, B_BYTES = GT_ROWS * BK * 2, STAGE = NACC * A_BYTES + B_BYTES;
   constexpr int TMEM = 128 * NACC;
-  kf_pdl_wait();                                                  // the plan and the rows come from the kernels ahead
+  const int drop = g_test_drop_from_stage;                        // asked for while the kernels ahead finish
+  kf_pdl_wait();                                                  // the plan and the rows come from them
   const int ti = blockIdx.y;
   if (ti >= *p.n_tiles) return;
   const int g = p.tile_group[ti];
@@ -79,15 +83,18 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   const uint32_t tmem = *tmem_slot;
   kf_pdl_trigger();                                               // after the allocation (tc_common.cuh); a block that left counts as triggered
   const int bytes = NACC * A_BYTES + (pair ? B_BYTES : B_BYTES / 2);
-  auto give_up = [&](int code) { record_error(p.error_flag, 48 + code); *s_abort = 1; };
+  int issued = 0;                                                 // stages this thread has asked for (the producer's count)
+  auto give_up = [&](int code) { record_error(p.error_flag, 48 + code); *s_abort = 1; __threadfence_block(); };
 
   if (warp == 0) {
     if (lane == 0) {
       const int w0 = g * NACC * p.N + f0;                         // the expert's gate rows, then its up rows
       int s = 0;
       uint32_t ph = 1;
-      for (int i = 0; i < nkb; ++i) {
+      const int last = drop >= 0 && drop < nkb ? drop : nkb;
+      for (; issued < last; ++issued) {
         if (!mbar_wait(&empty[s], ph)) { give_up(ERR_WAIT_EMPTY); break; }
+        const int i = issued;
         uint8_t* st = smem + (size_t)s * STAGE;
         mbar_expect_tx(&full[s], bytes);
         tma_load_2d(st, &tm_w, &full[s], i * BK, w0);
@@ -154,6 +161,9 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  // After a wait that ran out: loads that nobody waited for have landed before this block's shared memory becomes another's.
+  if (threadIdx.x == 0 && *s_abort)
+    for (int i = max(0, issued - p.stages); i < issued; ++i) mbar_wait(&full[i % p.stages], (uint32_t)(i / p.stages) & 1);
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM) : "memory");
@@ -215,4 +225,15 @@ KF_API int kf_grouped_tc(const void* x, const int* row_index, int row_div, void*
   if (out_dtype == KF_BF16) return gated ? launch<1, __nv_bfloat16>(tw, tx, p, max_tiles, stream) : launch<0, __nv_bfloat16>(tw, tx, p, max_tiles, stream);
   if (out_dtype == KF_F32) return gated ? launch<1, float>(tw, tx, p, max_tiles, stream) : launch<0, float>(tw, tx, p, max_tiles, stream);
   return KF_ERR_DTYPE;
+}
+
+// For tests: as kf_test_gemm_give_up, for the experts' kernel.
+KF_API int kf_test_grouped_give_up(unsigned long long limit_ns, int drop_from_stage) {
+  const unsigned long long lim = limit_ns ? limit_ns : WAIT_LIMIT_NS;
+  if (cudaMemcpyToSymbol(g_wait_limit_ns, &lim, sizeof(lim)) != cudaSuccess ||
+      cudaMemcpyToSymbol(g_test_drop_from_stage, &drop_from_stage, sizeof(int)) != cudaSuccess) {
+    kf_record_cuda_error(cudaGetLastError());
+    return KF_ERR_SETUP;
+  }
+  return KF_OK;
 }
