@@ -5,7 +5,7 @@
 // MMA's A operand (128 lanes), rows its N (64 or 128), K in stages of 64 through a TMA ring, one tile per block; roles as in
 // gemm_tc.cu.  Rows that are read through the plan (one row per token) are first copied in sorted order, which costs less
 // than a row-wise gather in every feature tile.  What bounds it is what an SM takes in: 48 KB a stage for 2.1 M multiply-adds.
-// 128 rows for each of 32 experts of 2,048 x 2,048, grouped.cu's kernel -> this one: gate and up 277 -> 125 us, down 133 -> 57 us.  Its results
+// 128 rows for each of 32 experts of 2,048 x 2,048, grouped.cu's kernel -> this one: gate and up 276 -> 118 us, down 133 -> 57 us.  Its results
 // are those of grouped.cu's tensor-core kernels bit for bit.
 #include "common.cuh"
 #include "tc_common.cuh"
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(256) sorted_rows_kernel(const uint4* src, cons
 }
 
 // Warps of the epilogue.  An activation is a chain of an exponential and a division, 0.16 us a row with one warp per scheduler, which
-// nothing hides: gated products have four (the product above 168 -> 125 us, N = K = 512 of two experts of 192 rows 24 -> 13 us).
+// nothing hides: gated products have four (the product above 168 -> 118 us, N = K = 512 of two experts of 192 rows 24 -> 13 us).
 template <int GATED> constexpr int EPI_WARPS = GATED ? 16 : 4;
 
 template <int GATED, typename TO>
